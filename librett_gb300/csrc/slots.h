@@ -1,0 +1,210 @@
+// Slot addressing of the flat and bulk-copy tile kernels (table-free tiles).
+//
+// Thread t of a CTA handles in-tile elements x = t * V + k * B of one side,
+// k = 0, 1, ... ("slots"), with B = TILE_THREADS * V.  The offset of x is the
+// sum of its mixed-radix digits times their steps.  Decoding every x costs a
+// multiply-high and two multiply-adds per rank and element; here the digits
+// of t * V are decoded once per thread, the digits c of k * B are the same
+// for every thread and are worked out on the host, and the sum of the two is
+// formed by adding with carry:
+//   d[r] + c[r] + carry >= ext[r]  <=>  d[r] + carry >= lim = ext[r] - c[r],
+// and each carry replaces ext[r] steps of rank r by one of rank r + 1
+// (corr = step[r + 1] - ext[r] * step[r]).  A slot then costs one addition
+// plus, per rank but the last, one comparison and one predicated addition
+// with operands in the parameter block.
+//
+// Narrow units are bound by instruction issue: float32 (127, 63, 65, 33) perm
+// (3, 1, 2, 0), which moves in 4-byte units on both sides, issued 74 warp
+// instructions per 32 elements with every element decoded on its own and 45
+// with slot sums (39.9 -> 30.9 us).
+//
+// Unused high ranks have ext 2^16 (in-tile indices are smaller, so their
+// lower neighbour never carries into them) and step 0.  Sums are unsigned: a
+// sum before its carries are applied may pass 2^31, the offset itself never
+// does.
+#pragma once
+
+#include <cstdint>
+
+#include "plan.h"
+
+#ifdef __CUDACC__
+#define LT_HD __host__ __device__ __forceinline__
+#else
+#define LT_HD inline
+#endif
+
+namespace lt {
+
+constexpr int SLOT_EXT_NONE = 1 << 16;
+
+LT_HD uint32_t slotMulHi(uint32_t a, uint32_t b) {
+#ifdef __CUDA_ARCH__
+  return __umulhi(a, b);
+#else
+  return (uint32_t)(((uint64_t)a * b) >> 32);
+#endif
+}
+
+// Load side: NS slots, NR ranks (>= 2), one offset.
+template <int NS, int NR>
+struct LoadSlots {
+  uint32_t mul[NR - 1];  // ceil(2^32 / ext)
+  int ext[NR - 1];
+  uint32_t step[NR];
+  uint32_t corr[NR - 1];
+  int lim[NS][NR - 1];
+  uint32_t off[NS];  // offset of k * B
+};
+
+// Store side: the global output offset and the input-order index (in bytes).
+template <int NS, int NR>
+struct StoreSlots {
+  uint32_t mul[NR - 1];
+  int ext[NR - 1];
+  uint32_t step[NR], stepJ[NR];
+  uint32_t corr[NR - 1], corrJ[NR - 1];
+  int lim[NS][NR - 1];
+  uint32_t off[NS], offJ[NS];
+};
+
+// Digits of in-tile index x (below 2^16): d[0 .. NR-2], the last digit
+// returned.
+template <int NR>
+LT_HD int slotDigits(const uint32_t* mul, const int* ext, uint32_t x, int* d) {
+#pragma unroll
+  for (int r = 0; r + 1 < NR; ++r) {
+    const uint32_t q = slotMulHi(x, mul[r]);
+    d[r] = (int)(x - q * (uint32_t)ext[r]);
+    x = q;
+  }
+  return (int)x;
+}
+
+template <int NS, int NR>
+LT_HD uint32_t loadThreadOffset(const LoadSlots<NS, NR>& s, uint32_t x, int* d) {
+  uint32_t off = (uint32_t)slotDigits<NR>(s.mul, s.ext, x, d) * s.step[NR - 1];
+#pragma unroll
+  for (int r = 0; r + 1 < NR; ++r) off += (uint32_t)d[r] * s.step[r];
+  return off;
+}
+
+template <int NS, int NR>
+LT_HD uint32_t loadSlotOffset(const LoadSlots<NS, NR>& s, int k, uint32_t offT, const int* d) {
+  uint32_t off = offT + s.off[k];
+  int carry = 0;
+#pragma unroll
+  for (int r = 0; r + 1 < NR; ++r) {
+    const bool c = d[r] + carry >= s.lim[k][r];
+    if (c) off += s.corr[r];
+    carry = c ? 1 : 0;
+  }
+  return off;
+}
+
+template <int NS, int NR>
+LT_HD void storeThreadOffset(const StoreSlots<NS, NR>& s, uint32_t x, int* d, uint32_t& off,
+                             uint32_t& j) {
+  const uint32_t top = (uint32_t)slotDigits<NR>(s.mul, s.ext, x, d);
+  off = top * s.step[NR - 1];
+  j = top * s.stepJ[NR - 1];
+#pragma unroll
+  for (int r = 0; r + 1 < NR; ++r) {
+    off += (uint32_t)d[r] * s.step[r];
+    j += (uint32_t)d[r] * s.stepJ[r];
+  }
+}
+
+template <int NS, int NR>
+LT_HD void storeSlotOffset(const StoreSlots<NS, NR>& s, int k, uint32_t offT, uint32_t jT,
+                           const int* d, uint32_t& off, uint32_t& j) {
+  off = offT + s.off[k];
+  j = jT + s.offJ[k];
+  int carry = 0;
+#pragma unroll
+  for (int r = 0; r + 1 < NR; ++r) {
+    const bool c = d[r] + carry >= s.lim[k][r];
+    if (c) {
+      off += s.corr[r];
+      j += s.corrJ[r];
+    }
+    carry = c ? 1 : 0;
+  }
+}
+
+// Load-side ranks of a tile: its ranks in input order, a rank whose input
+// stride continues the previous one's extent merged into it (a tile that
+// covers whole leading dims has one contiguous run there).  Returns their
+// number.
+inline int loadRanks(const TileParams& tp, int* ext, int* step) {
+  int n = 0;
+  for (int t = 0; t < tp.nTR; ++t) {
+    if (n > 0 && (int64_t)tp.trSin[t] == (int64_t)ext[n - 1] * step[n - 1]) {
+      ext[n - 1] *= tp.trE[t];
+    } else {
+      ext[n] = tp.trE[t];
+      step[n] = tp.trSin[t];
+      ++n;
+    }
+  }
+  return n;
+}
+
+namespace detail {
+
+// Fields shared by both sides: digits by ext (n ranks, padded to NR), limits
+// and offsets of slot k at element k * B for steps `step`.
+template <int NS, int NR>
+void fillSlots(int n, const int* ext, const int* step, int B, uint32_t* mul, int* extOut,
+               uint32_t* stepOut, uint32_t* corr, int (*lim)[NR - 1], uint32_t* off) {
+  int e[NR], st[NR];
+  for (int r = 0; r < NR; ++r) {
+    e[r] = r < n ? ext[r] : SLOT_EXT_NONE;
+    st[r] = r < n ? step[r] : 0;
+    stepOut[r] = (uint32_t)st[r];
+  }
+  for (int r = 0; r + 1 < NR; ++r) {
+    mul[r] = (uint32_t)(((uint64_t(1) << 32) + e[r] - 1) / e[r]);
+    extOut[r] = e[r];
+    // an unused neighbour is never carried into
+    corr[r] = r + 1 < n ? (uint32_t)st[r + 1] - (uint32_t)e[r] * (uint32_t)st[r] : 0;
+  }
+  for (int k = 0; k < NS; ++k) {
+    uint32_t x = (uint32_t)(k * B);
+    uint32_t o = 0;
+    for (int r = 0; r + 1 < NR; ++r) {
+      const uint32_t q = x / (uint32_t)e[r];
+      const int c = (int)(x - q * (uint32_t)e[r]);
+      lim[k][r] = e[r] - c;
+      o += (uint32_t)c * (uint32_t)st[r];
+      x = q;
+    }
+    off[k] = o + x * (uint32_t)st[NR - 1];  // slots past the tile are never used
+  }
+}
+
+}  // namespace detail
+
+template <int NS, int NR>
+void makeLoadSlots(const TileParams& tp, LoadSlots<NS, NR>& s) {
+  int ext[MAXR], step[MAXR];
+  const int n = loadRanks(tp, ext, step);
+  detail::fillSlots<NS, NR>(n, ext, step, TILE_THREADS * tp.lv, s.mul, s.ext, s.step, s.corr, s.lim,
+                            s.off);
+}
+
+template <int NS, int NR>
+void makeStoreSlots(const TileParams& tp, int esize, StoreSlots<NS, NR>& s) {
+  int stepJ[MAXR];
+  for (int i = 0; i < tp.nTR; ++i) stepJ[i] = tp.toInTile[i] * esize;
+  detail::fillSlots<NS, NR>(tp.nTR, tp.toE, tp.toSout, TILE_THREADS * tp.sv, s.mul, s.ext, s.step,
+                            s.corr, s.lim, s.off);
+  detail::fillSlots<NS, NR>(tp.nTR, tp.toE, stepJ, TILE_THREADS * tp.sv, s.mul, s.ext, s.stepJ,
+                            s.corrJ, s.lim, s.offJ);
+}
+
+// Rank counts the kernels are instantiated for: tiles of 1..6 ranks run as
+// 2, 3, 4 or 6 (high ranks unused).
+inline int storeRankClass(int nTR) { return nTR <= 2 ? 2 : nTR <= 4 ? nTR : 6; }
+
+}  // namespace lt

@@ -23,10 +23,13 @@
 
 #include "group.h"
 #include "kernels.cuh"
+#include "slots.h"
 
 namespace lt {
 
-__device__ __forceinline__ void decodeTile(const TileParams& p, uint32_t tile, long long& bin,
+// P: TileParams or FlatParams (the same grid-rank fields).
+template <typename P>
+__device__ __forceinline__ void decodeTile(const P& p, uint32_t tile, long long& bin,
                                            long long& bout) {
   bin = 0;
   bout = 0;
@@ -51,40 +54,6 @@ __device__ __forceinline__ int opaque(int x) {
 
 __device__ __forceinline__ int smemIndex(const TileParams& p, int j) {
   return j + ((j >> p.padShift) << p.padLog);
-}
-
-// Table-free addressing for tiles of NTR ranks (1 <= NTR <= ARITH_MAX_NTR):
-// the global input offset of input-order element j of a tile, and the global
-// output offset and the input-order index of output-order element q, from
-// their mixed-radix digits.  In-tile indices are below 2^16 and extents at
-// least 2, so the digit __umulhi(x, ceil(2^32 / extent)) is exact
-// (ceil(2^32 / e) * x / 2^32 exceeds x / e by less than x / 2^32 < 1 / e).
-template <int NTR>
-__device__ __forceinline__ int arithInOffset(const TileParams& p, uint32_t j) {
-  int off = 0;
-#pragma unroll
-  for (int t = 0; t + 1 < NTR; ++t) {
-    const uint32_t q = __umulhi(j, p.trMul[t]);
-    off += (int)(j - q * (uint32_t)p.trE[t]) * p.trSin[t];
-    j = q;
-  }
-  return off + (int)j * p.trSin[NTR - 1];
-}
-
-template <int NTR>
-__device__ __forceinline__ void arithOut(const TileParams& p, uint32_t q, int& off, int& jj) {
-  off = 0;
-  jj = 0;
-#pragma unroll
-  for (int i = 0; i + 1 < NTR; ++i) {
-    const uint32_t d = __umulhi(q, p.toMul[i]);
-    const int c = (int)(q - d * (uint32_t)p.toE[i]);
-    off += c * p.toSout[i];
-    jj += c * p.toInTile[i];
-    q = d;
-  }
-  off += (int)q * p.toSout[NTR - 1];
-  jj += (int)q * p.toInTile[NTR - 1];
 }
 
 __device__ __forceinline__ void cpAsync16(uint32_t dst, const void* src) {
@@ -119,17 +88,11 @@ __device__ __forceinline__ void cpAsyncUnit(uint32_t dst, const void* src) {
                  : "memory");
 }
 
-// L2 prefetch size of the single-plan flat kernel's cp.async loads: none.
-// On the 200-problem float64 suite (three interleaved runs each, one box)
-// 256 bytes measured 0.2 % slower and 128 bytes the same as none.
-#ifndef LT_FLAT_L2_PREFETCH
-#define LT_FLAT_L2_PREFETCH 0
-#endif
-
-// L2 prefetch size of the grouped kernel's data copies: 0 (none), 128 or 256
-// bytes (the .L2::128B / .L2::256B qualifier of cp.async).  256: the
-// 10,000-member batch 0.3 % faster than none (two interleaved runs each, one
-// box); 128 made no difference.
+// L2 prefetch size of the grouped kernel's data copies: 0 (none) or 256
+// bytes (the .L2::256B qualifier of cp.async).  256: the 10,000-member batch
+// 0.3 % faster than none (two interleaved runs each, one box); 128 made no
+// difference.  The single-plan flat kernel uses none: on the 200-problem
+// float64 suite 256 bytes measured 0.2 % slower and 128 bytes the same.
 #ifndef LT_GROUP_L2_PREFETCH
 #define LT_GROUP_L2_PREFETCH 256
 #endif
@@ -328,76 +291,6 @@ __device__ __forceinline__ void storeTileFlat(const TileParams& p, const int* __
     storeUnit<ES, SV>(s, loadSmIdx<SV>(stSm, w), outBase + stOff[w]);
 }
 
-// Store unit at output-order element q (SV consecutive elements), global
-// offset off and first input-order index jj, addressed arithmetically: the
-// unit's elements step along output tile rank 0 unless the unit crosses it
-// (p.storeStraddle), then each element is decoded.
-template <int ES, int SV, int NTR>
-__device__ __forceinline__ void storeUnitArith(const TileParams& p,
-                                               const typename Word<ES>::T* s, uint32_t q,
-                                               int off, int jj, typename Word<ES>::T* outBase) {
-  using T = typename Word<ES>::T;
-  using ST = typename Word<ES * SV>::T;
-  if constexpr (SV == 1) {
-    outBase[off] = s[smemIndex(p, jj)];
-  } else {
-    T e[SV];
-    e[0] = s[smemIndex(p, jj)];
-    if (!p.storeStraddle) {
-#pragma unroll
-      for (int m = 1; m < SV; ++m) e[m] = s[smemIndex(p, jj + m * p.toInTile[0])];
-    } else {
-#pragma unroll
-      for (int m = 1; m < SV; ++m) {
-        int o2, j2;
-        arithOut<NTR>(p, q + m, o2, j2);
-        e[m] = s[smemIndex(p, j2)];
-      }
-    }
-    ST v;
-    __builtin_memcpy(&v, e, sizeof(ST));
-    *reinterpret_cast<ST*>(outBase + off) = v;
-  }
-}
-
-// Addresses of a thread's first PF store units (table-free addressing),
-// computed while the tile's loads are in flight.
-template <int NTR, int PF>
-struct ArithPrefetch {
-  int off[PF > 0 ? PF : 1];
-  int jj[PF > 0 ? PF : 1];
-
-  template <int SV>
-  __device__ __forceinline__ void load(const TileParams& p) {
-#pragma unroll
-    for (int i = 0; i < PF; ++i) {
-      const int w = threadIdx.x + i * TILE_THREADS;
-      if (w < p.nOut) arithOut<NTR>(p, (uint32_t)(w * SV), off[i], jj[i]);
-    }
-  }
-};
-
-// Store phase of the flat and bulk-copy pipelines with table-free
-// addressing: the prefetched units first, then the rest.
-template <int ES, int SV, int NTR, int PF>
-__device__ __forceinline__ void storeTileArith(const TileParams& p,
-                                               const ArithPrefetch<NTR, PF>& pf,
-                                               const typename Word<ES>::T* s,
-                                               typename Word<ES>::T* outBase) {
-#pragma unroll
-  for (int i = 0; i < PF; ++i) {
-    const int w = threadIdx.x + i * TILE_THREADS;
-    if (w < p.nOut) storeUnitArith<ES, SV, NTR>(p, s, (uint32_t)(w * SV), pf.off[i], pf.jj[i], outBase);
-  }
-  const int tv = opaque(threadIdx.x);
-#pragma unroll 4
-  for (int w = tv + PF * TILE_THREADS; w < p.nOut; w += TILE_THREADS) {
-    int off, jj;
-    arithOut<NTR>(p, (uint32_t)(w * SV), off, jj);
-    storeUnitArith<ES, SV, NTR>(p, s, (uint32_t)(w * SV), off, jj, outBase);
-  }
-}
-
 // Register-staged pipeline: load units go global -> registers -> shared
 // memory; the next tile's loads are issued before the current tile's
 // stores.  Two shared data buffers, one barrier per tile.
@@ -504,64 +397,254 @@ tileKernelAsync(const __grid_constant__ TileParams p, const typename Word<ES>::T
   cpAsyncWait<0>();
 }
 
-// Flat pipeline: one tile per CTA and no persistent loop, so the hardware
-// block scheduler streams tiles through the SMs in order.  With NTR = 0 the
-// offset tables were written at plan time and are read from device memory
-// (L1/L2-resident: every CTA of the launch reads the same few kilobytes);
-// with NTR = 1..ARITH_MAX_NTR (the tile's rank count) every unit's offsets
-// are computed from its index instead and the table pointers are unused.
-template <int ES, int LV, int SV, int NL, int NTR>
+// p + i * scale bytes.  With a scale the compiler cannot see (opaque), the
+// offset is one wide integer multiply-add on the FMA pipe instead of a
+// sign extension and a shift-add pair on the ALU pipe, which the grouped
+// kernel's narrow units would otherwise saturate.
+template <typename P>
+__device__ __forceinline__ P* offsetBytes(P* p, int i, int scale) {
+  using B = typename std::conditional<std::is_const<P>::value, const unsigned char,
+                                      unsigned char>::type;
+  return reinterpret_cast<P*>(reinterpret_cast<B*>(p) + (long long)i * scale);
+}
+
+// cp.async of one unit, issued only where live: the guard is a predicate on
+// the instruction rather than a branch around it (the compiler cannot
+// if-convert inline assembly, so a guarded asm costs a branch per slot).
+template <int BYTES, int PF>
+__device__ __forceinline__ void cpAsyncUnitIf(bool live, uint32_t dst, const void* src) {
+  static_assert(BYTES == 4 || BYTES == 8 || BYTES == 16, "cp.async unit");
+  static_assert(PF == 0 || PF == 256, "L2 prefetch size");
+#define LT_CP_ASYNC_IF(OP, SIZE)                                                             \
+  asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %2, 0;\n @p " OP " [%0], [%1], " SIZE \
+               ";\n}\n" ::"r"(dst),                                                          \
+               "l"(src), "r"((int)live)                                                      \
+               : "memory")
+  if constexpr (BYTES == 16 && PF == 256)
+    LT_CP_ASYNC_IF("cp.async.cg.shared.global.L2::256B", "16");
+  else if constexpr (BYTES == 16)
+    LT_CP_ASYNC_IF("cp.async.cg.shared.global", "16");
+  else if constexpr (BYTES == 8 && PF == 256)
+    LT_CP_ASYNC_IF("cp.async.ca.shared.global.L2::256B", "8");
+  else if constexpr (BYTES == 8)
+    LT_CP_ASYNC_IF("cp.async.ca.shared.global", "8");
+  else if constexpr (PF == 256)
+    LT_CP_ASYNC_IF("cp.async.ca.shared.global.L2::256B", "4");
+  else
+    LT_CP_ASYNC_IF("cp.async.ca.shared.global", "4");
+#undef LT_CP_ASYNC_IF
+}
+
+// Kernel parameters of a table-free tile (NTR rank class, NI load rank class;
+// the host builds them per launch from the plan's TileParams).
+template <int ES, int LV, int SV, int NL, int NI, int NTR>
+struct FlatParams {
+  static constexpr int NS = (NL * LV + SV - 1) / SV;  // store slots
+  int nIn, nOut, tileVol;
+  int padShiftB;     // shared byte address of byte x: x + (x >> padShiftB) * padBytes
+  int padBytes;
+  int ldSmStep;      // padded shared bytes between two load slots
+  int elemStep;      // shared bytes between the elements of a store unit
+  int storeStraddle; // a store unit's elements may cross output tile rank 0
+  int segLen, testExtraTx;  // as in TileParams
+  uint32_t statusTag;
+  LoadSlots<NL, NI> ld;
+  StoreSlots<NS, NTR> st;
+  int nGR;           // grid ranks, as in TileParams
+  FastDiv grDiv[MAXR];
+  long long grSin[MAXR], grSout[MAXR], grLastIn[MAXR], grLastOut[MAXR];
+};
+
+template <int ES, int LV, int SV, int NL, int NI, int NTR>
+FlatParams<ES, LV, SV, NL, NI, NTR> makeFlatParams(const TileParams& tp) {
+  FlatParams<ES, LV, SV, NL, NI, NTR> p;
+  p.nIn = tp.nIn;
+  p.nOut = tp.nOut;
+  p.tileVol = tp.tileVol;
+  // in-tile byte indices are below 2^20: shift 31 gives no padding
+  p.padShiftB = tp.padShift >= PAD_NONE ? 31 : tp.padShift + (ES == 4 ? 2 : ES == 8 ? 3 : 4);
+  p.padBytes = ES << tp.padLog;
+  constexpr int B = TILE_THREADS * LV;  // a multiple of every padding period (2^2 .. 2^8)
+  p.ldSmStep = B * ES + (tp.padShift >= PAD_NONE ? 0 : (B >> tp.padShift) * p.padBytes);
+  p.elemStep = tp.toInTile[0] * ES;
+  p.storeStraddle = tp.storeStraddle;
+  p.segLen = tp.segLen;
+  p.testExtraTx = tp.testExtraTx;
+  p.statusTag = tp.statusTag;
+  makeLoadSlots(tp, p.ld);
+  makeStoreSlots(tp, ES, p.st);
+  p.nGR = tp.nGR;
+  for (int g = 0; g < tp.nGR; ++g) {
+    p.grDiv[g] = tp.grDiv[g];
+    p.grSin[g] = tp.grSin[g];
+    p.grSout[g] = tp.grSout[g];
+    p.grLastIn[g] = tp.grLastIn[g];
+    p.grLastOut[g] = tp.grLastOut[g];
+  }
+  return p;
+}
+
+template <typename P>
+__device__ __forceinline__ uint32_t padByte(const P& p, uint32_t x) {
+  return x + (x >> p.padShiftB) * (uint32_t)p.padBytes;
+}
+
+// A thread's part of the store addresses, decoded while the loads are in
+// flight.
+template <int NTR>
+struct StoreThread {
+  uint32_t off, j;
+  int d[NTR - 1];
+};
+
+// Store phase of the table-free flat and bulk-copy kernels.  Slots go in
+// chunks of four, whole chunks without a guard.
+template <int ES, int LV, int SV, int NL, int NI, int NTR>
+__device__ __forceinline__ void storeTileSlots(const FlatParams<ES, LV, SV, NL, NI, NTR>& p,
+                                               const StoreThread<NTR>& t,
+                                               const unsigned char* s,
+                                               typename Word<ES>::T* outBase) {
+  using T = typename Word<ES>::T;
+  using ST = typename Word<ES * SV>::T;
+  constexpr int NS = FlatParams<ES, LV, SV, NL, NI, NTR>::NS;
+  constexpr int CH = NS < 4 ? NS : 4;
+  const int wMax = p.nOut - (int)threadIdx.x;
+  const int esR = opaque(ES);
+  auto slot = [&](int k) {
+    uint32_t off, j;
+    storeSlotOffset<NS, NTR>(p.st, k, t.off, t.j, t.d, off, j);
+    T e[SV];
+    e[0] = *reinterpret_cast<const T*>(s + padByte(p, j));
+    if constexpr (SV > 1) {
+      if (!p.storeStraddle) {
+#pragma unroll
+        for (int m = 1; m < SV; ++m)
+          e[m] = *reinterpret_cast<const T*>(s + padByte(p, j + (uint32_t)(m * p.elemStep)));
+      } else {
+#pragma unroll
+        for (int m = 1; m < SV; ++m) {
+          StoreThread<NTR> u;
+          storeThreadOffset<NS, NTR>(
+              p.st, (uint32_t)((threadIdx.x + k * TILE_THREADS) * SV + m), u.d, u.off, u.j);
+          e[m] = *reinterpret_cast<const T*>(s + padByte(p, u.j));
+        }
+      }
+    }
+    ST v;
+    __builtin_memcpy(&v, e, sizeof(ST));
+    *reinterpret_cast<ST*>(offsetBytes(outBase, (int)off, esR)) = v;
+  };
+#pragma unroll
+  for (int k0 = 0; k0 < NS; k0 += CH) {
+    if ((k0 + CH) * TILE_THREADS <= p.nOut) {
+#pragma unroll
+      for (int i = 0; i < CH; ++i) slot(k0 + i);
+    } else if (k0 * TILE_THREADS < p.nOut) {
+#pragma unroll
+      for (int i = 0; i < CH; ++i)
+        if ((k0 + i) * TILE_THREADS < wMax) slot(k0 + i);
+    }
+  }
+}
+
+// Flat pipeline, tiles of at most ARITH_MAX_NTR ranks: one tile per CTA and
+// no persistent loop, so the hardware block scheduler streams tiles through
+// the SMs in order.  Unit addresses come from the slot sums (slots.h).
+template <int ES, int LV, int SV, int NL, int NI, int NTR>
 __global__ void __launch_bounds__(TILE_THREADS)
-tileKernelFlat(const __grid_constant__ TileParams p, const typename Word<ES>::T* __restrict__ in,
-               typename Word<ES>::T* __restrict__ out, const int* __restrict__ ldOff,
-               const int* __restrict__ stOff, const unsigned short* __restrict__ stSm) {
+tileKernelFlat(const __grid_constant__ FlatParams<ES, LV, SV, NL, NI, NTR> p,
+               const typename Word<ES>::T* __restrict__ in, typename Word<ES>::T* __restrict__ out) {
+  using LT = typename Word<ES * LV>::T;
+  extern __shared__ __align__(16) unsigned char smraw[];
+  long long bin, bout;
+  decodeTile(p, blockIdx.x, bin, bout);
+  const uint32_t jT = threadIdx.x * LV;
+  int d[NI - 1];
+  const uint32_t offT = loadThreadOffset<NL, NI>(p.ld, jT, d);
+  const auto* src = in + bin;
+  const int esR = opaque(ES);
+  const int uMax = p.nIn - (int)threadIdx.x;
+  const uint32_t dst0 = padByte(p, jT * ES);
+  auto source = [&](int k) {
+    return offsetBytes(src, (int)loadSlotOffset<NL, NI>(p.ld, k, offT, d), esR);
+  };
+  StoreThread<NTR> t;
+  if constexpr (NL >= flatAsyncMinNL<ES>()) {
+    // many load units per thread: cp.async straight into shared memory
+    // instead of NL data registers per thread
+    const uint32_t sBase = (uint32_t)__cvta_generic_to_shared(smraw) + dst0;
+    constexpr int CH = 4;
+#pragma unroll
+    for (int k0 = 0; k0 < NL; k0 += CH) {
+      if ((k0 + CH) * TILE_THREADS <= p.nIn) {
+#pragma unroll
+        for (int k = k0; k < k0 + CH; ++k)
+          cpAsyncUnit<ES * LV>(sBase + (uint32_t)(k * p.ldSmStep), source(k));
+      } else if (k0 * TILE_THREADS < p.nIn) {
+#pragma unroll
+        for (int k = k0; k < k0 + CH; ++k)
+          cpAsyncUnitIf<ES * LV, 0>(k * TILE_THREADS < uMax, sBase + (uint32_t)(k * p.ldSmStep),
+                                    source(k));
+      }
+    }
+    storeThreadOffset<FlatParams<ES, LV, SV, NL, NI, NTR>::NS, NTR>(p.st, threadIdx.x * SV, t.d,
+                                                                    t.off, t.j);
+    cpAsyncWaitAll();
+  } else {
+    LT v[NL];
+#pragma unroll
+    for (int k = 0; k < NL; ++k)
+      if (k * TILE_THREADS < uMax) v[k] = *reinterpret_cast<const LT*>(source(k));
+    storeThreadOffset<FlatParams<ES, LV, SV, NL, NI, NTR>::NS, NTR>(p.st, threadIdx.x * SV, t.d,
+                                                                    t.off, t.j);
+#pragma unroll
+    for (int k = 0; k < NL; ++k)
+      if (k * TILE_THREADS < uMax)
+        *reinterpret_cast<LT*>(smraw + dst0 + (uint32_t)(k * p.ldSmStep)) = v[k];
+  }
+  __syncthreads();
+  storeTileSlots<ES, LV, SV, NL, NI, NTR>(p, t, smraw, out + bout);
+}
+
+// The flat pipeline for larger tiles: the offset tables were written at plan
+// time and are read from device memory (L1/L2-resident: every CTA of the
+// launch reads the same few kilobytes).
+template <int ES, int LV, int SV, int NL>
+__global__ void __launch_bounds__(TILE_THREADS)
+tileKernelTables(const __grid_constant__ TileParams p, const typename Word<ES>::T* __restrict__ in,
+                 typename Word<ES>::T* __restrict__ out, const int* __restrict__ ldOff,
+                 const int* __restrict__ stOff, const unsigned short* __restrict__ stSm) {
   using T = typename Word<ES>::T;
   using LT = typename Word<ES * LV>::T;
   extern __shared__ __align__(16) unsigned char smraw[];
   T* s = reinterpret_cast<T*>(smraw);
   long long bin, bout;
   decodeTile(p, blockIdx.x, bin, bout);
-  auto ldOffset = [&](int u) -> int {
-    if constexpr (NTR > 0)
-      return arithInOffset<NTR>(p, (uint32_t)(u * LV));
-    else
-      return __ldg(ldOff + u);
-  };
   // store units per thread: nOut <= NL * TILE_THREADS * LV / SV; up to two
   // are prefetched, except where the register pipeline already holds
-  // NL >= 4 data words (measured slower there: C3b 2 % down)
+  // NL >= 4 data words (measured slower there)
   constexpr int NS = (NL * LV + SV - 1) / SV;
   constexpr int PF_MAX = (NL >= flatAsyncMinNL<ES>() || NL < 4) ? 2 : 0;
   constexpr int PF = NS < PF_MAX ? NS : PF_MAX;
-  StorePrefetch<SV, (NTR == 0 ? PF : 0)> pf;
-  ArithPrefetch<NTR, (NTR > 0 ? PF : 0)> apf;
-  auto prefetch = [&] {
-    if constexpr (NTR > 0)
-      apf.template load<SV>(p);
-    else
-      pf.load(p, stOff, stSm);
-  };
+  StorePrefetch<SV, PF> pf;
   if constexpr (NL >= flatAsyncMinNL<ES>()) {
-    // many load units per thread: cp.async straight into shared memory
-    // instead of NL data registers per thread
     const uint32_t sBase = (uint32_t)__cvta_generic_to_shared(s);
 #pragma unroll
     for (int k = 0; k < NL; ++k) {
       const int u = threadIdx.x + k * TILE_THREADS;
       if (u < p.nIn)
-        cpAsyncUnit<ES * LV, LT_FLAT_L2_PREFETCH>(sBase + (uint32_t)smemIndex(p, u * LV) * ES,
-                                                 in + bin + ldOffset(u));
+        cpAsyncUnit<ES * LV>(sBase + (uint32_t)smemIndex(p, u * LV) * ES, in + bin + __ldg(ldOff + u));
     }
-    prefetch();
+    pf.load(p, stOff, stSm);
     cpAsyncWaitAll();
   } else {
     LT v[NL];
 #pragma unroll
     for (int k = 0; k < NL; ++k) {
       const int u = threadIdx.x + k * TILE_THREADS;
-      if (u < p.nIn) v[k] = *reinterpret_cast<const LT*>(in + bin + ldOffset(u));
+      if (u < p.nIn) v[k] = *reinterpret_cast<const LT*>(in + bin + __ldg(ldOff + u));
     }
-    prefetch();
+    pf.load(p, stOff, stSm);
 #pragma unroll
     for (int k = 0; k < NL; ++k) {
       const int u = threadIdx.x + k * TILE_THREADS;
@@ -569,10 +652,7 @@ tileKernelFlat(const __grid_constant__ TileParams p, const typename Word<ES>::T*
     }
   }
   __syncthreads();
-  if constexpr (NTR > 0)
-    storeTileArith<ES, SV>(p, apf, s, out + bout);
-  else
-    storeTileFlat<ES, SV>(p, stOff, stSm, pf, s, out + bout);
+  storeTileFlat<ES, SV>(p, stOff, stSm, pf, s, out + bout);
 }
 
 // mbarrier and bulk-copy primitives (PTX ISA: mbarrier, cp.async.bulk).
@@ -644,21 +724,12 @@ constexpr unsigned long long BULK_WAIT_NS = 1000000000ull;  // 1 s
 // BULK_WAIT_NS without completion the CTA writes the plan's tag p.statusTag
 // to *status, waits once more (bounded) for its copies in flight, and
 // returns without storing.
-template <int ES, int LV, int SV, int NL, int NTR>
-__global__ void __launch_bounds__(TILE_THREADS)
-tileKernelBulk(const __grid_constant__ TileParams p, const typename Word<ES>::T* __restrict__ in,
-               typename Word<ES>::T* __restrict__ out, const int* __restrict__ ldOff,
-               const int* __restrict__ stOff, const unsigned short* __restrict__ stSm,
-               unsigned* status) {
-  static_assert(ES * LV == 16, "bulk copies need 16-byte load units");
-  using T = typename Word<ES>::T;
-  extern __shared__ __align__(16) unsigned char smraw[];
-  __shared__ __align__(8) unsigned long long bar;
-  T* s = reinterpret_cast<T*>(smraw);
-  long long bin, bout;
-  decodeTile(p, blockIdx.x, bin, bout);
-  const uint32_t mb = (uint32_t)__cvta_generic_to_shared(&bar);
-  const uint32_t sBase = (uint32_t)__cvta_generic_to_shared(s);
+// Issue half of the bulk-copy kernels: `off` gives a tile element's global
+// input offset, `pad` its shared byte address.  Returns after the copies are
+// issued and the mbarrier is armed.
+template <int ES, typename P, typename Off, typename Pad>
+__device__ __forceinline__ void bulkIssue(const P& p, const typename Word<ES>::T* src,
+                                          uint32_t sBase, uint32_t mb, Off off, Pad pad) {
   if (threadIdx.x == 0) {
     mbarInit(mb, 1);
     mbarInitFence();
@@ -667,73 +738,73 @@ tileKernelBulk(const __grid_constant__ TileParams p, const typename Word<ES>::T*
   const int L = p.segLen;
   const int nSeg = p.tileVol / L;
   const uint32_t segBytes = (uint32_t)(L * ES);
-  const T* src = in + bin;
   for (int k = threadIdx.x; k < nSeg; k += TILE_THREADS) {
     const int j0 = k * L;
-    int off;
-    if constexpr (NTR > 0)
-      off = arithInOffset<NTR>(p, (uint32_t)j0);
-    else
-      off = __ldg(ldOff + j0 / LV);
-    bulkLoad(sBase + (uint32_t)smemIndex(p, j0) * ES, src + off, segBytes, mb);
+    bulkLoad(sBase + pad(j0), src + off(j0), segBytes, mb);
   }
   if (threadIdx.x == 0) mbarArriveExpectTx(mb, (uint32_t)nSeg * segBytes + (uint32_t)p.testExtraTx);
+}
+
+// Wait half: false after the time limit, with the plan's tag in *status.
+template <typename P>
+__device__ __forceinline__ bool bulkWait(const P& p, uint32_t mb, unsigned* status) {
+  if (mbarWaitBounded(mb, 0, BULK_WAIT_NS)) return true;
+  if (threadIdx.x == 0) atomicExch(status, p.statusTag);
+  mbarWaitBounded(mb, 0, BULK_WAIT_NS);  // copies in flight write this CTA's shared memory
+  return false;
+}
+
+template <int ES, int LV, int SV, int NL, int NI, int NTR>
+__global__ void __launch_bounds__(TILE_THREADS)
+tileKernelBulk(const __grid_constant__ FlatParams<ES, LV, SV, NL, NI, NTR> p,
+               const typename Word<ES>::T* __restrict__ in, typename Word<ES>::T* __restrict__ out,
+               unsigned* status) {
+  static_assert(ES * LV == 16, "bulk copies need 16-byte load units");
+  extern __shared__ __align__(16) unsigned char smraw[];
+  __shared__ __align__(8) unsigned long long bar;
+  long long bin, bout;
+  decodeTile(p, blockIdx.x, bin, bout);
+  const uint32_t mb = (uint32_t)__cvta_generic_to_shared(&bar);
+  bulkIssue<ES>(
+      p, in + bin, (uint32_t)__cvta_generic_to_shared(smraw), mb,
+      [&](int j) {
+        int d[NI - 1];
+        return (int)loadThreadOffset<NL, NI>(p.ld, (uint32_t)j, d);
+      },
+      [&](int j) { return padByte(p, (uint32_t)(j * ES)); });
+  StoreThread<NTR> t;
+  storeThreadOffset<FlatParams<ES, LV, SV, NL, NI, NTR>::NS, NTR>(p.st, threadIdx.x * SV, t.d,
+                                                                  t.off, t.j);
+  if (!bulkWait(p, mb, status)) return;
+  storeTileSlots<ES, LV, SV, NL, NI, NTR>(p, t, smraw, out + bout);
+}
+
+// Bulk copies with offset tables (tiles of more than ARITH_MAX_NTR ranks).
+template <int ES, int LV, int SV, int NL>
+__global__ void __launch_bounds__(TILE_THREADS)
+tileKernelBulkTables(const __grid_constant__ TileParams p,
+                     const typename Word<ES>::T* __restrict__ in,
+                     typename Word<ES>::T* __restrict__ out, const int* __restrict__ ldOff,
+                     const int* __restrict__ stOff, const unsigned short* __restrict__ stSm,
+                     unsigned* status) {
+  static_assert(ES * LV == 16, "bulk copies need 16-byte load units");
+  using T = typename Word<ES>::T;
+  extern __shared__ __align__(16) unsigned char smraw[];
+  __shared__ __align__(8) unsigned long long bar;
+  T* s = reinterpret_cast<T*>(smraw);
+  long long bin, bout;
+  decodeTile(p, blockIdx.x, bin, bout);
+  const uint32_t mb = (uint32_t)__cvta_generic_to_shared(&bar);
+  bulkIssue<ES>(
+      p, in + bin, (uint32_t)__cvta_generic_to_shared(s), mb,
+      [&](int j) { return __ldg(ldOff + j / LV); },
+      [&](int j) { return (uint32_t)smemIndex(p, j) * ES; });
   constexpr int NS = (NL * LV + SV - 1) / SV;
   constexpr int PF = NS < 2 ? NS : 2;
-  StorePrefetch<SV, (NTR == 0 ? PF : 0)> pf;
-  ArithPrefetch<NTR, (NTR > 0 ? PF : 0)> apf;
-  if constexpr (NTR > 0)
-    apf.template load<SV>(p);
-  else
-    pf.load(p, stOff, stSm);
-  if (!mbarWaitBounded(mb, 0, BULK_WAIT_NS)) {
-    if (threadIdx.x == 0) atomicExch(status, p.statusTag);
-    mbarWaitBounded(mb, 0, BULK_WAIT_NS);  // copies in flight write this CTA's shared memory
-    return;
-  }
-  if constexpr (NTR > 0)
-    storeTileArith<ES, SV>(p, apf, s, out + bout);
-  else
-    storeTileFlat<ES, SV>(p, stOff, stSm, pf, s, out + bout);
-}
-
-// p + i * scale bytes.  With a scale the compiler cannot see (opaque), the
-// offset is one wide integer multiply-add on the FMA pipe instead of a
-// sign extension and a shift-add pair on the ALU pipe, which the grouped
-// kernel's narrow units would otherwise saturate.
-template <typename P>
-__device__ __forceinline__ P* offsetBytes(P* p, int i, int scale) {
-  using B = typename std::conditional<std::is_const<P>::value, const unsigned char,
-                                      unsigned char>::type;
-  return reinterpret_cast<P*>(reinterpret_cast<B*>(p) + (long long)i * scale);
-}
-
-// cp.async of one unit, issued only where live: the guard is a predicate on
-// the instruction rather than a branch around it (the compiler cannot
-// if-convert inline assembly, so a guarded asm costs a branch per slot).
-template <int BYTES>
-__device__ __forceinline__ void cpAsyncUnitIf(bool live, uint32_t dst, const void* src) {
-  static_assert(BYTES == 4 || BYTES == 8 || BYTES == 16, "cp.async unit");
-#if LT_GROUP_L2_PREFETCH == 256
-#define LT_GROUP_PF ".L2::256B"
-#elif LT_GROUP_L2_PREFETCH == 128
-#define LT_GROUP_PF ".L2::128B"
-#else
-#define LT_GROUP_PF ""
-#endif
-  if constexpr (BYTES == 16)
-    asm volatile(
-        "{\n .reg .pred p;\n setp.ne.b32 p, %2, 0;\n"
-        " @p cp.async.cg.shared.global" LT_GROUP_PF " [%0], [%1], 16;\n}\n" ::"r"(dst),
-        "l"(src), "r"((int)live)
-        : "memory");
-  else
-    asm volatile(
-        "{\n .reg .pred p;\n setp.ne.b32 p, %3, 0;\n"
-        " @p cp.async.ca.shared.global" LT_GROUP_PF " [%0], [%1], %2;\n}\n" ::"r"(dst),
-        "l"(src), "n"(BYTES), "r"((int)live)
-        : "memory");
-#undef LT_GROUP_PF
+  StorePrefetch<SV, PF> pf;
+  pf.load(p, stOff, stSm);
+  if (!bulkWait(p, mb, status)) return;
+  storeTileFlat<ES, SV>(p, stOff, stSm, pf, s, out + bout);
 }
 
 // Shared load where live (predicated as above); the result is undefined
@@ -860,7 +931,7 @@ __device__ __forceinline__ void groupTileBody(const GroupTensor* __restrict__ te
 #pragma unroll
         for (int k = 0; k < NL; ++k)
           if constexpr (STEP)  // the source is arithmetic only: predicate the copy
-            cpAsyncUnitIf<ES * LV>(k * TILE_THREADS < uMax, dst0 + (uint32_t)(k * stepBytes),
+            cpAsyncUnitIf<ES * LV, LT_GROUP_L2_PREFETCH>(k * TILE_THREADS < uMax, dst0 + (uint32_t)(k * stepBytes),
                                    unitSrc(k));
           else if (k * TILE_THREADS < uMax)  // a dead slot's run would index past ldRow
             cpAsyncUnit<ES * LV>(dst0 + (uint32_t)(k * stepBytes), unitSrc(k));
