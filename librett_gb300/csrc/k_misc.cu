@@ -81,8 +81,7 @@ cudaError_t launchCopy(const void* in, void* out, long long n, cudaStream_t s, i
   const long long g = (n + per - 1) / per;
   if (g < 1 || g > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
   *grid = (int)g;
-  copyKernel<US><<<(unsigned)g, COPY_THREADS, 0, s>>>((const T*)in, (T*)out, n);
-  return cudaGetLastError();
+  return launchDependent(copyKernel<US>, (unsigned)g, COPY_THREADS, 0, s, (const T*)in, (T*)out, n);
 }
 
 template <int US>
@@ -91,8 +90,8 @@ cudaError_t launchRows(const RowParams& rp, const void* in, void* out, cudaStrea
   const long long g = ((long long)rp.numItems + ROW_ITEMS_PER_CTA - 1) / ROW_ITEMS_PER_CTA;
   if (g < 1) return cudaErrorInvalidConfiguration;
   *grid = (int)g;
-  rowCopyKernel<US><<<(unsigned)g, ROW_THREADS, 0, s>>>(rp, (const T*)in, (T*)out);
-  return cudaGetLastError();
+  return launchDependent(rowCopyKernel<US>, (unsigned)g, ROW_THREADS, 0, s, rp, (const T*)in,
+                         (T*)out);
 }
 
 cudaError_t launchCopyUnit(int unit, const void* in, void* out, long long n, cudaStream_t s,

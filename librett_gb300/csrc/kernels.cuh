@@ -25,6 +25,60 @@ __device__ __forceinline__ uint32_t fdiv(uint32_t n, const FastDiv& f) {
   return (uint32_t)(((unsigned long long)n * f.mul) >> f.shift);
 }
 
+// Programmatic dependent launch: a kernel launched by launchDependent may
+// start while the stream's previous kernel is still draining, so its launch
+// latency and address decode overlap that kernel's tail.  It must call
+// dependencyWait before its first access to global memory (which returns when
+// every earlier kernel has completed and its writes are visible; at once for
+// an ordinary launch) and calls dependencyRelease first, which lets its own
+// successor do the same as soon as all its CTAs run.  Loads that the compiler
+// may treat as invariant (const __restrict__ pointers) can be moved above the
+// wait, so such kernels load through ldGlobal.
+__device__ __forceinline__ void dependencyRelease() {
+  asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+}
+
+__device__ __forceinline__ void dependencyWait() {
+  asm volatile("griddepcontrol.wait;\n" ::: "memory");
+}
+
+template <int BYTES>
+__device__ __forceinline__ typename Word<BYTES>::T ldGlobal(const void* p) {
+  typename Word<BYTES>::T v;
+  if constexpr (BYTES == 4)
+    asm volatile("ld.global.nc.b32 %0, [%1];\n" : "=r"(v) : "l"(p) : "memory");
+  else if constexpr (BYTES == 8)
+    asm volatile("ld.global.nc.v2.b32 {%0, %1}, [%2];\n" : "=r"(v.x), "=r"(v.y) : "l"(p) : "memory");
+  else
+    asm volatile("ld.global.nc.v4.b32 {%0, %1, %2, %3}, [%4];\n"
+                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+                 : "l"(p)
+                 : "memory");
+  return v;
+}
+
+// Launches fn with programmatic stream serialization; as an ordinary launch
+// while s is being captured, so a caller's graph keeps its plain edges.
+template <typename... Params, typename... Args>
+cudaError_t launchDependent(void (*fn)(Params...), unsigned grid, unsigned threads, size_t smem,
+                            cudaStream_t s, const Args&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr = {};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone) {
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+  }
+  cudaLaunchKernelEx(&cfg, fn, Params(args)...);
+  return cudaGetLastError();
+}
+
 // ---------------------------------------------------------------------------
 // Trivial: contiguous copy in units of US bytes.  Each CTA copies one block
 // of COPY_THREADS * COPY_UNROLL units (four independent loads per thread,
@@ -40,9 +94,11 @@ copyKernel(const typename Word<US>::T* __restrict__ in, typename Word<US>::T* __
   using T = typename Word<US>::T;
   const long long base = (long long)blockIdx.x * (COPY_THREADS * COPY_UNROLL) + threadIdx.x;
   T v[COPY_UNROLL];
+  dependencyRelease();
+  dependencyWait();
 #pragma unroll
   for (int u = 0; u < COPY_UNROLL; ++u)
-    if (base + u * COPY_THREADS < n) v[u] = in[base + u * COPY_THREADS];
+    if (base + u * COPY_THREADS < n) v[u] = ldGlobal<US>(in + base + u * COPY_THREADS);
 #pragma unroll
   for (int u = 0; u < COPY_UNROLL; ++u)
     if (base + u * COPY_THREADS < n) out[base + u * COPY_THREADS] = v[u];
@@ -66,8 +122,9 @@ rowCopyKernel(const __grid_constant__ RowParams p, const typename Word<US>::T* _
   const uint32_t first =
       blockIdx.x * ROW_ITEMS_PER_CTA + (threadIdx.x >> 5) * ROW_ITEMS_PER_WARP;
   T v[ROW_ITEMS_PER_WARP];
-  long long dst[ROW_ITEMS_PER_WARP];
+  long long src[ROW_ITEMS_PER_WARP], dst[ROW_ITEMS_PER_WARP];
   bool ok[ROW_ITEMS_PER_WARP];
+  dependencyRelease();
 #pragma unroll
   for (int u = 0; u < ROW_ITEMS_PER_WARP; ++u) {
     const uint32_t item = first + u;
@@ -86,11 +143,15 @@ rowCopyKernel(const __grid_constant__ RowParams p, const typename Word<US>::T* _
       }
       if (col < p.rowUnits) {
         ok[u] = true;
-        v[u] = in[bi + col];
+        src[u] = bi + col;
         dst[u] = bo + col;
       }
     }
   }
+  dependencyWait();
+#pragma unroll
+  for (int u = 0; u < ROW_ITEMS_PER_WARP; ++u)
+    if (ok[u]) v[u] = ldGlobal<US>(in + src[u]);
 #pragma unroll
   for (int u = 0; u < ROW_ITEMS_PER_WARP; ++u)
     if (ok[u]) out[dst[u]] = v[u];

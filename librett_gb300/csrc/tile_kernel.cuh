@@ -556,6 +556,7 @@ tileKernelFlat(const __grid_constant__ FlatParams<ES, LV, SV, NL, NI, NTR> p,
                const typename Word<ES>::T* __restrict__ in, typename Word<ES>::T* __restrict__ out) {
   using LT = typename Word<ES * LV>::T;
   extern __shared__ __align__(16) unsigned char smraw[];
+  dependencyRelease();
   long long bin, bout;
   decodeTile(p, blockIdx.x, bin, bout);
   const uint32_t jT = threadIdx.x * LV;
@@ -569,6 +570,7 @@ tileKernelFlat(const __grid_constant__ FlatParams<ES, LV, SV, NL, NI, NTR> p,
     return offsetBytes(src, (int)loadSlotOffset<NL, NI>(p.ld, k, offT, d), esR);
   };
   StoreThread<NTR> t;
+  dependencyWait();
   if constexpr (NL >= flatAsyncMinNL<ES>()) {
     // many load units per thread: cp.async straight into shared memory
     // instead of NL data registers per thread
@@ -594,7 +596,7 @@ tileKernelFlat(const __grid_constant__ FlatParams<ES, LV, SV, NL, NI, NTR> p,
     LT v[NL];
 #pragma unroll
     for (int k = 0; k < NL; ++k)
-      if (k * TILE_THREADS < uMax) v[k] = *reinterpret_cast<const LT*>(source(k));
+      if (k * TILE_THREADS < uMax) v[k] = ldGlobal<ES * LV>(source(k));
     storeThreadOffset<FlatParams<ES, LV, SV, NL, NI, NTR>::NS, NTR>(p.st, threadIdx.x * SV, t.d,
                                                                     t.off, t.j);
 #pragma unroll
@@ -735,6 +737,7 @@ __device__ __forceinline__ void bulkIssue(const P& p, const typename Word<ES>::T
     mbarInitFence();
   }
   __syncthreads();
+  dependencyWait();
   const int L = p.segLen;
   const int nSeg = p.tileVol / L;
   const uint32_t segBytes = (uint32_t)(L * ES);
@@ -762,6 +765,7 @@ tileKernelBulk(const __grid_constant__ FlatParams<ES, LV, SV, NL, NI, NTR> p,
   static_assert(ES * LV == 16, "bulk copies need 16-byte load units");
   extern __shared__ __align__(16) unsigned char smraw[];
   __shared__ __align__(8) unsigned long long bar;
+  dependencyRelease();
   long long bin, bout;
   decodeTile(p, blockIdx.x, bin, bout);
   const uint32_t mb = (uint32_t)__cvta_generic_to_shared(&bar);
