@@ -222,7 +222,8 @@ int librett_c_group_create_policy(librettGroupHandle* group, int count,
                                   const librettHandle* plans, void* const* idata,
                                   void* const* odata, void* stream, const int* policy);
 int librett_c_group_tune(librettGroupHandle group);
-/* Bucket `index` (launch order) of the group's graph: shape[6] = element
+/* Bucket `index` of the group's graph, in launch order (the small ones that
+ * share the mixed launch last): shape[6] = element
  * bytes, load unit, store unit (elements), load units per thread, dynamic
  * shared memory bytes, loads (0/1/2 as in the policy); its members, tiles
  * and algorithmic bytes. */
@@ -256,6 +257,18 @@ int librett_c_group_run_check(int rank, const int* dim, const int* permutation, 
 int librett_c_slot_check(int rank, const int* dim, const int* permutation, size_t sizeofType,
                          int num_sms, int candidate, int element_units);
 
+/* Host-only self-check of the mixed launch's box addressing for flat-tile
+ * candidate `candidate`: variant 0 its tile, 1 in element units, 2 with extents
+ * and units widened as a group does, 3 doubled.  Replays every thread and slot
+ * of a CTA: each element of the tile must be loaded once into shared memory,
+ * aligned and in bounds, and stored once where it belongs.  Returns
+ * LIBRETT_SUCCESS when they are, LIBRETT_INTERNAL_ERROR on a violation,
+ * LIBRETT_INVALID_DEVICE when the tile has no box (its bucket then keeps its
+ * own launch) or its units cross a run, LIBRETT_INVALID_PARAMETER for a bad
+ * problem, candidate or variant. */
+int librett_c_group_box_check(int rank, const int* dim, const int* permutation, size_t sizeofType,
+                              int num_sms, int candidate, int variant);
+
 /* Host-only self-check of the bulk-copy pipeline for candidate `candidate`
  * of the planner's candidate list (candidate set 1): every segment the
  * kernel copies with one cp.async.bulk must be contiguous in global memory
@@ -286,7 +299,7 @@ int librett_c_plan_batch(int count, const int* ranks, const int* dims, const int
  * the first error. */
 int librett_c_execute_batch(int count, const librettHandle* plans, void* const* idata,
                             void* const* odata);
-/* members, buckets (launches), members run separately, tiles, algorithmic bytes */
+/* members, launches (the large buckets' and the mixed one), members run separately, tiles, algorithmic bytes */
 int librett_c_group_info(librettGroupHandle group, int* members, int* buckets, int* separate,
                          long long* tiles, long long* bytes);
 

@@ -152,14 +152,17 @@ class Group:
             raise LibrettError(rc, "librett_c_group_tune")
 
     def buckets(self) -> list[dict]:
-        """The graph's bucket launches in launch order."""
+        """The graph's buckets in launch order (several small ones may share
+        one mixed launch, so there can be more than info()["buckets"])."""
         out = []
         lib = _lib.load()
-        for b in range(self.info()["buckets"]):
+        while True:
             shape = (ctypes.c_int * 6)()
             m, t, by = ctypes.c_int(), ctypes.c_longlong(), ctypes.c_longlong()
-            rc = lib.librett_c_group_bucket(self.handle, b, shape, ctypes.byref(m), ctypes.byref(t),
-                                            ctypes.byref(by))
+            rc = lib.librett_c_group_bucket(self.handle, len(out), shape, ctypes.byref(m),
+                                            ctypes.byref(t), ctypes.byref(by))
+            if rc == LIBRETT_INVALID_PARAMETER:
+                break
             if rc != LIBRETT_SUCCESS:
                 raise LibrettError(rc, "librett_c_group_bucket")
             out.append({"es": shape[0], "lv": shape[1], "sv": shape[2], "nl": shape[3],

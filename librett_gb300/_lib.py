@@ -141,6 +141,12 @@ C_FUNCTIONS = [
     ("librett_c_slot_check", ctypes.c_int,
      [ctypes.c_int, ctypes.POINTER(ctypes.c_int), ctypes.POINTER(ctypes.c_int), ctypes.c_size_t,
       ctypes.c_int, ctypes.c_int, ctypes.c_int]),
+    ("librett_c_group_box_check", ctypes.c_int,
+     [ctypes.c_int, ctypes.POINTER(ctypes.c_int), ctypes.POINTER(ctypes.c_int), ctypes.c_size_t,
+      ctypes.c_int, ctypes.c_int, ctypes.c_int]),
+    ("librett_c_slot_check", ctypes.c_int,
+     [ctypes.c_int, ctypes.POINTER(ctypes.c_int), ctypes.POINTER(ctypes.c_int), ctypes.c_size_t,
+      ctypes.c_int, ctypes.c_int, ctypes.c_int]),
     ("librett_c_bulk_check", ctypes.c_int,
      [ctypes.c_int, ctypes.POINTER(ctypes.c_int), ctypes.POINTER(ctypes.c_int), ctypes.c_size_t,
       ctypes.c_int, ctypes.c_int]),

@@ -19,6 +19,7 @@
 #include <unordered_map>
 #include <vector>
 
+#include "box.h"
 #include "fault.h"
 #include "launch.h"
 #include "librett.h"
@@ -620,6 +621,101 @@ int librett_c_slot_check(int rank, const int* dim, const int* permutation, size_
     default: ok = few ? go(slotsMatch<2, 6>) : go(slotsMatch<6, 6>); break;
   }
   return ok ? LIBRETT_SUCCESS : LIBRETT_INTERNAL_ERROR;
+}
+
+}  // extern "C"
+
+namespace {
+
+// Replays box addressing on the host: every unit a thread and slot load must
+// be a unit of the tile, every element must arrive in shared memory exactly
+// once, at an address inside the allocation and aligned to its unit, and
+// every unit stored must gather the elements that its output offset names.
+bool boxMatches(const lt::TileParams& tp, const lt::BoxParams& b, int es) {
+  const int vol = tp.tileVol;
+  // global offset -> input-order element, on both sides
+  lt::TileParams one = tp;
+  one.lv = one.sv = 1;
+  one.nIn = one.nOut = vol;
+  one.padShift = lt::PAD_NONE;
+  std::vector<int> in(vol), out(vol);
+  std::vector<unsigned short> jOf(vol);
+  lt::tileTablesHost(one, in.data(), out.data(), jOf.data());
+  std::unordered_map<uint32_t, int> byIn, byOut;
+  for (int x = 0; x < vol; ++x) {
+    byIn[(uint32_t)in[x]] = x;
+    byOut[(uint32_t)out[x]] = jOf[x];
+  }
+  std::vector<int> shared(b.smBytes / es, -1);
+  int loaded = 0, stored = 0;
+  const int lv = b.ld.h.unit, sv = b.st.h.unit;
+  if (b.ld.h.active > lt::TILE_THREADS || b.st.h.active > lt::TILE_THREADS) return false;
+  for (int t = 0; t < b.ld.h.active; ++t) {
+    uint32_t off, sm;
+    const int top = lt::boxDecode(b.ld.rank, b.ld.h.p, (uint32_t)(t * lv), off, sm);
+    const int n = b.ld.h.nFull + (top < b.ld.h.rem ? b.ld.h.nRagged : 0);
+    for (int k = 0; k < n; ++k) {
+      const uint32_t at = sm + b.ld.slot[k].sm;
+      if (at % (uint32_t)(lv * es) || at + (uint32_t)(lv * es) > (uint32_t)b.smBytes) return false;
+      for (int m = 0; m < lv; ++m) {
+        const auto it = byIn.find(off + b.ld.slot[k].off + (uint32_t)m);
+        int& cell = shared[at / es + m];
+        if (it == byIn.end() || cell >= 0) return false;
+        cell = it->second;
+        ++loaded;
+      }
+    }
+  }
+  if (loaded != vol) return false;
+  for (int t = 0; t < b.st.h.active; ++t) {
+    uint32_t off, sm;
+    const int top = lt::boxDecode(b.st.rank, b.st.h.p, (uint32_t)(t * sv), off, sm);
+    const int n = b.st.h.nFull + (top < b.st.h.rem ? b.st.h.nRagged : 0);
+    for (int k = 0; k < n; ++k)
+      for (int m = 0; m < sv; ++m) {
+        uint32_t o2, at = sm + (uint32_t)m * b.elemStep;
+        if (b.straddle && m > 0)
+          lt::boxDecode(b.st.rank, b.st.h.p, (uint32_t)(t * sv + m), o2, at);
+        at += b.st.slot[k].sm;
+        const auto it = byOut.find(off + b.st.slot[k].off + (uint32_t)m);
+        if (at % (uint32_t)es || at >= (uint32_t)b.smBytes || it == byOut.end() ||
+            shared[at / es] != it->second)
+          return false;
+        byOut.erase(it);  // once
+        ++stored;
+      }
+  }
+  return stored == vol;
+}
+
+}  // namespace
+
+extern "C" {
+
+int librett_c_group_box_check(int rank, const int* dim, const int* permutation, size_t sizeofType,
+                              int num_sms, int candidate, int variant) {
+  if (lt::checkInput(rank, dim, permutation, sizeofType) != 0 || variant < 0 || variant > 3)
+    return LIBRETT_INVALID_PARAMETER;
+  const int sms = num_sms > 0 ? num_sms : 152;
+  lt::Fused f;
+  lt::fuseRanks(rank, dim, permutation, (int)sizeofType, f);
+  std::vector<lt::PlanDesc> cands = lt::flatTileCandidates(f, sms);
+  if (candidate < 0 || candidate >= (int)cands.size()) return LIBRETT_INVALID_PARAMETER;
+  lt::PlanDesc pd = cands[candidate];
+  if (variant == 1) {
+    if (!lt::finalizePlan(pd)) return LIBRETT_INTERNAL_ERROR;
+    pd.tile = pd.tileScalar;
+  } else if (variant == 2) {
+    lt::widenUnitsByExtents(pd, sms, true);
+    lt::widenUnits8(pd, true);
+  } else if (variant == 3) {
+    lt::groupDoubleTile(pd, sms);
+  }
+  const lt::GroupRunSplit rs = lt::groupRunSplit(pd.tile);
+  if (rs.inRun % pd.tile.lv || rs.outRun % pd.tile.sv) return LIBRETT_INVALID_DEVICE;
+  lt::BoxParams b;
+  if (!lt::makeBox(pd.tile, (int)sizeofType, b)) return LIBRETT_INVALID_DEVICE;
+  return boxMatches(pd.tile, b, (int)sizeofType) ? LIBRETT_SUCCESS : LIBRETT_INTERNAL_ERROR;
 }
 
 int librett_c_candidate_features(int rank, const int* dim, const int* permutation,

@@ -1,0 +1,103 @@
+// Addressing of a tile by boxes, which the grouped kernel reads instead of
+// decoding every unit.
+//
+// On each side the tile's ranks are listed in that side's order (input order
+// for loads, output order for stores), ranks that continue each other in
+// global and in shared memory merged.  The CTA's threads cover a box: the
+// leading ranks whole, then as much of the next rank (the top rank) as fits
+// TILE_THREADS units.  Slots move that box over the tile: chunks of the top
+// rank, times every digit of the ranks above it.  A thread decodes its place
+// in the box once; a slot is the same for all threads, a global offset and a
+// shared-memory offset that the host works out.  So a unit costs one 64-bit
+// multiply-add for its global address and one addition for its shared one,
+// with no division, for any number of ranks, and the code is one short loop
+// per side and unit size.  Slots of whole chunks need no guard; the ones of
+// the ragged last chunk apply to threads whose top digit is below rem.
+//
+// Shared memory holds the tile at strides of its own per rank (stepS), which
+// place the padding: some elements after a rank, or after the V rows that one
+// store unit reads (the output-fastest rank is split there).  The layout is
+// picked by counting the bank wavefronts of the warps' real accesses.
+#pragma once
+
+#include <cstdint>
+
+#include "plan.h"
+
+namespace lt {
+
+constexpr int BOX_SLOTS = 64;         // of a side, at most
+constexpr int BOX_RANKS = MAXR + 1;   // of a side, with one split
+
+struct alignas(16) BoxRank {
+  uint32_t mul;    // ceil(2^32 / ext)
+  uint32_t ext;
+  uint32_t step;   // global step (elements)
+  uint32_t stepS;  // shared step (bytes)
+};
+
+struct alignas(8) BoxSlot {
+  uint32_t off;  // elements
+  uint32_t sm;   // bytes
+};
+
+// One side without its arrays.
+struct alignas(16) BoxHead {
+  int active;          // threads of the box
+  int p;               // the top rank: a thread decodes ranks 0 .. p
+  int rem;             // top digits below rem take part in the ragged chunk
+  int nFull, nRagged;  // slots of whole chunks, then of the ragged chunk
+  int rankAt, slotAt;  // grouped execution: byte offsets of the arrays in the block
+  int unit;            // elements
+};
+
+struct BoxSide {
+  BoxHead h;
+  BoxRank rank[BOX_RANKS];
+  BoxSlot slot[BOX_SLOTS];
+};
+
+struct BoxParams {
+  BoxSide ld, st;
+  int straddle;       // a store unit's elements cross output rank 0
+  uint32_t elemStep;  // shared bytes between a store unit's elements otherwise
+  int smBytes;        // shared memory of the tile
+};
+
+// Box addressing of a tile (its units lv and sv; the store unit may be 1
+// where no box can be cut at a unit boundary).  False when a side needs more
+// slots than BOX_SLOTS.
+bool makeBox(const TileParams& tp, int esize, BoxParams& b);
+
+#ifdef __CUDACC__
+#define LT_HD __host__ __device__ __forceinline__
+#else
+#define LT_HD inline
+#endif
+
+LT_HD uint32_t boxMulHi(uint32_t a, uint32_t b) {
+#ifdef __CUDA_ARCH__
+  return __umulhi(a, b);
+#else
+  return (uint32_t)(((uint64_t)a * b) >> 32);
+#endif
+}
+
+// Decodes box element x (below 2^16; the multiply-high is exact there): its
+// offsets, and the top digit returned.
+LT_HD int boxDecode(const BoxRank* rank, int p, uint32_t x, uint32_t& off, uint32_t& sm) {
+  off = sm = 0;
+  for (int r = 0; r < p; ++r) {
+    const BoxRank k = rank[r];
+    const uint32_t q = boxMulHi(x, k.mul);
+    const uint32_t d = x - q * k.ext;
+    off += d * k.step;
+    sm += d * k.stepS;
+    x = q;
+  }
+  off += x * rank[p].step;
+  sm += x * rank[p].stepS;
+  return (int)x;
+}
+
+}  // namespace lt

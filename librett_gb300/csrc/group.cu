@@ -7,6 +7,8 @@
 #include <array>
 #include <atomic>
 #include <cstring>
+#include <functional>
+#include <iterator>
 #include <map>
 #include <memory>
 #include <mutex>
@@ -33,7 +35,8 @@ __global__ void __launch_bounds__(256) writeGroupTablesKernel(const GroupTableJo
   const GroupTableJob& jb = jobs[blockIdx.x];
   const TileParams& p = jb.tp;
   const GroupRunSplit rs = jb.rs;
-  const int nL = p.tileVol / rs.inRun, nS = p.tileVol / rs.outRun;
+  const bool tables = jb.ldRow != nullptr;  // not for members of a mixed launch
+  const int nL = tables ? p.tileVol / rs.inRun : 0, nS = tables ? p.tileVol / rs.outRun : 0;
   for (int r = threadIdx.x; r < nL; r += blockDim.x) {
     int rem = r, off = 0;
     for (int t = rs.kIn; t < p.nTR; ++t) {
@@ -57,7 +60,7 @@ __global__ void __launch_bounds__(256) writeGroupTablesKernel(const GroupTableJo
     }
     jb.outRows[r] = make_int2(off, jj);
   }
-  for (int a = threadIdx.x; a < rs.outRun; a += blockDim.x) {
+  for (int a = threadIdx.x; tables && a < rs.outRun; a += blockDim.x) {
     int rem = a, jj = 0;
     for (int i = 0; i < rs.kOut; ++i) {
       const int t = p.trOut[i];
@@ -83,7 +86,7 @@ __global__ void __launch_bounds__(256) writeGroupTablesKernel(const GroupTableJo
       bout += last ? p.grLastOut[g] : (long long)c * p.grSout[g];
     }
     jb.tiles[x].inAndTensor = bin | (jb.tensor << GROUP_TILE_SHIFT);
-    jb.tiles[x].out = bout;
+    jb.tiles[x].out = bout | jb.outTag;
   }
 }
 
@@ -117,6 +120,7 @@ enum GroupPolicy {
 // occupancy.  On the 10k batch: 37 buckets instead of 92 with 4 KB
 // shared-memory classes, 10.445 -> 10.383 ms (three interleaved runs each).
 int occClass(int smem) { return std::min(8, (228 * 1024) / (smem + 1024)); }
+constexpr int MIXED_SMEM = (228 * 1024) / 6 - 1024;  // of a CTA, six on an SM
 constexpr int STAGE_MAX = 8192;   // largest store-side table set staged in shared memory
 
 // Bytes of a member's store-side run tables (outRows, smRun) when they are
@@ -157,6 +161,7 @@ struct BucketSummary {
   long long tiles, bytes;
 };
 
+
 struct Build {
   void* alloc = nullptr;
   cudaGraph_t graph = nullptr;
@@ -164,6 +169,7 @@ struct Build {
   int buckets = 0, separate = 0;
   long long tiles = 0;
   std::vector<BucketSummary> summary;  // in launch order
+  std::function<cudaError_t(cudaStream_t)> single;  // the one launch of a graph of one
 };
 
 void releaseBuild(Build& b, cudaStream_t s) {
@@ -223,10 +229,12 @@ uint64_t fnv(uint64_t h, uint64_t v) {
   return h;
 }
 
-cudaError_t launchGroupBucket(int es, int lv, int sv, int nl, int loads, const GroupTensor* tens,
-                              const GroupTile* map, uint32_t tiles, int smem, cudaStream_t s,
-                              int numSMs) {
+// es 0: a mixed launch, tens its blocks.
+cudaError_t launchGroupBucket(int es, int lv, int sv, int nl, int loads, int blockBytes,
+                              const GroupTensor* tens, const GroupTile* map, uint32_t tiles,
+                              int smem, cudaStream_t s, int numSMs) {
   switch (es) {
+    case 0: return launchGroupMixed(tens, map, tiles, blockBytes, smem, s);
     case 4: return launchGroupTile4(lv, sv, nl, loads, tens, map, tiles, smem, s, numSMs);
     case 8: return launchGroupTile8(lv, sv, nl, loads, tens, map, tiles, smem, s, numSMs);
     case 16: return launchGroupTile16(lv, sv, nl, loads, tens, map, tiles, smem, s, numSMs);
@@ -318,13 +326,122 @@ bool pickTile(const Member& m, int policy, int sms, const std::string& dev, Plan
 }
 
 struct Bucket {
-  int es, lv, sv, nl, loads;
+  int es = 0, lv = 0, sv = 0, nl = 0, loads = 0;  // es 0: a mixed launch
   int smem = 0;
   uint32_t tiles = 0;
   long long bytes = 0;
   std::vector<int> members;  // indices into GroupObj::members
   size_t tensOff = 0, mapOff = 0;
+  // mixed launch: its buckets, its members' blocks, and the shared memory in
+  // front of a tile for a block
+  std::vector<BucketSummary> parts;
+  std::vector<std::vector<unsigned char>> blocks;
+  int blockBytes = 0, dataBytes = 0;
 };
+
+BucketSummary summaryOf(const Bucket& b) {
+  return {b.es, b.lv, b.sv, b.nl, b.loads, (int)b.members.size(), b.smem, (long long)b.tiles, b.bytes};
+}
+
+// A member's block for a mixed launch (GroupBlock); empty when its tile has no
+// box.  *dataBytes: shared memory of the tile.
+std::vector<unsigned char> makeBlock(const Member& m, int* dataBytes) {
+  static thread_local BoxParams b;
+  if (!makeBox(m.pd.tile, m.pd.f.esize, b)) return {};
+  *dataBytes = b.smBytes;
+  size_t at = sizeof(GroupBlock);
+  auto place = [&](BoxSide& side) {
+    side.h.rankAt = (int)at;
+    at = align16(at + (size_t)(side.h.p + 1) * sizeof(BoxRank));
+    side.h.slotAt = (int)at;
+    at = align16(at + (size_t)(side.h.nFull + side.h.nRagged) * sizeof(BoxSlot));
+  };
+  place(b.ld);
+  place(b.st);
+  std::vector<unsigned char> block(at, 0);
+  GroupBlock g{};
+  g.in = m.in;
+  g.out = m.out;
+  g.ld = b.ld.h;
+  g.st = b.st.h;
+  g.es = m.pd.f.esize;
+  g.store = groupStore(g.es, b.st.h.unit);
+  g.straddle = b.straddle;
+  g.elemStep = b.elemStep;
+  std::memcpy(block.data(), &g, sizeof(g));
+  for (const BoxSide* side : {&b.ld, &b.st}) {
+    std::memcpy(block.data() + side->h.rankAt, side->rank, (side->h.p + 1) * sizeof(BoxRank));
+    std::memcpy(block.data() + side->h.slotAt, side->slot,
+                (side->h.nFull + side->h.nRagged) * sizeof(BoxSlot));
+  }
+  return block;
+}
+
+// Moves the members of the cp.async buckets into mixed launches: one for
+// tiles that leave room for six CTAs per SM and one for larger tiles,
+// so that those do not cost the others occupancy.  Members whose tile has no
+// box keep their bucket.
+void mixBuckets(std::vector<Bucket>& buckets, const std::vector<Member>& members) {
+  // narrow units, whose tiles take longest, first: the last CTAs end together
+  std::stable_sort(buckets.begin(), buckets.end(), [](const Bucket& a, const Bucket& b) {
+    const int ua = a.es * std::min(a.lv, a.sv), ub = b.es * std::min(b.lv, b.sv);
+    return ua != ub ? ua < ub : a.bytes > b.bytes;
+  });
+  std::vector<Bucket> out;
+  Bucket mixed[2];
+  size_t blockUnits[2] = {};
+  for (Bucket& b : buckets) {
+    if (b.loads != 1) {
+      out.push_back(std::move(b));
+      continue;
+    }
+    Bucket left = b, part[2] = {b, b};
+    for (Bucket* x : {&left, &part[0], &part[1]}) {
+      x->members.clear();
+      x->tiles = 0;
+      x->bytes = 0;
+      x->smem = 0;
+    }
+    for (int i : b.members) {
+      const Member& m = members[i];
+      int data = 0;
+      std::vector<unsigned char> block = makeBlock(m, &data);
+      const int smem = data + (int)block.size();
+      const int cls = smem <= MIXED_SMEM ? 0 : 1;
+      Bucket& x = mixed[cls];
+      // a tile holds its block's position in 23 bits
+      const bool fits = !block.empty() &&
+                        blockUnits[cls] + block.size() / 16 < (size_t(1) << (63 - GROUP_TILE_SHIFT)) &&
+                        (uint64_t)x.tiles + m.pd.tile.numTiles < (uint64_t(1) << 31);
+      if (fits) {
+        blockUnits[cls] += block.size() / 16;
+        x.members.push_back(i);
+        x.tiles += m.pd.tile.numTiles;
+        x.blockBytes = std::max(x.blockBytes, (int)block.size());
+        x.dataBytes = std::max(x.dataBytes, data);
+        x.blocks.push_back(std::move(block));
+      }
+      Bucket& y = fits ? part[cls] : left;  // as the member's bucket
+      y.members.push_back(i);
+      y.tiles += m.pd.tile.numTiles;
+      y.bytes += 2 * m.pd.f.vol * (long long)m.pd.f.esize;
+      y.smem = std::max(y.smem, m.pd.smemBytes);
+    }
+    for (int c = 0; c < 2; ++c)
+      if (!part[c].members.empty()) {
+        mixed[c].bytes += part[c].bytes;
+        mixed[c].parts.push_back(summaryOf(part[c]));
+      }
+    if (!left.members.empty()) out.push_back(std::move(left));
+  }
+  for (Bucket& x : mixed)
+    if (!x.members.empty()) {
+      x.loads = 1;
+      x.smem = x.blockBytes + x.dataBytes;
+      out.push_back(std::move(x));
+    }
+  buckets.swap(out);
+}
 
 // (Re)builds the device image and the graph for a policy.  Synchronises the
 // group's stream.
@@ -373,6 +490,7 @@ librettResult build(GroupObj& g, const Policy& pol) {
     b.bytes += 2 * pd.f.vol * (long long)pd.f.esize;
     b.smem = std::max(b.smem, pd.smemBytes);
   }
+  mixBuckets(buckets, g.members);
   B.buckets = (int)buckets.size();
   // a tile packs its descriptor index above a 40-bit offset
   for (const Bucket& b : buckets)
@@ -383,7 +501,10 @@ librettResult build(GroupObj& g, const Policy& pol) {
   size_t off = 0;
   for (Bucket& b : buckets) {
     b.tensOff = off;
-    off = align16(off + b.members.size() * sizeof(GroupTensor));
+    if (b.es == 0)
+      for (const auto& x : b.blocks) off += x.size();
+    else
+      off = align16(off + b.members.size() * sizeof(GroupTensor));
   }
   for (Bucket& b : buckets) {
     b.mapOff = off;
@@ -400,6 +521,7 @@ librettResult build(GroupObj& g, const Policy& pol) {
   std::vector<size_t> tabOff(g.members.size(), 0);
   for (const Bucket& b : buckets)
     for (int i : b.members) {
+      if (b.es == 0) continue;
       size_t sub[3];
       const TileParams& tp = g.members[i].pd.tile;
       tabOff[i] = off;
@@ -417,10 +539,25 @@ librettResult build(GroupObj& g, const Policy& pol) {
     GroupTensor* tens = reinterpret_cast<GroupTensor*>(host.data() + b.tensOff);
     GroupTile* map = reinterpret_cast<GroupTile*>(base + b.mapOff);  // device
     uint32_t first = 0;
+    size_t blockAt = 0;
     for (size_t k = 0; k < b.members.size(); ++k) {
       const int i = b.members[k];
       const Member& m = g.members[i];
       const TileParams& tp = m.pd.tile;
+      if (b.es == 0) {
+        const std::vector<unsigned char>& block = b.blocks[k];
+        std::memcpy(host.data() + b.tensOff + blockAt, block.data(), block.size());
+        GroupTableJob jb;
+        std::memset(&jb, 0, sizeof(jb));
+        jb.tp = tp;
+        jb.tiles = map + first;
+        jb.tensor = (long long)(blockAt / 16);
+        jb.outTag = (long long)(block.size() / 16) << GROUP_TILE_SHIFT;
+        std::memcpy(jobs + jobOf[i], &jb, sizeof(jb));
+        blockAt += block.size();
+        first += tp.numTiles;
+        continue;
+      }
       const GroupRunSplit rs = groupRunSplit(tp);
       size_t sub[3];
       runTableBytes(tp, rs, sub);
@@ -506,9 +643,11 @@ librettResult build(GroupObj& g, const Policy& pol) {
       load[br] += nd.bytes;
       if (nd.bucket >= 0) {
         const Bucket& b = buckets[nd.bucket];
-        B.summary.push_back({b.es, b.lv, b.sv, b.nl, b.loads, (int)b.members.size(), b.smem,
-                             (long long)b.tiles, b.bytes});
-        launched = launchGroupBucket(b.es, b.lv, b.sv, b.nl, b.loads,
+        if (b.es == 0)
+          B.summary.insert(B.summary.end(), b.parts.begin(), b.parts.end());
+        else
+          B.summary.push_back(summaryOf(b));
+        launched = launchGroupBucket(b.es, b.lv, b.sv, b.nl, b.loads, b.blockBytes,
                                      reinterpret_cast<const GroupTensor*>(base + b.tensOff),
                                      reinterpret_cast<const GroupTile*>(base + b.mapOff), b.tiles,
                                      b.smem, side[br], g.numSMs) == cudaSuccess;
@@ -522,6 +661,15 @@ librettResult build(GroupObj& g, const Policy& pol) {
     for (int b = 0; b < branches; ++b) {
       cudaEventRecord(ev[b], side[b]);
       cudaStreamWaitEvent(cap, ev[b], 0);
+    }
+    if (nodes.size() == 1 && nodes[0].bucket >= 0) {
+      const Bucket& b = buckets[nodes[0].bucket];
+      B.single = [es = b.es, lv = b.lv, sv = b.sv, nl = b.nl, loads = b.loads, tiles = b.tiles,
+                  smem = b.smem, sms = g.numSMs, bb = b.blockBytes,
+                  tens = reinterpret_cast<const GroupTensor*>(base + b.tensOff),
+                  map = reinterpret_cast<const GroupTile*>(base + b.mapOff)](cudaStream_t s) {
+        return launchGroupBucket(es, lv, sv, nl, loads, bb, tens, map, tiles, smem, s, sms);
+      };
     }
     cudaGraph_t graph = nullptr;
     const bool ended = cudaStreamEndCapture(cap, &graph) == cudaSuccess;
@@ -648,9 +796,14 @@ std::shared_ptr<GroupObj> findGroup(librettGroupHandle h) {
   return it == gGroups.end() ? nullptr : it->second;
 }
 
+// A graph of one launch goes to the stream as that launch: @@ (not while the
+// stream is being captured, where the graph call decides).
 librettResult launch(GroupObj& g) {
-  if (g.built.exec == nullptr || injectFault(FAULT_LAUNCH) ||
-      cudaGraphLaunch(g.built.exec, g.stream) != cudaSuccess)
+  if (g.built.exec == nullptr || injectFault(FAULT_LAUNCH)) return LIBRETT_INTERNAL_ERROR;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  const bool direct = g.built.single && cudaStreamIsCapturing(g.stream, &cap) == cudaSuccess &&
+                      cap == cudaStreamCaptureStatusNone;
+  if ((direct ? g.built.single(g.stream) : cudaGraphLaunch(g.built.exec, g.stream)) != cudaSuccess)
     return LIBRETT_INTERNAL_ERROR;
   gLaunchCount.fetch_add((unsigned long long)g.built.buckets + g.built.separate,
                          std::memory_order_relaxed);

@@ -21,6 +21,7 @@
 
 #include <cstdint>
 
+#include "box.h"
 #include "plan.h"
 
 namespace lt {
@@ -54,6 +55,25 @@ struct GroupTensor {
   int outStepBytes, rowSmStep, smStep;
 };
 
+// Member of a mixed launch: this header, then the arrays of both sides (box.h)
+// at their byte offsets, in one block of 16-byte units.
+struct alignas(16) GroupBlock {
+  const unsigned char* in;
+  unsigned char* out;
+  BoxHead ld, st;
+  int es;
+  int store;  // groupStore(es, store unit)
+  int straddle;
+  uint32_t elemStep;
+};
+
+// Element size and store unit (elements) as one number, which selects the
+// store code of a mixed launch.
+__host__ __device__ constexpr int groupStore(int es, int sv) { return es * 8 + sv; }
+
+constexpr int GROUP_BLOCK_MAX =
+    (int)(sizeof(GroupBlock) + 2 * (BOX_RANKS * sizeof(BoxRank) + BOX_SLOTS * sizeof(BoxSlot)));
+
 // One tile of a bucket, written on the device at group creation: the
 // element offset of its input corner with its tensor's descriptor index in
 // the top 24 bits (offsets are < 2^40 elements), and the element offset of
@@ -64,6 +84,9 @@ struct GroupTile {
   long long out;
 };
 constexpr int GROUP_TILE_SHIFT = 40;
+// In a mixed launch the descriptor index is the member's block in 16-byte units
+// from the first, and the top 24 bits of `out` hold the block's length in
+// 16-byte units.
 
 // Run-table job for one member (written once, at group creation).
 struct GroupTableJob {
@@ -74,6 +97,7 @@ struct GroupTableJob {
   int* smRun;
   GroupTile* tiles;  // this member's tiles in its bucket's tile list
   long long tensor;  // descriptor index in the bucket
+  long long outTag;  // added to every tile's out (mixed launch)
 };
 
 // Launch of one bucket's kernel (defined per element size in k_tile*.cu);
@@ -88,6 +112,11 @@ cudaError_t launchGroupTile8(int lv, int sv, int nl, int loads, const GroupTenso
 cudaError_t launchGroupTile4Half(int lv, int sv, int nl, int loads, const GroupTensor* tens,
                                  const GroupTile* tiles, uint32_t numTiles, int smem,
                                  cudaStream_t s, int numSMs);
+// Launch over tiles of members of any element size and units (blocks:
+// GroupBlock), cp.async loads; blockBytes: shared memory in front of a tile for
+// its block, smem: with it.
+cudaError_t launchGroupMixed(const void* blocks, const GroupTile* tiles, uint32_t numTiles,
+                             int blockBytes, int smem, cudaStream_t s);
 cudaError_t launchGroupTile16(int lv, int sv, int nl, int loads, const GroupTensor* tens,
                               const GroupTile* tiles, uint32_t numTiles, int smem,
                               cudaStream_t s, int numSMs);

@@ -1,0 +1,150 @@
+// Grouped execution, mixed launch: tiles of every element size and unit in
+// one grid.
+//
+// A launch of one bucket costs about 5 us whatever its work (graph node, first
+// descriptor reads, one tile), and a batch of small tensors has tens of buckets
+// of a few CTAs each.  500 tensors of 2^10 .. 2^16 elements: 33 launches on 8
+// graph branches 77.0 us, one mixed launch @@ us.
+//
+// The code of a tile must be short here, because neighbouring CTAs run
+// different units: with the buckets' unrolled bodies behind a switch, warps
+// waited for instructions 13 cycles per issue (29.5 us).  Box addressing
+// (box.h) needs one rolled loop per side, chosen by the load unit's bytes and
+// by element size and store unit.  A CTA first copies its member's block (a few
+// hundred bytes) into shared memory, where the slots are read from.
+#include "tile_kernel.cuh"
+
+namespace lt {
+namespace {
+
+struct Place {  // of a thread on one side
+  uint32_t off, sm;
+  int slots;  // it takes part in
+};
+
+__device__ __forceinline__ Place placeOf(const unsigned char* block, const BoxHead& h) {
+  Place t;
+  const BoxRank* rank = reinterpret_cast<const BoxRank*>(block + h.rankAt);
+  const int top = boxDecode(rank, h.p, threadIdx.x * h.unit, t.off, t.sm);
+  t.slots = (int)threadIdx.x >= h.active ? 0 : h.nFull + (top < h.rem ? h.nRagged : 0);
+  return t;
+}
+
+// Runs f(slot) for slots 0 .. n - 1 (n may differ between threads).
+template <typename F>
+__device__ __forceinline__ void forSlots(const unsigned char* block, const BoxHead& h, int n, F f) {
+  const BoxSlot* slot = reinterpret_cast<const BoxSlot*>(block + h.slotAt);
+  int k = 0;
+#pragma unroll 1
+  for (; k + 4 <= n; k += 4) {
+    const uint4 a = reinterpret_cast<const uint4*>(slot + k)[0];
+    const uint4 b = reinterpret_cast<const uint4*>(slot + k)[1];
+    f(BoxSlot{a.x, a.y}, BoxSlot{a.z, a.w}, BoxSlot{b.x, b.y}, BoxSlot{b.z, b.w});
+  }
+#pragma unroll 1
+  for (; k < n; ++k) f(slot[k]);
+}
+
+template <int BYTES>
+__device__ __forceinline__ void loadTile(const unsigned char* block, const BoxHead& h, int n,
+                                         const unsigned char* src, uint32_t dst, int es) {
+  forSlots(block, h, n, [&](auto... s) {
+    (cpAsyncUnit<BYTES, LT_GROUP_L2_PREFETCH>(dst + s.sm, offsetBytes(src, (int)s.off, es)), ...);
+  });
+}
+
+template <int ES, int SV>
+__device__ __forceinline__ void storeTileOf(const unsigned char* block, const GroupBlock& g, int n,
+                                            unsigned char* dst, uint32_t sm0) {
+  using T = typename Word<ES>::T;
+  using ST = typename Word<ES * SV>::T;
+  uint32_t sm[SV];
+  sm[0] = sm0;
+#pragma unroll
+  for (int m = 1; m < SV; ++m) sm[m] = sm0 + (uint32_t)m * g.elemStep;
+  if (SV > 1 && g.straddle) {
+    const BoxRank* rank = reinterpret_cast<const BoxRank*>(block + g.st.rankAt);
+    uint32_t off, first, j;
+    boxDecode(rank, g.st.p, threadIdx.x * SV, off, first);
+#pragma unroll
+    for (int m = 1; m < SV; ++m) {
+      boxDecode(rank, g.st.p, threadIdx.x * SV + m, off, j);
+      sm[m] = sm0 + j - first;
+    }
+  }
+  const int esR = opaque(ES);
+  auto one = [&](const BoxSlot& s) {
+    T e[SV];
+#pragma unroll
+    for (int m = 0; m < SV; ++m) e[m] = ldShared<ES>(sm[m] + s.sm);
+    ST v;
+    __builtin_memcpy(&v, e, sizeof(ST));
+    return v;
+  };
+  forSlots(block, g.st, n, [&](auto... s) {
+    const ST v[] = {one(s)...};
+    const uint32_t off[] = {s.off...};
+#pragma unroll
+    for (int i = 0; i < (int)sizeof...(s); ++i)
+      *reinterpret_cast<ST*>(offsetBytes(dst, (int)off[i], esR)) = v[i];
+  });
+}
+
+__global__ void __launch_bounds__(TILE_THREADS, 6)
+groupMixedKernel(const uint4* __restrict__ blocks, const GroupTile* __restrict__ tiles,
+                 int blockBytes) {
+  extern __shared__ __align__(16) unsigned char smraw[];
+  dependencyRelease();
+  const longlong2 tile = __ldg(reinterpret_cast<const longlong2*>(tiles) + blockIdx.x);
+  constexpr long long LOW = (1LL << GROUP_TILE_SHIFT) - 1;
+  const uint32_t sBase = (uint32_t)__cvta_generic_to_shared(smraw);
+  if (threadIdx.x < (uint32_t)(tile.y >> GROUP_TILE_SHIFT))
+    cpAsyncUnit<16>(sBase + 16 * threadIdx.x, blocks + (tile.x >> GROUP_TILE_SHIFT) + threadIdx.x);
+  cpAsyncWaitAll();
+  __syncthreads();
+  const GroupBlock& g = *reinterpret_cast<const GroupBlock*>(smraw);
+  const uint32_t sData = sBase + (uint32_t)blockBytes;
+  const int es = g.es;
+  {
+    const Place t = placeOf(smraw, g.ld);
+    const unsigned char* src = g.in + (tile.x & LOW) * es;
+    src = offsetBytes(src, (int)t.off, es);
+    // blocks and tile list are written once, at group creation (which
+    // synchronises), so only the tensors' data waits for the stream
+    dependencyWait();
+    switch (es * g.ld.unit) {
+      case 16: loadTile<16>(smraw, g.ld, t.slots, src, sData + t.sm, es); break;
+      case 8: loadTile<8>(smraw, g.ld, t.slots, src, sData + t.sm, es); break;
+      default: loadTile<4>(smraw, g.ld, t.slots, src, sData + t.sm, es); break;
+    }
+  }
+  const Place t = placeOf(smraw, g.st);  // while the loads are in flight
+  unsigned char* dst = offsetBytes(g.out + (tile.y & LOW) * es, (int)t.off, es);
+  cpAsyncWaitAll();
+  __syncthreads();
+  switch (g.store) {
+#define LT_STORE(ES, SV) \
+  case groupStore(ES, SV): storeTileOf<ES, SV>(smraw, g, t.slots, dst, sData + t.sm); break;
+    LT_STORE(4, 4)
+    LT_STORE(4, 2)
+    LT_STORE(4, 1)
+    LT_STORE(8, 2)
+    LT_STORE(8, 1)
+    LT_STORE(16, 1)
+#undef LT_STORE
+    default: break;
+  }
+}
+
+}  // namespace
+
+cudaError_t launchGroupMixed(const void* blocks, const GroupTile* tiles, uint32_t numTiles,
+                             int blockBytes, int smem, cudaStream_t s) {
+  if (smem > 48 * 1024 &&
+      cachedOccupancy((const void*)groupMixedKernel, TILE_THREADS, smem) < 1)
+    return cudaErrorInvalidConfiguration;
+  return launchDependent(groupMixedKernel, numTiles, TILE_THREADS, smem, s, (const uint4*)blocks,
+                         tiles, blockBytes);
+}
+
+}  // namespace lt

@@ -883,16 +883,12 @@ __device__ __forceinline__ void stShared(uint32_t addr, const typename Word<BYTE
 // multiply-add per slot.  Byte offsets are multiply-adds by a scale the
 // compiler cannot fold into shifts.
 template <int ES, int LV, int SV, int NL, int LOADS>
-__device__ __forceinline__ void groupTileBody(const GroupTensor* __restrict__ tens,
-                                              const GroupTile* __restrict__ tiles,
-                                              uint32_t tileIndex) {
+__device__ __forceinline__ void groupTileBody(const GroupTensor* __restrict__ g, long long bin,
+                                              long long bout) {
   using T = typename Word<ES>::T;
   using LT = typename Word<ES * LV>::T;
   using ST = typename Word<ES * SV>::T;
   extern __shared__ __align__(16) unsigned char smraw[];
-  const longlong2 tile = __ldg(reinterpret_cast<const longlong2*>(tiles) + tileIndex);
-  const GroupTensor* g = tens + (int)(tile.x >> GROUP_TILE_SHIFT);
-  const long long bin = tile.x & ((1LL << GROUP_TILE_SHIFT) - 1), bout = tile.y;
   // shared memory: [store-side run tables, when staged][tile data]
   const int tabBytes = g->tabBytes;
   T* s = reinterpret_cast<T*>(smraw + tabBytes);
@@ -944,12 +940,15 @@ __device__ __forceinline__ void groupTileBody(const GroupTensor* __restrict__ te
         LT v[NL];
 #pragma unroll
         for (int k = 0; k < NL; ++k)
-          if (k * TILE_THREADS < uMax) v[k] = *unitSrc(k);
+          if (k * TILE_THREADS < uMax) v[k] = ldGlobal<ES * LV>(unitSrc(k));
 #pragma unroll
         for (int k = 0; k < NL; ++k)
           if (k * TILE_THREADS < uMax) stShared<ES * LV>(dst0 + (uint32_t)(k * stepBytes), v[k]);
       }
     };
+    // the tile list, descriptor and tables are written once, at group creation
+    // (which synchronises), so only the tensors' data waits for the stream
+    dependencyWait();
     if (ldStepB >= 0)
       loadAll(std::true_type{});
     else
@@ -1054,6 +1053,17 @@ __device__ __forceinline__ void groupTileBody(const GroupTensor* __restrict__ te
   }
 }
 
+// Tile `index` of a bucket: its tensor's descriptor and its corner offsets.
+__device__ __forceinline__ const GroupTensor* groupTile(const GroupTensor* __restrict__ tens,
+                                                        const GroupTile* __restrict__ tiles,
+                                                        uint32_t index, long long& bin,
+                                                        long long& bout) {
+  const longlong2 tile = __ldg(reinterpret_cast<const longlong2*>(tiles) + index);
+  bin = tile.x & ((1LL << GROUP_TILE_SHIFT) - 1);
+  bout = tile.y;
+  return tens + (int)(tile.x >> GROUP_TILE_SHIFT);
+}
+
 // One tile of a group bucket per CTA (LOADS 0: loads through registers,
 // 1: cp.async), or, with LOADS 2, persistent CTAs (grid = SMs x occupancy)
 // that walk the bucket's tile list with a grid stride, cp.async loads.
@@ -1061,13 +1071,17 @@ template <int ES, int LV, int SV, int NL, int LOADS>
 __global__ void __launch_bounds__(TILE_THREADS)
 groupTileKernel(const GroupTensor* __restrict__ tens, const GroupTile* __restrict__ tiles,
                 uint32_t numTiles) {
+  long long bin, bout;
+  dependencyRelease();
   if constexpr (LOADS == 2) {
     for (uint32_t t = blockIdx.x; t < numTiles; t += gridDim.x) {
-      groupTileBody<ES, LV, SV, NL, 1>(tens, tiles, t);
+      const GroupTensor* g = groupTile(tens, tiles, t, bin, bout);
+      groupTileBody<ES, LV, SV, NL, 1>(g, bin, bout);
       __syncthreads();  // the next tile reuses the shared buffers
     }
   } else {
-    groupTileBody<ES, LV, SV, NL, LOADS>(tens, tiles, blockIdx.x);
+    const GroupTensor* g = groupTile(tens, tiles, blockIdx.x, bin, bout);
+    groupTileBody<ES, LV, SV, NL, LOADS>(g, bin, bout);
   }
 }
 
