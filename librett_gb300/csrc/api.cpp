@@ -671,7 +671,20 @@ bool boxMatches(const lt::TileParams& tp, const lt::BoxParams& b, int es) {
     uint32_t off, sm;
     const int top = lt::boxDecode(b.st.rank, b.st.h.p, (uint32_t)(t * sv), off, sm);
     const int n = b.st.h.nFull + (top < b.st.h.rem ? b.st.h.nRagged : 0);
-    for (int k = 0; k < n; ++k)
+    for (int k = 0; k < n && b.block; ++k) {
+      const int V = 16 / es;
+      for (int m = 0; m < V; ++m) {
+        const uint32_t at = sm + b.st.slot[k].sm + (uint32_t)m * b.elemStep;
+        if (at % 16 || at + 16 > (uint32_t)b.smBytes) return false;
+        for (int c = 0; c < V; ++c) {
+          const auto it = byOut.find(off + b.st.slot[k].off + (uint32_t)(c * b.colStep) + (uint32_t)m);
+          if (it == byOut.end() || shared[at / es + c] != it->second) return false;
+          byOut.erase(it);
+          ++stored;
+        }
+      }
+    }
+    for (int k = 0; k < n && !b.block; ++k)
       for (int m = 0; m < sv; ++m) {
         uint32_t o2, at = sm + (uint32_t)m * b.elemStep;
         if (b.straddle && m > 0)

@@ -94,11 +94,13 @@ struct Layout {
 
 struct Built {
   Ranks ld, st;
-  int vol;  // padded elements
+  int vol;            // padded elements
+  uint32_t elemStep;  // shared step of the output-fastest rank
 };
 
-// Ranks of both sides under a layout (shared steps in bytes).
-void applyLayout(const TileParams& tp, int esize, const Layout& L, Built& b) {
+// Ranks of both sides under a layout (shared steps in bytes).  blockV > 1: the
+// store side in blocks of blockV along its fastest rank and input rank 0.
+void applyLayout(const TileParams& tp, int esize, const Layout& L, int blockV, Built& b) {
   uint32_t P[MAXR], PS = 0;  // stride of each tile rank; of the split rank's upper part
   const int t0 = tp.trOut[0];
   int s = 1, last = 0;
@@ -126,7 +128,19 @@ void applyLayout(const TileParams& tp, int esize, const Layout& L, Built& b) {
     }
   };
   for (int t = 0; t < tp.nTR; ++t) add(b.ld, t, tp.trSin);
-  for (int i = 0; i < tp.nTR; ++i) add(b.st, tp.trOut[i], tp.trSout);
+  for (int i = 0; i < tp.nTR; ++i) {
+    const int t = tp.trOut[i];
+    if (blockV > 1 && (t == t0 || t == 0)) {
+      const int n = tp.trE[t] / blockV;
+      if (n > 1)
+        b.st.add(n, (uint32_t)(blockV * tp.trSout[t]),
+                 t == t0 && L.split > 0 ? PS : (uint32_t)blockV * P[t]);
+    } else {
+      add(b.st, t, tp.trSout);
+    }
+  }
+  if (b.st.n == 0) b.st.add(1, 0, 0);  // one block
+  b.elemStep = P[t0];
 }
 
 // Wavefronts of the first two warps' accesses on both sides; *ideal: without
@@ -144,6 +158,13 @@ int layoutCost(const BoxParams& b, int esize, int* ideal) {
       *ideal += (lanes * b.ld.h.unit * esize + 127) / 128;
     }
     lanes = std::min(32, b.st.h.active - 32 * w);
+    if (b.block && lanes > 0) {
+      for (int l = 0; l < lanes; ++l)
+        boxDecode(b.st.rank, b.st.h.p, (uint32_t)(32 * w + l), off, addr[l]);
+      cost += accessCost(addr, lanes, 16);  // the V reads are shifted copies
+      *ideal += (lanes * 16 + 127) / 128;
+      continue;
+    }
     for (int m = 0; m < b.st.h.unit && lanes > 0; ++m) {
       for (int l = 0; l < lanes; ++l) {
         if (m == 0 || b.straddle)
@@ -163,12 +184,16 @@ int layoutCost(const BoxParams& b, int esize, int* ideal) {
 bool makeBox(const TileParams& tp, int esize, BoxParams& b) {
   if (tp.nTR < 1) return false;
   const int t0 = tp.trOut[0];
+  const int V = 16 / esize;
+  b.block = V > 1 && tp.lv == V && tp.sv == V && t0 != 0 && tp.trE[0] % V == 0 && tp.trE[t0] % V == 0;
+  b.colStep = tp.trSout[0];
   auto build = [&](const Layout& L, int sv) {
     Built r;
-    applyLayout(tp, esize, L, r);
+    applyLayout(tp, esize, L, b.block ? V : 1, r);
+    if (b.block) sv = 1;  // an item of the store side is one block
     b.straddle = sv > 1 && tp.trE[t0] % sv != 0;
     // (a split at the unit's rows leaves its elements inside the lower part)
-    b.elemStep = r.st.stepS[0];
+    b.elemStep = r.elemStep;
     b.smBytes = (r.vol * esize + 15) / 16 * 16;
     // shared memory is what limits the CTAs of an SM: an eighth for padding
     if (8 * r.vol > 9 * tp.tileVol && L.pad > 0) return false;
@@ -199,7 +224,7 @@ bool makeBox(const TileParams& tp, int esize, BoxParams& b) {
     for (int t = 0; t <= last; ++t) prod *= tp.trE[t];
     return prod % lv == 0;
   };
-  for (int sv = tp.sv;; sv = 1) {
+  for (int sv = tp.sv;;) {
     int best = -1, bestCost = 0;
     int tried = -1;  // the layout b holds, whole or in part
     for (int c = 0; c < n; ++c) {
@@ -218,8 +243,13 @@ bool makeBox(const TileParams& tp, int esize, BoxParams& b) {
       if (tried != best) build(cand[best], sv);
       return true;
     }
-    // no box cut at a unit boundary: element stores
-    if (sv == 1) return false;
+    // no box of blocks: units; none cut at a unit boundary: elements
+    if (b.block)
+      b.block = 0;
+    else if (sv > 1)
+      sv = 1;
+    else
+      return false;
   }
 }
 

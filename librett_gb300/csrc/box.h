@@ -14,6 +14,13 @@
 // per side and unit size.  Slots of whole chunks need no guard; the ones of
 // the ragged last chunk apply to threads whose top digit is below rem.
 //
+// Where both sides move 16-byte units of V elements along whole multiples of V
+// of the input's and the output's fastest rank, a store item is a block of V x
+// V elements: V 16-byte reads of shared memory, transposed in registers, V
+// 16-byte stores.  That takes a V-th of the shared-memory reads of single
+// elements, and their 4-byte (float32) or 8-byte accesses V units apart cannot
+// be free of bank conflicts under padding that keeps 16-byte units aligned.
+//
 // Shared memory holds the tile at strides of its own per rank (stepS), which
 // place the padding: some elements after a rank, or after the V rows that one
 // store unit reads (the output-fastest rank is split there).  The layout is
@@ -59,8 +66,11 @@ struct BoxSide {
 
 struct BoxParams {
   BoxSide ld, st;
+  int block;          // store items are V x V blocks (unit 1 in st.h: one item)
+  long long colStep;  // global output step (elements) between a block's V stores
   int straddle;       // a store unit's elements cross output rank 0
-  uint32_t elemStep;  // shared bytes between a store unit's elements otherwise
+  uint32_t elemStep;  // shared bytes between a store unit's elements otherwise,
+                      // and between a block's V reads
   int smBytes;        // shared memory of the tile
 };
 

@@ -65,10 +65,12 @@ struct alignas(16) GroupBlock {
   int store;  // groupStore(es, store unit)
   int straddle;
   uint32_t elemStep;
+  long long colStep;  // bytes
+  int unused[2];
 };
 
-// Element size and store unit (elements) as one number, which selects the
-// store code of a mixed launch.
+// Element size and store unit (elements; 0: blocks) as one number, which
+// selects the store code of a mixed launch.
 __host__ __device__ constexpr int groupStore(int es, int sv) { return es * 8 + sv; }
 
 constexpr int GROUP_BLOCK_MAX =

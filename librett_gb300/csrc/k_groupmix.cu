@@ -30,16 +30,23 @@ __device__ __forceinline__ Place placeOf(const unsigned char* block, const BoxHe
   return t;
 }
 
-// Runs f(slot) for slots 0 .. n - 1 (n may differ between threads).
-template <typename F>
+// Runs f(slots...) for slots 0 .. n - 1 (n may differ between threads), PER (1,
+// 2 or 4) at a time and the rest one by one.
+template <int PER, typename F>
 __device__ __forceinline__ void forSlots(const unsigned char* block, const BoxHead& h, int n, F f) {
   const BoxSlot* slot = reinterpret_cast<const BoxSlot*>(block + h.slotAt);
   int k = 0;
+  if constexpr (PER > 1) {
 #pragma unroll 1
-  for (; k + 4 <= n; k += 4) {
-    const uint4 a = reinterpret_cast<const uint4*>(slot + k)[0];
-    const uint4 b = reinterpret_cast<const uint4*>(slot + k)[1];
-    f(BoxSlot{a.x, a.y}, BoxSlot{a.z, a.w}, BoxSlot{b.x, b.y}, BoxSlot{b.z, b.w});
+    for (; k + PER <= n; k += PER) {
+      const uint4 a = reinterpret_cast<const uint4*>(slot + k)[0];
+      if constexpr (PER == 4) {
+        const uint4 b = reinterpret_cast<const uint4*>(slot + k)[1];
+        f(BoxSlot{a.x, a.y}, BoxSlot{a.z, a.w}, BoxSlot{b.x, b.y}, BoxSlot{b.z, b.w});
+      } else {
+        f(BoxSlot{a.x, a.y}, BoxSlot{a.z, a.w});
+      }
+    }
   }
 #pragma unroll 1
   for (; k < n; ++k) f(slot[k]);
@@ -48,7 +55,7 @@ __device__ __forceinline__ void forSlots(const unsigned char* block, const BoxHe
 template <int BYTES>
 __device__ __forceinline__ void loadTile(const unsigned char* block, const BoxHead& h, int n,
                                          const unsigned char* src, uint32_t dst, int es) {
-  forSlots(block, h, n, [&](auto... s) {
+  forSlots<4>(block, h, n, [&](auto... s) {
     (cpAsyncUnit<BYTES, LT_GROUP_L2_PREFETCH>(dst + s.sm, offsetBytes(src, (int)s.off, es)), ...);
   });
 }
@@ -81,12 +88,47 @@ __device__ __forceinline__ void storeTileOf(const unsigned char* block, const Gr
     __builtin_memcpy(&v, e, sizeof(ST));
     return v;
   };
-  forSlots(block, g.st, n, [&](auto... s) {
+  forSlots<4>(block, g.st, n, [&](auto... s) {
     const ST v[] = {one(s)...};
     const uint32_t off[] = {s.off...};
 #pragma unroll
     for (int i = 0; i < (int)sizeof...(s); ++i)
       *reinterpret_cast<ST*>(offsetBytes(dst, (int)off[i], esR)) = v[i];
+  });
+}
+
+// Blocks of V x V elements, transposed in registers.
+template <int ES>
+__device__ __forceinline__ void storeBlocks(const unsigned char* block, const GroupBlock& g, int n,
+                                            unsigned char* dst, uint32_t sm0) {
+  using T = typename Word<ES>::T;
+  constexpr int V = 16 / ES;
+  const int esR = opaque(ES);
+  forSlots<V == 2 ? 2 : 1>(block, g.st, n, [&](auto... s) {
+    constexpr int N = (int)sizeof...(s);
+    const uint32_t sm[] = {s.sm...}, off[] = {s.off...};
+    T e[N][V][V];
+#pragma unroll
+    for (int i = 0; i < N; ++i)
+#pragma unroll
+      for (int m = 0; m < V; ++m) {
+        const uint4 r = ldShared<16>(sm0 + sm[i] + (uint32_t)m * g.elemStep);
+        __builtin_memcpy(e[i][m], &r, 16);
+      }
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      unsigned char* d = offsetBytes(dst, (int)off[i], esR);
+#pragma unroll
+      for (int c = 0; c < V; ++c) {
+        T col[V];
+#pragma unroll
+        for (int m = 0; m < V; ++m) col[m] = e[i][m][c];
+        uint4 r;
+        __builtin_memcpy(&r, col, 16);
+        *reinterpret_cast<uint4*>(d) = r;
+        d += g.colStep;
+      }
+    }
   });
 }
 
@@ -132,6 +174,8 @@ groupMixedKernel(const uint4* __restrict__ blocks, const GroupTile* __restrict__
     LT_STORE(8, 1)
     LT_STORE(16, 1)
 #undef LT_STORE
+    case groupStore(4, 0): storeBlocks<4>(smraw, g, t.slots, dst, sData + t.sm); break;
+    case groupStore(8, 0): storeBlocks<8>(smraw, g, t.slots, dst, sData + t.sm); break;
     default: break;
   }
 }
