@@ -690,6 +690,7 @@ bool boxMatches(const lt::TileParams& tp, const lt::BoxParams& b, int es) {
         if (b.straddle && m > 0)
           lt::boxDecode(b.st.rank, b.st.h.p, (uint32_t)(t * sv + m), o2, at);
         at += b.st.slot[k].sm;
+        if (b.wide && (at - (uint32_t)(m * es)) % (uint32_t)(sv * es)) return false;
         const auto it = byOut.find(off + b.st.slot[k].off + (uint32_t)m);
         if (at % (uint32_t)es || at >= (uint32_t)b.smBytes || it == byOut.end() ||
             shared[at / es] != it->second)

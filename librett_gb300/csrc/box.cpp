@@ -131,10 +131,14 @@ void applyLayout(const TileParams& tp, int esize, const Layout& L, int blockV, B
   for (int i = 0; i < tp.nTR; ++i) {
     const int t = tp.trOut[i];
     if (blockV > 1 && (t == t0 || t == 0)) {
-      const int n = tp.trE[t] / blockV;
-      if (n > 1)
-        b.st.add(n, (uint32_t)(blockV * tp.trSout[t]),
-                 t == t0 && L.split > 0 ? PS : (uint32_t)blockV * P[t]);
+      const uint32_t so = (uint32_t)blockV * (uint32_t)tp.trSout[t];
+      if (t == t0 && L.split > 0) {
+        if (L.split > blockV) b.st.add(L.split / blockV, so, (uint32_t)blockV * P[t]);
+        if (tp.trE[t] > L.split)
+          b.st.add(tp.trE[t] / L.split, (uint32_t)L.split * (uint32_t)tp.trSout[t], PS);
+      } else if (tp.trE[t] > blockV) {
+        b.st.add(tp.trE[t] / blockV, so, (uint32_t)blockV * P[t]);
+      }
     } else {
       add(b.st, t, tp.trSout);
     }
@@ -165,15 +169,16 @@ int layoutCost(const BoxParams& b, int esize, int* ideal) {
       *ideal += (lanes * 16 + 127) / 128;
       continue;
     }
-    for (int m = 0; m < b.st.h.unit && lanes > 0; ++m) {
+    const int reads = b.wide ? 1 : b.st.h.unit, bytes = b.wide ? b.st.h.unit * esize : esize;
+    for (int m = 0; m < reads && lanes > 0; ++m) {
       for (int l = 0; l < lanes; ++l) {
         if (m == 0 || b.straddle)
           boxDecode(b.st.rank, b.st.h.p, (uint32_t)((32 * w + l) * b.st.h.unit + m), off, addr[l]);
         else
           addr[l] += b.elemStep;
       }
-      cost += accessCost(addr, lanes, esize);
-      *ideal += (lanes * esize + 127) / 128;
+      cost += accessCost(addr, lanes, bytes);
+      *ideal += (lanes * bytes + 127) / 128;
     }
   }
   return cost;
@@ -192,30 +197,37 @@ bool makeBox(const TileParams& tp, int esize, BoxParams& b) {
     applyLayout(tp, esize, L, b.block ? V : 1, r);
     if (b.block) sv = 1;  // an item of the store side is one block
     b.straddle = sv > 1 && tp.trE[t0] % sv != 0;
-    // (a split at the unit's rows leaves its elements inside the lower part)
     b.elemStep = r.elemStep;
     b.smBytes = (r.vol * esize + 15) / 16 * 16;
     // shared memory is what limits the CTAs of an SM: an eighth for padding
     if (8 * r.vol > 9 * tp.tileVol && L.pad > 0) return false;
     if (tp.lv > 1 && (r.ld.step[0] != 1 || r.ld.ext[0] % tp.lv != 0)) return false;
-    return buildSide(r.ld, tp.lv, b.ld) && buildSide(r.st, sv, b.st);
+    if (!buildSide(r.ld, tp.lv, b.ld) || !buildSide(r.st, sv, b.st)) return false;
+    b.wide = sv > 1 && !b.straddle && b.elemStep == (uint32_t)esize;
+    const uint32_t unit = (uint32_t)(sv * esize);
+    for (int k = 1; k <= b.st.h.p; ++k) b.wide = b.wide && b.st.rank[k].stepS % unit == 0;
+    for (int k = 0; k < b.st.h.nFull + b.st.h.nRagged; ++k)
+      b.wide = b.wide && b.st.slot[k].sm % unit == 0;
+    return true;
   };
   // Candidate layouts, likeliest first.  The padding keeps load units whole
-  // and aligned: multiples of lv, after products that are multiples of lv.
-  Layout cand[16];
+  // and aligned (multiples of lv, after products that are multiples of lv), and
+  // wide store units too.
+  Layout cand[24];
   int n = 0;
-  const int lv = tp.lv;
+  const int lv = tp.lv, unit = t0 == 0 ? std::max(lv, tp.sv) : lv;
   if (t0 > 0) {
-    if (tp.sv > 1 && tp.trE[t0] % tp.sv == 0) {
-      cand[n++] = {0, lv, tp.sv};
-    }
+    // after the rows of a unit; after each row; after a few short rows
+    if (tp.sv > 1 && tp.trE[t0] % tp.sv == 0) cand[n++] = {0, lv, tp.sv};
     for (int k = 1; k <= 3; ++k) cand[n++] = {t0 - 1, k * lv, 0};
+    for (int k = 2; k <= 32; k *= 2)
+      if (k != tp.sv && k < tp.trE[t0] && tp.trE[t0] % k == 0) cand[n++] = {0, lv, k};
   }
   cand[n++] = {-1, 0, 0};
-  for (int t = 0; t + 1 < tp.nTR && n < 12; ++t)
+  for (int t = 0; t + 1 < tp.nTR && n < 20; ++t)
     if (t != t0 - 1) {
-      cand[n++] = {t, lv, 0};
-      cand[n++] = {t, 2 * lv, 0};
+      cand[n++] = {t, unit, 0};
+      cand[n++] = {t, 2 * unit, 0};
     }
   auto whole = [&](const Layout& L) {
     if (L.pad == 0) return true;
@@ -228,7 +240,8 @@ bool makeBox(const TileParams& tp, int esize, BoxParams& b) {
     int best = -1, bestCost = 0;
     int tried = -1;  // the layout b holds, whole or in part
     for (int c = 0; c < n; ++c) {
-      if (!whole(cand[c]) || (cand[c].split > 0 && cand[c].split != sv)) continue;
+      // (a store unit stays inside a split's lower part)
+      if (!whole(cand[c]) || (cand[c].split > 0 && cand[c].split % sv != 0)) continue;
       tried = c;
       if (!build(cand[c], sv)) continue;
       int ideal;

@@ -68,6 +68,7 @@ struct BoxParams {
   BoxSide ld, st;
   int block;          // store items are V x V blocks (unit 1 in st.h: one item)
   long long colStep;  // global output step (elements) between a block's V stores
+  int wide;           // a store unit's elements are one aligned piece of shared memory
   int straddle;       // a store unit's elements cross output rank 0
   uint32_t elemStep;  // shared bytes between a store unit's elements otherwise,
                       // and between a block's V reads

@@ -365,7 +365,9 @@ std::vector<unsigned char> makeBlock(const Member& m, int* dataBytes) {
   g.ld = b.ld.h;
   g.st = b.st.h;
   g.es = m.pd.f.esize;
-  g.store = groupStore(g.es, b.block ? 0 : b.st.h.unit);
+  g.store = b.block  ? groupStore(g.es, 0)
+            : b.wide ? groupStore(g.es * b.st.h.unit, 1)  // as one element
+                     : groupStore(g.es, b.st.h.unit);
   g.colStep = b.colStep * g.es;
   g.straddle = b.straddle;
   g.elemStep = b.elemStep;

@@ -69,9 +69,9 @@ struct alignas(16) GroupBlock {
   int unused[2];
 };
 
-// Element size and store unit (elements; 0: blocks) as one number, which
-// selects the store code of a mixed launch.
-__host__ __device__ constexpr int groupStore(int es, int sv) { return es * 8 + sv; }
+// Bytes of a shared-memory read and reads per store unit (0: blocks) as one
+// number, which selects the store code of a mixed launch.
+__host__ __device__ constexpr int groupStore(int bytes, int reads) { return bytes * 8 + reads; }
 
 constexpr int GROUP_BLOCK_MAX =
     (int)(sizeof(GroupBlock) + 2 * (BOX_RANKS * sizeof(BoxRank) + BOX_SLOTS * sizeof(BoxSlot)));

@@ -63,6 +63,7 @@ __device__ __forceinline__ void loadTile(const unsigned char* block, const BoxHe
 template <int ES, int SV>
 __device__ __forceinline__ void storeTileOf(const unsigned char* block, const GroupBlock& g, int n,
                                             unsigned char* dst, uint32_t sm0) {
+  // (a wide unit is one read of its bytes: ES is not the element size then)
   using T = typename Word<ES>::T;
   using ST = typename Word<ES * SV>::T;
   uint32_t sm[SV];
@@ -79,7 +80,7 @@ __device__ __forceinline__ void storeTileOf(const unsigned char* block, const Gr
       sm[m] = sm0 + j - first;
     }
   }
-  const int esR = opaque(ES);
+  const int es = g.es;
   auto one = [&](const BoxSlot& s) {
     T e[SV];
 #pragma unroll
@@ -93,7 +94,7 @@ __device__ __forceinline__ void storeTileOf(const unsigned char* block, const Gr
     const uint32_t off[] = {s.off...};
 #pragma unroll
     for (int i = 0; i < (int)sizeof...(s); ++i)
-      *reinterpret_cast<ST*>(offsetBytes(dst, (int)off[i], esR)) = v[i];
+      *reinterpret_cast<ST*>(offsetBytes(dst, (int)off[i], es)) = v[i];
   });
 }
 
