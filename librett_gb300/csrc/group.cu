@@ -250,9 +250,9 @@ bool pickTile(const Member& m, int policy, int sms, const std::string& dev, Plan
   if (policy == GP_SELECTOR && own.kernel == K_TILE && flatTables(own.pipe)) {
     out = own;  // the group uses the tile geometry only
   } else {
-    // the selector ranks screened candidates (as for librettPlan)
-    std::vector<PlanDesc> c =
-        flatTileCandidates(own.f, policy == GP_FILL ? sms * 64 : sms, policy == GP_SELECTOR);
+    // screened candidates (as librettPlan ranks): no policy looks at the
+    // padding, and the pick is completed below
+    std::vector<PlanDesc> c = flatTileCandidates(own.f, policy == GP_FILL ? sms * 64 : sms, true);
     if (c.empty()) return false;
     int k = 0;
     auto eff = [](const PlanDesc& p) { return std::min(p.effIn, p.effOut); };
