@@ -186,11 +186,11 @@ int layoutCost(const BoxParams& b, int esize, int* ideal) {
 
 }  // namespace
 
-bool makeBox(const TileParams& tp, int esize, BoxParams& b) {
+bool makeBox(const TileParams& tp, int esize, BoxParams& b, bool blocks) {
   if (tp.nTR < 1) return false;
   const int t0 = tp.trOut[0];
   const int V = 16 / esize;
-  b.block = V > 1 && tp.lv == V && tp.sv == V && t0 != 0 && tp.trE[0] % V == 0 && tp.trE[t0] % V == 0;
+  b.block = blocks && V > 1 && tp.lv == V && tp.sv == V && t0 != 0 && tp.trE[0] % V == 0 && tp.trE[t0] % V == 0;
   b.colStep = tp.trSout[0];
   auto build = [&](const Layout& L, int sv) {
     Built r;
@@ -264,6 +264,37 @@ bool makeBox(const TileParams& tp, int esize, BoxParams& b) {
     else
       return false;
   }
+}
+
+std::vector<unsigned char> packBlock(BoxParams& b, int esize, const void* in, void* out) {
+  auto align16 = [](size_t x) { return (x + 15) / 16 * 16; };
+  size_t at = sizeof(TileBlock);
+  for (BoxSide* side : {&b.ld, &b.st}) {
+    side->h.rankAt = (int)at;
+    at = align16(at + (size_t)(side->h.p + 1) * sizeof(BoxRank));
+    side->h.slotAt = (int)at;
+    at = align16(at + (size_t)(side->h.nFull + side->h.nRagged) * sizeof(BoxSlot));
+  }
+  std::vector<unsigned char> block(at, 0);
+  TileBlock t{};
+  t.in = static_cast<const unsigned char*>(in);
+  t.out = static_cast<unsigned char*>(out);
+  t.ld = b.ld.h;
+  t.st = b.st.h;
+  t.es = esize;
+  t.store = b.block  ? blockStore(esize, 0)
+            : b.wide ? blockStore(esize * b.st.h.unit, 1)  // as one element
+                     : blockStore(esize, b.st.h.unit);
+  t.straddle = b.straddle;
+  t.elemStep = b.elemStep;
+  t.colStep = b.colStep * esize;
+  std::memcpy(block.data(), &t, sizeof(t));
+  for (const BoxSide* side : {&b.ld, &b.st}) {
+    std::memcpy(block.data() + side->h.rankAt, side->rank, (side->h.p + 1) * sizeof(BoxRank));
+    std::memcpy(block.data() + side->h.slotAt, side->slot,
+                (side->h.nFull + side->h.nRagged) * sizeof(BoxSlot));
+  }
+  return block;
 }
 
 }  // namespace lt

@@ -28,8 +28,15 @@
 #pragma once
 
 #include <cstdint>
+#include <vector>
 
 #include "plan.h"
+
+#ifdef __CUDACC__
+#define LT_HD __host__ __device__ __forceinline__
+#else
+#define LT_HD inline
+#endif
 
 namespace lt {
 
@@ -78,13 +85,31 @@ struct BoxParams {
 // Box addressing of a tile (its units lv and sv; the store unit may be 1
 // where no box can be cut at a unit boundary).  False when a side needs more
 // slots than BOX_SLOTS.
-bool makeBox(const TileParams& tp, int esize, BoxParams& b);
+bool makeBox(const TileParams& tp, int esize, BoxParams& b, bool blocks = true);
 
-#ifdef __CUDACC__
-#define LT_HD __host__ __device__ __forceinline__
-#else
-#define LT_HD inline
-#endif
+// What a kernel reads of a box: this header, then the arrays of both sides at
+// their byte offsets, in one block of 16-byte units.
+struct alignas(16) TileBlock {
+  const unsigned char* in;
+  unsigned char* out;
+  BoxHead ld, st;
+  int es;
+  int store;  // blockStore
+  int straddle;
+  uint32_t elemStep;
+  long long colStep;  // bytes
+  int unused[2];
+};
+
+constexpr int TILE_BLOCK_MAX =
+    (int)(sizeof(TileBlock) + 2 * (BOX_RANKS * sizeof(BoxRank) + BOX_SLOTS * sizeof(BoxSlot)));
+
+// Bytes of a shared-memory read and reads per store unit (0: blocks) as one
+// number, which selects the store code.  A wide unit is one read of its bytes.
+LT_HD constexpr int blockStore(int bytes, int reads) { return bytes * 8 + reads; }
+
+// The block of a box, at most TILE_BLOCK_MAX bytes.
+std::vector<unsigned char> packBlock(BoxParams& b, int esize, const void* in, void* out);
 
 LT_HD uint32_t boxMulHi(uint32_t a, uint32_t b) {
 #ifdef __CUDA_ARCH__

@@ -55,27 +55,6 @@ struct GroupTensor {
   int outStepBytes, rowSmStep, smStep;
 };
 
-// Member of a mixed launch: this header, then the arrays of both sides (box.h)
-// at their byte offsets, in one block of 16-byte units.
-struct alignas(16) GroupBlock {
-  const unsigned char* in;
-  unsigned char* out;
-  BoxHead ld, st;
-  int es;
-  int store;  // groupStore(es, store unit)
-  int straddle;
-  uint32_t elemStep;
-  long long colStep;  // bytes
-  int unused[2];
-};
-
-// Bytes of a shared-memory read and reads per store unit (0: blocks) as one
-// number, which selects the store code of a mixed launch.
-__host__ __device__ constexpr int groupStore(int bytes, int reads) { return bytes * 8 + reads; }
-
-constexpr int GROUP_BLOCK_MAX =
-    (int)(sizeof(GroupBlock) + 2 * (BOX_RANKS * sizeof(BoxRank) + BOX_SLOTS * sizeof(BoxSlot)));
-
 // One tile of a bucket, written on the device at group creation: the
 // element offset of its input corner with its tensor's descriptor index in
 // the top 24 bits (offsets are < 2^40 elements), and the element offset of
@@ -86,7 +65,7 @@ struct GroupTile {
   long long out;
 };
 constexpr int GROUP_TILE_SHIFT = 40;
-// In a mixed launch the descriptor index is the member's block in 16-byte units
+// In a mixed launch the descriptor index is the member's TileBlock in 16-byte units
 // from the first, and the top 24 bits of `out` hold the block's length in
 // 16-byte units.
 
@@ -115,7 +94,7 @@ cudaError_t launchGroupTile4Half(int lv, int sv, int nl, int loads, const GroupT
                                  const GroupTile* tiles, uint32_t numTiles, int smem,
                                  cudaStream_t s, int numSMs);
 // Launch over tiles of members of any element size and units (blocks:
-// GroupBlock), cp.async loads; blockBytes: shared memory in front of a tile for
+// TileBlock), cp.async loads; blockBytes: shared memory in front of a tile for
 // its block, smem: with it.
 cudaError_t launchGroupMixed(const void* blocks, const GroupTile* tiles, uint32_t numTiles,
                              int blockBytes, int smem, cudaStream_t s);

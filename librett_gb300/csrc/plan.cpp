@@ -948,7 +948,7 @@ void modelRows(PlanDesc& pd, int numSMs) {
 // it (bulk copies need 16-byte load units and whole segments of 128 bytes or
 // more).
 void appendTileCandidates(const Fused& f, int numSMs, int pipes, std::vector<PlanDesc>& out,
-                          bool screen) {
+                          bool screen, int maxTiles) {
   const int knobs[][3] = {{512, 16384, 8192},  {256, 8192, 4096},   {128, 4096, 2048},
                           {1024, 32768, 16384}, {512, 32768, 16384}, {256, 4096, 0},
                           {2048, 65536, 32768}, {64, 2048, 0},       {256, 16384, 16384}};
@@ -958,6 +958,7 @@ void appendTileCandidates(const Fused& f, int numSMs, int pipes, std::vector<Pla
   ExtentMemo memo;  // the element size is fixed for the problem (V)
   const int V = 16 / f.esize;
   for (auto& kb : knobs) {
+    if (maxTiles > 0 && nSeen == maxTiles) break;
     int64_t target = std::max<int64_t>(1, kb[0] / f.esize);
     int64_t maxVol = std::min<int64_t>(TILE_MAX_VOL, std::max<int64_t>(1, kb[1] / f.esize));
     int64_t fillVol = std::min<int64_t>(maxVol, kb[2] / f.esize);
@@ -1012,10 +1013,10 @@ void appendTileCandidates(const Fused& f, int numSMs, int pipes, std::vector<Pla
   }
 }
 
-std::vector<PlanDesc> flatTileCandidates(const Fused& f, int numSMs, bool screen) {
+std::vector<PlanDesc> flatTileCandidates(const Fused& f, int numSMs, bool screen, int maxTiles) {
   std::vector<PlanDesc> out;
-  out.reserve(12);
-  appendTileCandidates(f, numSMs < 1 ? 1 : numSMs, PIPES_FLAT, out, screen);
+  out.reserve(maxTiles > 0 ? maxTiles : 12);
+  appendTileCandidates(f, numSMs < 1 ? 1 : numSMs, PIPES_FLAT, out, screen, maxTiles);
   for (size_t i = 0; i < out.size(); ++i) {
     out[i].candidate = (int)i;
     out[i].numCandidates = (int)out.size();

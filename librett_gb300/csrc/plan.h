@@ -268,7 +268,9 @@ bool allPipelines();
 // Tile candidates in the one-tile-per-CTA pipeline only, for any fused
 // problem (a fused rank-1 copy becomes a one-rank tile); used where every
 // member of a batch must run in that pipeline (grouped execution).
-std::vector<PlanDesc> flatTileCandidates(const Fused& f, int numSMs, bool screen = false);
+// maxTiles > 0: the first maxTiles tiles only.
+std::vector<PlanDesc> flatTileCandidates(const Fused& f, int numSMs, bool screen = false,
+                                         int maxTiles = 0);
 
 // Pipelines a tile enumeration builds candidates for (bits 1 << Pipe): the
 // default set is the one-tile-per-CTA pipeline with per-unit and bulk-copy
@@ -279,7 +281,7 @@ enum PipeSet {
   PIPES_ALL = (1 << PIPE_REG) | (1 << PIPE_ASYNC) | (1 << PIPE_FLAT) | (1 << PIPE_BULK)
 };
 void appendTileCandidates(const Fused& f, int numSMs, int pipes, std::vector<PlanDesc>& out,
-                          bool screen = false);
+                          bool screen = false, int maxTiles = 0);
 
 // Index of the candidate the analytic model prefers.
 int chooseHeuristic(const std::vector<PlanDesc>& cands);

@@ -4,12 +4,25 @@
 // (src/TensorTester.cpp:47-126, checkTransposeKernel), which compares the
 // output with an index pattern; this one compares with the actual input, so
 // any input data works.
+//
+// The input is read a tile at a time through shared memory (box.h), because the
+// elements that consecutive output elements name lie far apart: gathering them
+// one by one from global memory (verifyKernel, kept for tiles without a box)
+// fetched 32 bytes for 4 and took 745 us for 66.8M float32 elements (64, 128,
+// 96, 85) perm (3, 1, 0, 2), where the two tensors' bytes take 80 us; this
+// kernel takes 121 us (4-byte output units: two thirds of the issue slots).
+// The check shares no addressing with the single-plan kernels (slots.h).
 #include <cuda_runtime.h>
 
-#include "kernels.cuh"
+#include <cstring>
+#include <mutex>
+#include <vector>
+
+#include "box_kernel.cuh"
 #include "librett.h"
 #include "librett_c.h"
 #include "plan.h"
+#include "plans.h"
 
 namespace lt {
 namespace {
@@ -22,7 +35,17 @@ struct VerifyParams {
   long long inStride[MAXR];       // input stride of output rank i (elements)
 };
 
-// result[0]: mismatching elements; result[1]: smallest mismatching output index
+// Adds a CTA's findings to the result, one pair of atomics per CTA that has any
+// (the result lies in host memory).
+__device__ __forceinline__ void report(unsigned long long bad, unsigned long long first,
+                                       unsigned long long* result) {
+  if (bad == 0) return;
+  atomicAdd_system(result, bad);
+  atomicMax_system(result + 1, ~first);
+}
+
+// result[0]: mismatching elements; result[1]: complement of the smallest
+// mismatching output index (both start at 0)
 template <int ES>
 __global__ void __launch_bounds__(256)
 verifyKernel(const __grid_constant__ VerifyParams p, const typename Word<ES>::T* __restrict__ in,
@@ -61,11 +84,336 @@ verifyKernel(const __grid_constant__ VerifyParams p, const typename Word<ES>::T*
       if (q < first) first = q;
     }
   }
+  __shared__ unsigned long long sum, low;
+  if (threadIdx.x == 0) {
+    sum = 0;
+    low = ~0ull;
+  }
+  __syncthreads();
   if (bad) {
-    atomicAdd(result, bad);
-    atomicMin(result + 1, first);
+    atomicAdd(&sum, bad);
+    atomicMin(&low, first);
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) report(sum, low, result);
+}
+
+// Launches the element-by-element check.
+cudaError_t verifyElements(const Fused& f, int sms, const void* in, const void* out,
+                           unsigned long long* d, cudaStream_t s) {
+  VerifyParams p{};
+  p.rank = f.rank;
+  p.vol = (unsigned long long)f.vol;
+  for (int i = 0; i < f.rank; ++i) {
+    const int r = f.perm[i];
+    p.outD[i] = (unsigned long long)f.dim[r];
+    p.outDim[i] = makeFastDiv(f.dim[r] < (int64_t(1) << 31) ? (uint32_t)f.dim[r] : 1u);
+    p.inStride[i] = f.sin[r];
+  }
+  unsigned long long blocks = (p.vol + 255) / 256;
+  const unsigned long long cap = (unsigned long long)sms * 8;
+  if (blocks > cap) blocks = cap;
+  if (blocks < 1) blocks = 1;
+  auto launch = [&](auto kernel, auto word) {
+    using T = decltype(word);
+    kernel<<<(unsigned)blocks, 256, 0, s>>>(p, (const T*)in, (const T*)out, d);
+  };
+  switch (f.esize) {
+    case 4: launch(verifyKernel<4>, Word<4>::T()); break;
+    case 8: launch(verifyKernel<8>, Word<8>::T()); break;
+    default: launch(verifyKernel<16>, Word<16>::T()); break;
+  }
+  return cudaGetLastError();
+}
+
+// A tile's box and its place in the tensor.
+struct VerifyTiles {
+  uint32_t numTiles;
+  int blockBytes;
+  int nGR;  // grid ranks, decode order
+  FastDiv grDiv[MAXR];
+  long long grSin[MAXR], grSout[MAXR], grLastIn[MAXR], grLastOut[MAXR];
+  // grid rank g's dim, extent and output stride, to find the tile that owns an
+  // element: a ragged last chunk overlaps its neighbour, which owns the overlap
+  long long dim[MAXR], ext[MAXR], sout[MAXR];
+  uint4 block[TILE_BLOCK_MAX / 16];
+};
+
+// A CTA's findings, in shared memory.
+struct Findings {
+  unsigned long long bad, first;
+};
+
+// The tile that owns output element q.
+__device__ uint32_t ownerTile(const VerifyTiles& p, unsigned long long q) {
+  uint32_t owner = 0, scale = 1;
+  for (int g = 0; g < p.nGR; ++g) {
+    const unsigned long long coord = q / (unsigned long long)p.sout[g] % (unsigned long long)p.dim[g];
+    owner += (uint32_t)(coord / (unsigned long long)p.ext[g]) * scale;
+    scale *= p.grDiv[g].d;
+  }
+  return owner;
+}
+
+// Counts the mismatching elements of a thread's store units that `tile` owns,
+// one by one.
+__device__ __noinline__ void countMismatches(const unsigned char* block, const VerifyTiles& p,
+                                             uint32_t tile, int n, long long q0, uint32_t sTile,
+                                             Findings* found) {
+  const TileBlock& g = *reinterpret_cast<const TileBlock*>(block);
+  const BoxRank* rank = reinterpret_cast<const BoxRank*>(block + g.st.rankAt);
+  const BoxSlot* slot = reinterpret_cast<const BoxSlot*>(block + g.st.slotAt);
+  const int unit = g.st.unit;
+  for (int k = 0; k < n; ++k)
+    for (int m = 0; m < unit; ++m) {
+      uint32_t off, sm;
+      boxDecode(rank, g.st.p, threadIdx.x * unit + (g.straddle ? m : 0), off, sm);
+      if (!g.straddle) sm += (uint32_t)m * g.elemStep;
+      const unsigned long long q = (unsigned long long)(q0 + (int)slot[k].off + m);
+      uint32_t differ = 0;
+      for (int w = 0; w < g.es; w += 4)
+        differ |= ldShared<4>(sTile + sm + slot[k].sm + (uint32_t)w) ^
+                  ldGlobal<4>(g.out + q * (unsigned long long)g.es + w);
+      if (differ == 0 || ownerTile(p, q) != tile) continue;
+      atomicAdd(&found->bad, 1ull);
+      atomicMin(&found->first, q);
+    }
+}
+
+constexpr uint32_t VERIFY_LIST = 64;  // tiles with differences a CTA lists
+
+__device__ __forceinline__ void tileCorner(const VerifyTiles& p, uint32_t tile, long long& bin,
+                                           long long& bout) {
+  bin = bout = 0;
+  uint32_t rem = tile;
+  for (int r = 0; r < p.nGR; ++r) {
+    const uint32_t q = fdiv(rem, p.grDiv[r]);
+    const uint32_t c = rem - q * p.grDiv[r].d;
+    rem = q;
+    const bool last = c + 1 == p.grDiv[r].d;
+    bin += last ? p.grLastIn[r] : (long long)c * p.grSin[r];
+    bout += last ? p.grLastOut[r] : (long long)c * p.grSout[r];
   }
 }
+
+__device__ __forceinline__ void loadInput(const unsigned char* block, const TileBlock& g,
+                                          const Place& l, long long bin, uint32_t sTile) {
+  const int es = g.es;
+  const unsigned char* src = offsetBytes(g.in + bin * es, (int)l.off, es);
+  switch (es * g.ld.unit) {
+    case 16: loadTile<16>(block, g.ld, l.slots, src, sTile + l.sm, es); break;
+    case 8: loadTile<8>(block, g.ld, l.slots, src, sTile + l.sm, es); break;
+    default: loadTile<4>(block, g.ld, l.slots, src, sTile + l.sm, es); break;
+  }
+}
+
+// Persistent CTAs over the tensor's tiles: the input tile goes to shared memory
+// by cp.async; output units are read in batches, the first of them while the
+// tile is on its way, and compared with the elements gathered from the tile.
+// ES and SV as in the grouped store (a wide unit is one read of its bytes).
+template <int ES, int SV>
+__global__ void __launch_bounds__(TILE_THREADS, 6)
+verifyTilesKernel(const __grid_constant__ VerifyTiles p, unsigned long long* result) {
+  using T = typename Word<ES>::T;
+  using ST = typename Word<ES * SV>::T;
+  constexpr int N = ES * SV == 16 ? 4 : 8;  // units of a batch
+  extern __shared__ __align__(16) unsigned char smraw[];
+  __shared__ Findings found;
+  __shared__ uint32_t listed[VERIFY_LIST], numListed;  // tiles with a difference
+  if (threadIdx.x == 0) {
+    found = {0ull, ~0ull};
+    numListed = 0;
+  }
+  for (int c = threadIdx.x; c < p.blockBytes / 16; c += blockDim.x)
+    reinterpret_cast<uint4*>(smraw)[c] = p.block[c];
+  __syncthreads();
+  const TileBlock& g = *reinterpret_cast<const TileBlock*>(smraw);
+  const uint32_t sTile = (uint32_t)__cvta_generic_to_shared(smraw) + (uint32_t)p.blockBytes;
+  {
+    const BoxSlot* slot = reinterpret_cast<const BoxSlot*>(smraw + g.st.slotAt);
+    const int es = g.es;
+    const Place l = placeOf(smraw, g.ld), t = placeOf(smraw, g.st);
+    uint32_t sm[SV];
+    elementsOf<SV>(smraw, g, sTile + t.sm, sm);
+    for (uint32_t tile = blockIdx.x; tile < p.numTiles; tile += gridDim.x) {
+      long long bin, bout;
+      tileCorner(p, tile, bin, bout);
+      loadInput(smraw, g, l, bin, sTile);
+      const unsigned char* out = g.out + (bout + (int)t.off) * es;
+      ST w[N];
+      auto read = [&](int k) {
+#pragma unroll
+        for (int i = 0; i < N; ++i)
+          if (k + i < t.slots) w[i] = ldGlobal<ES * SV>(offsetBytes(out, (int)slot[k + i].off, es));
+      };
+      read(0);
+      cpAsyncWaitAll();
+      __syncthreads();
+      uint32_t differ = 0;
+#pragma unroll 1
+      for (int k = 0; k < t.slots; k += N) {
+        if (k > 0) read(k);
+#pragma unroll
+        for (int i = 0; i < N; ++i)
+          if (k + i < t.slots) {
+            T e[SV];
+#pragma unroll
+            for (int m = 0; m < SV; ++m) e[m] = ldShared<ES>(sm[m] + slot[k + i].sm);
+            uint32_t a[ES * SV / 4], b[ES * SV / 4];
+            __builtin_memcpy(a, e, ES * SV);
+            __builtin_memcpy(b, &w[i], ES * SV);
+#pragma unroll
+            for (int x = 0; x < ES * SV / 4; ++x) differ |= a[x] ^ b[x];
+          }
+      }
+      // (also: the next tile reuses the buffer)
+      if (__syncthreads_or((int)differ) && threadIdx.x == 0) {
+        if (numListed < VERIFY_LIST) listed[numListed] = tile;
+        ++numListed;
+      }
+    }
+  }
+  // the tiles that differ once more, counted; all of the CTA's when there are
+  // too many to list
+  __syncthreads();
+  if (numListed == 0) return;
+  const bool all = numListed > VERIFY_LIST;
+  const uint32_t n = all ? (p.numTiles - blockIdx.x + gridDim.x - 1) / gridDim.x : numListed;
+  for (uint32_t i = 0; i < n; ++i) {
+    const uint32_t tile = all ? blockIdx.x + i * gridDim.x : listed[i];
+    const Place l = placeOf(smraw, g.ld), t = placeOf(smraw, g.st);
+    long long bin, bout;
+    tileCorner(p, tile, bin, bout);
+    loadInput(smraw, g, l, bin, sTile);
+    cpAsyncWaitAll();
+    __syncthreads();
+    countMismatches(smraw, p, tile, t.slots, bout + (int)t.off, sTile, &found);
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) report(found.bad, found.first, result);
+}
+
+using VerifyKernel = void (*)(const VerifyTiles, unsigned long long*);
+
+VerifyKernel verifyKernelOf(int store) {
+  switch (store) {
+    case blockStore(4, 4): return verifyTilesKernel<4, 4>;
+    case blockStore(4, 1): return verifyTilesKernel<4, 1>;
+    case blockStore(8, 2): return verifyTilesKernel<8, 2>;
+    case blockStore(8, 1): return verifyTilesKernel<8, 1>;
+    case blockStore(16, 1): return verifyTilesKernel<16, 1>;
+    default: return nullptr;
+  }
+}
+
+// Fills p for a check of in against out; the kernel's shared memory returned,
+// 0 when the problem has no tile with a box.
+int verifyTiles(const Fused& f, int sms, const void* in, const void* out, VerifyTiles& p) {
+  // for a small tensor, whose check takes less time than ranking the planner's
+  // tiles (7 us of host time), the planner's first tile
+  const bool few = f.vol * f.esize < (4 << 20);
+  std::vector<PlanDesc> c = flatTileCandidates(f, sms, true, few ? 1 : 0);
+  if (c.empty()) return 0;
+  PlanDesc pd = c[chooseHeuristic(c)];
+  if (!refineCandidate(pd, sms)) return 0;
+  const GroupRunSplit rs = groupRunSplit(pd.tile);
+  if (((uintptr_t)in | (uintptr_t)out) % 16 != 0 || rs.inRun % pd.tile.lv || rs.outRun % pd.tile.sv) {
+    if (!finalizePlan(pd)) return 0;
+    pd.tile = pd.tileScalar;
+  }
+  const TileParams& tp = pd.tile;
+  static thread_local BoxParams b;
+  if (!makeBox(tp, f.esize, b, false)) return 0;
+  p.numTiles = tp.numTiles;
+  p.nGR = tp.nGR;
+  for (int g = 0; g < tp.nGR; ++g) {
+    p.grDiv[g] = tp.grDiv[g];
+    p.grSin[g] = tp.grSin[g];
+    p.grSout[g] = tp.grSout[g];
+    p.grLastIn[g] = tp.grLastIn[g];
+    p.grLastOut[g] = tp.grLastOut[g];
+    int r = 0;  // the rank: input strides of a chunk differ between ranks
+    while (r < f.rank && (pd.extent[r] * f.sin[r] != tp.grSin[g] ||
+                          pd.extent[r] * f.sout[r] != tp.grSout[g] || f.dim[r] <= pd.extent[r]))
+      ++r;
+    if (r == f.rank) return 0;
+    p.dim[g] = f.dim[r];
+    p.ext[g] = pd.extent[r];
+    p.sout[g] = f.sout[r];
+  }
+  const std::vector<unsigned char> block =
+      packBlock(b, f.esize, in, const_cast<void*>(out));
+  p.blockBytes = (int)block.size();
+  std::memcpy(p.block, block.data(), block.size());
+  return p.blockBytes + b.smBytes;
+}
+
+// A call's result: two zeroed words of mapped host memory that the kernel adds
+// to and the host reads after its synchronisation, so that a call makes no
+// device allocation, memset or copy (together 150 us a call, with the default
+// pool giving its memory back at every synchronisation).  The slots come from
+// one page, kept until the process exits; a call beyond them allocates its own.
+class ResultSlot {
+ public:
+  ResultSlot() {
+    {
+      std::lock_guard<std::mutex> lk(mutex());
+      std::vector<unsigned long long*>& f = freeSlots();
+      static bool made = false;
+      if (!made) {
+        made = true;
+        if (void* page = allocate(PAGE))
+          for (size_t k = 0; k < PAGE / SLOT; ++k)
+            f.push_back(reinterpret_cast<unsigned long long*>(static_cast<char*>(page) + k * SLOT));
+      }
+      if (!f.empty()) {
+        p_ = f.back();
+        f.pop_back();
+      }
+    }
+    if (p_ == nullptr) {
+      p_ = static_cast<unsigned long long*>(allocate(SLOT));
+      own_ = true;
+    }
+    if (p_ != nullptr) p_[0] = p_[1] = 0;
+  }
+  ~ResultSlot() {
+    if (p_ == nullptr) return;
+    if (own_) {
+      cudaFreeHost(p_);
+      return;
+    }
+    std::lock_guard<std::mutex> lk(mutex());
+    freeSlots().push_back(p_);
+  }
+  ResultSlot(const ResultSlot&) = delete;
+  ResultSlot& operator=(const ResultSlot&) = delete;
+  volatile unsigned long long* host() const { return p_; }
+  // Its address on the current device, nullptr when there is none.
+  unsigned long long* device() const {
+    void* d = nullptr;
+    if (p_ == nullptr || cudaHostGetDevicePointer(&d, p_, 0) != cudaSuccess) return nullptr;
+    return static_cast<unsigned long long*>(d);
+  }
+
+ private:
+  static constexpr size_t PAGE = 4096, SLOT = 64;  // bytes
+  static void* allocate(size_t bytes) {
+    void* p = nullptr;
+    const unsigned flags = cudaHostAllocMapped | cudaHostAllocPortable;
+    return cudaHostAlloc(&p, bytes, flags) == cudaSuccess ? p : nullptr;
+  }
+  static std::mutex& mutex() {
+    static std::mutex m;
+    return m;
+  }
+  static std::vector<unsigned long long*>& freeSlots() {
+    static auto* f = new std::vector<unsigned long long*>();  // lives until the process exits
+    return *f;
+  }
+  unsigned long long* p_ = nullptr;
+  bool own_ = false;
+};
 
 }  // namespace
 }  // namespace lt
@@ -81,51 +429,31 @@ extern "C" int librett_c_verify(int rank, const int* dim, const int* permutation
   if ((uintptr_t)idata % a || (uintptr_t)odata % a) return LIBRETT_INVALID_PARAMETER;
   lt::Fused f;
   lt::fuseRanks(rank, dim, permutation, (int)sizeofType, f);
-  lt::VerifyParams p{};
-  p.rank = f.rank;
-  p.vol = (unsigned long long)f.vol;
-  for (int i = 0; i < f.rank; ++i) {
-    const int r = f.perm[i];
-    p.outD[i] = (unsigned long long)f.dim[r];
-    p.outDim[i] = lt::makeFastDiv(f.dim[r] < (int64_t(1) << 31) ? (uint32_t)f.dim[r] : 1u);
-    p.inStride[i] = f.sin[r];
-  }
-  cudaStream_t s = (cudaStream_t)stream;
-  unsigned long long* d = nullptr;
-  if (cudaMallocAsync(&d, 2 * sizeof(unsigned long long), s) != cudaSuccess)
-    return LIBRETT_INTERNAL_ERROR;
-  const unsigned long long init[2] = {0ull, ~0ull};
-  unsigned long long host[2] = {0ull, ~0ull};
-  cudaError_t err = cudaMemcpyAsync(d, init, sizeof(init), cudaMemcpyHostToDevice, s);
   int sms = 0, dev = 0;
-  if (err == cudaSuccess) err = cudaGetDevice(&dev);
-  if (err == cudaSuccess) err = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  if (err == cudaSuccess) {
-    unsigned long long blocks = (p.vol + 255) / 256;
-    const unsigned long long cap = (unsigned long long)sms * 8;
-    if (blocks > cap) blocks = cap;
-    if (blocks < 1) blocks = 1;
-    switch (sizeofType) {
-      case 4:
-        lt::verifyKernel<4><<<(unsigned)blocks, 256, 0, s>>>(
-            p, (const lt::Word<4>::T*)idata, (const lt::Word<4>::T*)odata, d);
-        break;
-      case 8:
-        lt::verifyKernel<8><<<(unsigned)blocks, 256, 0, s>>>(
-            p, (const lt::Word<8>::T*)idata, (const lt::Word<8>::T*)odata, d);
-        break;
-      default:
-        lt::verifyKernel<16><<<(unsigned)blocks, 256, 0, s>>>(
-            p, (const lt::Word<16>::T*)idata, (const lt::Word<16>::T*)odata, d);
-        break;
-    }
+  if (!lt::currentDevice(dev, sms)) return LIBRETT_INTERNAL_ERROR;
+  cudaStream_t s = (cudaStream_t)stream;
+  lt::ResultSlot slot;
+  unsigned long long* d = slot.device();
+  if (d == nullptr) return LIBRETT_INTERNAL_ERROR;
+  static thread_local lt::VerifyTiles tiles;
+  const int smem = lt::verifyTiles(f, sms, idata, odata, tiles);
+  const lt::VerifyKernel kernel =
+      smem > 0 ? lt::verifyKernelOf(reinterpret_cast<const lt::TileBlock*>(tiles.block)->store) : nullptr;
+  const int occ =
+      kernel ? lt::cachedOccupancy((const void*)kernel, lt::TILE_THREADS, smem) : 0;
+  cudaError_t err;
+  if (occ > 0) {
+    const uint32_t wave = (uint32_t)(sms * occ);
+    kernel<<<tiles.numTiles < wave ? tiles.numTiles : wave, lt::TILE_THREADS, smem, s>>>(tiles, d);
     err = cudaGetLastError();
+  } else {
+    err = lt::verifyElements(f, sms, idata, odata, d, s);
   }
-  if (err == cudaSuccess) err = cudaMemcpyAsync(host, d, sizeof(host), cudaMemcpyDeviceToHost, s);
-  cudaFreeAsync(d, s);
-  if (err == cudaSuccess) err = cudaStreamSynchronize(s);
-  if (err != cudaSuccess) return LIBRETT_INTERNAL_ERROR;
+  // also after an error: a launch may have been made
+  const cudaError_t done = cudaStreamSynchronize(s);
+  if (err != cudaSuccess || done != cudaSuccess) return LIBRETT_INTERNAL_ERROR;
+  const unsigned long long host[2] = {slot.host()[0], slot.host()[1]};
   *mismatches = host[0];
-  if (first_bad) *first_bad = host[0] ? (long long)host[1] : -1;
+  if (first_bad) *first_bad = host[0] ? (long long)~host[1] : -1;
   return LIBRETT_SUCCESS;
 }
