@@ -2,122 +2,495 @@
 // (NFEAT -> 128 -> 128 -> 128 -> 1, ReLU), exposed through the C-ABI on
 // device pointers so that a driver (Python or C++) can run the training
 // loop while every forward, backward, loss and optimiser step runs in these
-// kernels.  The sizes are small (batch <= a few thousand rows, 128-wide
-// layers), so a plain tiled SIMT GEMM is used; there is no tensor-core path.
+// kernels.
+//
+// A training step is a chain of small dependent products (1,024 rows: 0.2
+// GFLOP), so its time is latency: launches, and the serial sum of each output.
+// The forward pass is one launch and the backward pass two:
+//   mlpForwardKernel   a CTA takes R rows through all layers; the weights
+//                      (152 KB) are copied to shared memory at the start, each
+//                      layer waits for its own;
+//   mlpBackwardRows    a CTA takes R rows back through layers 3 and 2 (the
+//                      gradients of their inputs, D2 and D1);
+//   mlpWeightGrads     a cluster of 8 CTAs per 64 x 64 tile of a weight
+//                      gradient, each summing an eighth of the rows, combined
+//                      through distributed shared memory in a fixed order.
+// A layer-by-layer version (a 64 x 64-tiled SGEMM, bias, mask and column-sum
+// kernels, 22 launches) took 721 us for a step of 1,024 rows, most of it in the
+// weight gradients, whose four CTAs each summed all rows one after the other;
+// this takes @@ us.
+//
+// Everything is float32 on the FMA units: an output's products are added in
+// input order, one fused multiply-add each, as a plain loop would.  The tensor
+// cores have no float32 product, and at 0.2 GFLOP they would save nothing.
 //
 // Parameter layout (also used by the host inference in select.cpp): W1
 // [128][NFEAT], b1 [128], W2 [128][128], b2, W3 [128][128], b3, W4 [1][128],
 // b4 [1]; weights row-major [out][in].
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <cmath>
 
+#include "kernels.cuh"
 #include "librett.h"
 #include "librett_c.h"
+#include "plans.h"
 #include "select.h"
 
 namespace lt {
 namespace {
 
+namespace cg = cooperative_groups;
+
+// Kernel arguments carry no __restrict__: a load that the compiler may take for
+// invariant could be moved above dependencyWait.
+
 constexpr int H = MLP_HIDDEN;
-constexpr int BM = 64, BN = 64, BK = 16;
+constexpr int MLP_THREADS = 256;
+static_assert(H == 128, "thread layout");
+constexpr int LD = H + 4;           // padded row of 128 in shared memory (16-byte aligned,
+                                    // rows 33 16-byte units apart: no bank conflict)
+constexpr int XLD = (NFEAT + 3) / 4 * 4;
 
-// C[M][N] = alpha * op(A) * op(B) + beta * C, row-major.
-// op(A)(m,k) = TA ? A[k*lda + m] : A[m*lda + k]
-// op(B)(k,n) = TB ? B[n*ldb + k] : B[k*ldb + n]
-template <bool TA, bool TB>
-__global__ void __launch_bounds__(256)
-sgemmKernel(int M, int N, int K, float alpha, const float* __restrict__ A, int lda,
-            const float* __restrict__ B, int ldb, float beta, float* __restrict__ C, int ldc) {
-  __shared__ float As[BK][BM + 4];
-  __shared__ float Bs[BK][BN + 4];
-  const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
-  const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-  float acc[4][4] = {};
-  for (int k0 = 0; k0 < K; k0 += BK) {
-    for (int i = threadIdx.x; i < BM * BK; i += 256) {
-      const int mm = i % BM, kk = i / BM;
-      const int m = m0 + mm, k = k0 + kk;
-      float v = 0.f;
-      if (m < M && k < K) v = TA ? A[(size_t)k * lda + m] : A[(size_t)m * lda + k];
-      As[kk][mm] = v;
+__device__ __forceinline__ void copyAsync4(float* dst, const float* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(
+                   (uint32_t)__cvta_generic_to_shared(dst)),
+               "l"(src)
+               : "memory");
+}
+
+__device__ __forceinline__ void copyAsync16(float* dst, const float* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(
+                   (uint32_t)__cvta_generic_to_shared(dst)),
+               "l"(src)
+               : "memory");
+}
+
+__device__ __forceinline__ void copyCommit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+
+template <int N>
+__device__ __forceinline__ void copyWait() {
+  asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
+}
+
+// rows x cols of src (row stride sld) into dst (row stride dld) by cp.async, in
+// 16-byte units when vec (cols, sld and dld multiples of 4, src 16-byte aligned).
+__device__ __forceinline__ void copyRows(float* dst, int dld, const float* src, int sld, int rows,
+                                         int cols, bool vec) {
+  if (vec) {
+    const int c4 = cols / 4;
+    for (int i = threadIdx.x; i < rows * c4; i += blockDim.x) {
+      const int r = i / c4, c = (i - r * c4) * 4;
+      copyAsync16(dst + r * dld + c, src + (size_t)r * sld + c);
     }
-    for (int i = threadIdx.x; i < BN * BK; i += 256) {
-      const int nn = i % BN, kk = i / BN;
-      const int n = n0 + nn, k = k0 + kk;
-      float v = 0.f;
-      if (n < N && k < K) v = TB ? B[(size_t)n * ldb + k] : B[(size_t)k * ldb + n];
-      Bs[kk][nn] = v;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int kk = 0; kk < BK; ++kk) {
-      float a[4], b[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) a[i] = As[kk][ty * 4 + i];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) b[j] = Bs[kk][tx * 4 + j];
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] += a[i] * b[j];
-    }
-    __syncthreads();
-  }
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int m = m0 + ty * 4 + i;
-    if (m >= M) continue;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int n = n0 + tx * 4 + j;
-      if (n >= N) continue;
-      float* c = C + (size_t)m * ldc + n;
-      *c = alpha * acc[i][j] + (beta == 0.f ? 0.f : beta * *c);
+  } else {
+    for (int i = threadIdx.x; i < rows * cols; i += blockDim.x) {
+      const int r = i / cols, c = i - r * cols;
+      copyAsync4(dst + r * dld + c, src + (size_t)r * sld + c);
     }
   }
 }
 
-cudaError_t sgemm(bool ta, bool tb, int M, int N, int K, float alpha, const float* A, int lda,
-                  const float* B, int ldb, float beta, float* C, int ldc, cudaStream_t s) {
-  dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
-  if (ta && tb) sgemmKernel<true, true><<<grid, 256, 0, s>>>(M, N, K, alpha, A, lda, B, ldb, beta, C, ldc);
-  else if (ta) sgemmKernel<true, false><<<grid, 256, 0, s>>>(M, N, K, alpha, A, lda, B, ldb, beta, C, ldc);
-  else if (tb) sgemmKernel<false, true><<<grid, 256, 0, s>>>(M, N, K, alpha, A, lda, B, ldb, beta, C, ldc);
-  else sgemmKernel<false, false><<<grid, 256, 0, s>>>(M, N, K, alpha, A, lda, B, ldb, beta, C, ldc);
-  return cudaGetLastError();
+__device__ __forceinline__ bool aligned16(const void* p) { return ((uintptr_t)p & 15) == 0; }
+
+struct Layout {
+  const float *W1, *b1, *W2, *b2, *W3, *b3, *W4, *b4;
+};
+
+__host__ __device__ Layout layout(const float* p) {
+  Layout L;
+  L.W1 = p;
+  L.b1 = L.W1 + H * NFEAT;
+  L.W2 = L.b1 + H;
+  L.b2 = L.W2 + H * H;
+  L.W3 = L.b2 + H;
+  L.b3 = L.W3 + H * H;
+  L.W4 = L.b3 + H;
+  L.b4 = L.W4 + H;
+  return L;
 }
 
-// Y[b][o] = act(Y[b][o] + bias[o])
-__global__ void biasActKernel(float* Y, const float* bias, int rows, int cols, int relu) {
-  const size_t n = (size_t)rows * cols;
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
-       i += (size_t)gridDim.x * blockDim.x) {
-    float v = Y[i] + bias[i % cols];
-    Y[i] = (relu && v < 0.f) ? 0.f : v;
+// Rows a CTA takes: the fewest that fill the device once, so that small batches
+// spread over it and large ones read the weights as seldom as possible.
+int rowsPerCta(int batch, int sms) {
+  return batch <= 8 * sms ? 8 : batch <= 16 * sms ? 16 : 32;
+}
+
+// A thread's outputs of a layer for R rows and 128 columns: TM rows from
+// row(), TN columns col() + 64 * j (TN 2) or one column.
+template <int R>
+struct Place {
+  static constexpr int TN = R == 32 ? 2 : 1;
+  static constexpr int TM = R * H / MLP_THREADS / TN;
+  static constexpr int COLS = H / TN;
+  __device__ static int col() { return threadIdx.x % COLS; }
+  __device__ static int row() { return threadIdx.x / COLS * TM; }
+};
+
+// acc += in[rows][0..K) * w[cols][0..K)^T, both padded rows of LD; products in
+// input order.
+template <int R>
+__device__ __forceinline__ void layerTimesRows(const float* in, const float* w,
+                                               float (&acc)[Place<R>::TM][Place<R>::TN]) {
+  using P = Place<R>;
+  const float* a = in + P::row() * LD;
+  const float* b = w + P::col() * LD;
+#pragma unroll 4
+  for (int k = 0; k < H; k += 4) {
+    float4 wv[P::TN];
+#pragma unroll
+    for (int j = 0; j < P::TN; ++j)
+      wv[j] = *reinterpret_cast<const float4*>(b + j * P::COLS * LD + k);
+#pragma unroll
+    for (int i = 0; i < P::TM; ++i) {
+      const float4 av = *reinterpret_cast<const float4*>(a + i * LD + k);
+#pragma unroll
+      for (int j = 0; j < P::TN; ++j) {
+        acc[i][j] = __fmaf_rn(av.x, wv[j].x, acc[i][j]);
+        acc[i][j] = __fmaf_rn(av.y, wv[j].y, acc[i][j]);
+        acc[i][j] = __fmaf_rn(av.z, wv[j].z, acc[i][j]);
+        acc[i][j] = __fmaf_rn(av.w, wv[j].w, acc[i][j]);
+      }
+    }
   }
 }
 
-// dZ = dA where the layer's activation A is positive, else 0 (ReLU').
-__global__ void reluMaskKernel(float* dA, const float* A, size_t n) {
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
-       i += (size_t)gridDim.x * blockDim.x)
-    if (!(A[i] > 0.f)) dA[i] = 0.f;
+// acc += in[rows][0..H) * w[0..H)[cols]: w in rows of H, one per input.
+template <int R>
+__device__ __forceinline__ void layerTimesCols(const float* in, const float* w,
+                                               float (&acc)[Place<R>::TM][Place<R>::TN]) {
+  using P = Place<R>;
+  const float* a = in + P::row() * LD;
+  const float* b = w + P::col();
+#pragma unroll 4
+  for (int k = 0; k < H; k += 4) {
+    float wv[4][P::TN];
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+#pragma unroll
+      for (int j = 0; j < P::TN; ++j) wv[q][j] = b[(k + q) * H + j * P::COLS];
+#pragma unroll
+    for (int i = 0; i < P::TM; ++i) {
+      const float4 av = *reinterpret_cast<const float4*>(a + i * LD + k);
+#pragma unroll
+      for (int j = 0; j < P::TN; ++j) {
+        acc[i][j] = __fmaf_rn(av.x, wv[0][j], acc[i][j]);
+        acc[i][j] = __fmaf_rn(av.y, wv[1][j], acc[i][j]);
+        acc[i][j] = __fmaf_rn(av.z, wv[2][j], acc[i][j]);
+        acc[i][j] = __fmaf_rn(av.w, wv[3][j], acc[i][j]);
+      }
+    }
+  }
 }
 
-// out[o] = sum_b D[b][o]; one block per column.
-__global__ void colSumKernel(const float* D, int rows, int cols, float* out) {
-  __shared__ float red[256];
-  const int o = blockIdx.x;
-  float s = 0.f;
-  for (int b = threadIdx.x; b < rows; b += blockDim.x) s += D[(size_t)b * cols + o];
-  red[threadIdx.x] = s;
+template <int R>
+struct ForwardShared {
+  float W2[H * LD], W3[H * LD];
+  float X[R * XLD];
+  float A[R * LD], B[R * LD];
+  float W1[H * NFEAT];
+  float b1[H], b2[H], b3[H], W4[H];
+};
+
+// Bias, ReLU; the activation to shared memory and to global memory.
+template <int R>
+__device__ __forceinline__ void activate(const float (&acc)[Place<R>::TM][Place<R>::TN],
+                                         const float* bias, float* shared, float* global, int rows) {
+  using P = Place<R>;
+#pragma unroll
+  for (int i = 0; i < P::TM; ++i)
+#pragma unroll
+    for (int j = 0; j < P::TN; ++j) {
+      const int r = P::row() + i, c = P::col() + j * P::COLS;
+      float v = acc[i][j] + bias[c];
+      v = v < 0.f ? 0.f : v;
+      shared[r * LD + c] = v;
+      if (r < rows) global[(size_t)r * H + c] = v;
+    }
+}
+
+template <int R>
+__global__ void __launch_bounds__(MLP_THREADS)
+mlpForwardKernel(const float* params, const float* X, int batch,
+                 float* ws, float* out) {
+  using P = Place<R>;
+  extern __shared__ __align__(16) unsigned char smraw[];
+  ForwardShared<R>& s = *reinterpret_cast<ForwardShared<R>*>(smraw);
+  dependencyRelease();
+  const int r0 = blockIdx.x * R, rows = min(R, batch - r0);
+  const Layout L = layout(params);
+  const bool vec = aligned16(params);
+  dependencyWait();
+  copyRows(s.X, XLD, X + (size_t)r0 * NFEAT, NFEAT, rows, NFEAT, false);
+  copyRows(s.W1, H * NFEAT, L.W1, H * NFEAT, 1, H * NFEAT, vec && H * NFEAT % 4 == 0);
+  copyRows(s.b1, H, L.b1, H, 1, H, vec);
+  copyRows(s.b2, H, L.b2, H, 1, H, vec);
+  copyRows(s.b3, H, L.b3, H, 1, H, vec);
+  copyRows(s.W4, H, L.W4, H, 1, H, vec);
+  copyCommit();
+  copyRows(s.W2, LD, L.W2, H, H, H, vec);
+  copyCommit();
+  copyRows(s.W3, LD, L.W3, H, H, H, vec);
+  copyCommit();
+  float* A1 = ws + (size_t)r0 * H;
+  float* A2 = A1 + (size_t)batch * H;
+  float* A3 = A2 + (size_t)batch * H;
+  // rows past the batch: any finite input
+  for (int i = rows * XLD + threadIdx.x; i < R * XLD; i += MLP_THREADS) s.X[i] = 0.f;
+  copyWait<2>();
   __syncthreads();
-  for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-    if (threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
-    __syncthreads();
+  {
+    float acc[P::TM][P::TN] = {};
+    const float* a = s.X + P::row() * XLD;
+    const float* w = s.W1 + P::col() * NFEAT;  // NFEAT odd: no bank conflict
+#pragma unroll 8
+    for (int k = 0; k < NFEAT; ++k) {
+      float wv[P::TN];
+#pragma unroll
+      for (int j = 0; j < P::TN; ++j) wv[j] = w[j * P::COLS * NFEAT + k];
+#pragma unroll
+      for (int i = 0; i < P::TM; ++i)
+#pragma unroll
+        for (int j = 0; j < P::TN; ++j) acc[i][j] = __fmaf_rn(a[i * XLD + k], wv[j], acc[i][j]);
+    }
+    activate<R>(acc, s.b1, s.A, A1, rows);
   }
-  if (threadIdx.x == 0) out[o] = red[0];
+  copyWait<1>();
+  __syncthreads();
+  {
+    float acc[P::TM][P::TN] = {};
+    layerTimesRows<R>(s.A, s.W2, acc);
+    activate<R>(acc, s.b2, s.B, A2, rows);
+  }
+  copyWait<0>();
+  __syncthreads();
+  {
+    float acc[P::TM][P::TN] = {};
+    layerTimesRows<R>(s.B, s.W3, acc);
+    activate<R>(acc, s.b3, s.A, A3, rows);
+  }
+  __syncthreads();
+  if ((int)threadIdx.x < rows) {
+    const float* a = s.A + threadIdx.x * LD;
+    float v = 0.f;
+#pragma unroll 8
+    for (int k = 0; k < H; ++k) v = __fmaf_rn(a[k], s.W4[k], v);
+    out[r0 + threadIdx.x] = v + *L.b4;
+  }
+}
+
+// The gradient of the network's output with respect to activation 3 of a row,
+// where that is positive (ReLU'): dout * W4.
+__device__ __forceinline__ float outputGrad(float a3, float dout, float w4) {
+  return a3 > 0.f ? __fmaf_rn(dout, w4, 0.f) : 0.f;
+}
+
+template <int R>
+struct BackwardShared {
+  float W3[H * H], W2[H * H];
+  float D[R * LD], E[R * LD];
+};
+
+// The product masked with the layer's activation; to shared memory (the next
+// product's input) and to global memory.
+template <int R>
+__device__ __forceinline__ void maskGrad(const float (&acc)[Place<R>::TM][Place<R>::TN],
+                                         const float* act, float* shared, float* global, int rows) {
+  using P = Place<R>;
+#pragma unroll
+  for (int i = 0; i < P::TM; ++i)
+#pragma unroll
+    for (int j = 0; j < P::TN; ++j) {
+      const int r = P::row() + i, c = P::col() + j * P::COLS;
+      float v = 0.f;
+      if (r < rows) {
+        v = act[(size_t)r * H + c] > 0.f ? acc[i][j] : 0.f;
+        global[(size_t)r * H + c] = v;
+      }
+      if (shared) shared[r * LD + c] = v;
+    }
+}
+
+// D2 = (D3 W3) masked by A2 and D1 = (D2 W2) masked by A1, with D3 = dout W4
+// masked by A3.  D2 goes to the workspace's fifth part, D1 to its fourth.
+template <int R>
+__global__ void __launch_bounds__(MLP_THREADS)
+mlpBackwardRows(const float* params, int batch, float* ws,
+                const float* dout) {
+  using P = Place<R>;
+  extern __shared__ __align__(16) unsigned char smraw[];
+  BackwardShared<R>& s = *reinterpret_cast<BackwardShared<R>*>(smraw);
+  dependencyRelease();
+  const int r0 = blockIdx.x * R, rows = min(R, batch - r0);
+  const Layout L = layout(params);
+  const bool vec = aligned16(params);
+  dependencyWait();
+  copyRows(s.W3, H, L.W3, H, H, H, vec);
+  copyCommit();
+  copyRows(s.W2, H, L.W2, H, H, H, vec);
+  copyCommit();
+  const size_t part = (size_t)batch * H;
+  const float* A1 = ws + (size_t)r0 * H;
+  const float* A2 = A1 + part;
+  const float* A3 = A2 + part;
+  float* D1 = ws + 3 * part + (size_t)r0 * H;
+  float* D2 = D1 + part;
+  for (int i = threadIdx.x; i < R * H; i += MLP_THREADS) {
+    const int r = i / H, c = i % H;
+    s.D[r * LD + c] = r < rows ? outputGrad(A3[i], dout[r0 + r], L.W4[c]) : 0.f;
+  }
+  copyWait<1>();
+  __syncthreads();
+  {
+    float acc[P::TM][P::TN] = {};
+    layerTimesCols<R>(s.D, s.W3, acc);
+    maskGrad<R>(acc, A2, s.E, D2, rows);
+  }
+  copyWait<0>();
+  __syncthreads();
+  {
+    float acc[P::TM][P::TN] = {};
+    layerTimesCols<R>(s.E, s.W2, acc);
+    maskGrad<R>(acc, A1, nullptr, D1, rows);
+  }
+}
+
+// Weight gradients: gW[o][i] = sum over rows of D[row][o] * In[row][i] and gb[o]
+// = sum of D[row][o], in tiles of GT x GT.  A cluster of GC CTAs shares a tile;
+// CTA c takes GROWS-row chunks c, c + GC, ... of the batch.
+constexpr int GT = 64, GC = 8, GROWS = 64;
+constexpr int GLD = GT + 4;
+// tiles: W3 and W2 four each, W1 two (NFEAT <= GT), the output layer one
+constexpr int GTILES = 2 * (H / GT) * (H / GT) + H / GT + 1;
+static_assert(NFEAT <= GT, "one tile covers the features");
+
+struct GradShared {
+  float D[GROWS * GLD], In[GROWS * GLD];  // a chunk; then the CTA's partial tile in D
+  float dout[GROWS], W4[H];
+  float bias[GT];
+};
+
+__global__ void __cluster_dims__(GC, 1, 1) __launch_bounds__(MLP_THREADS)
+mlpWeightGrads(const float* params, const float* X, int batch,
+               const float* ws, const float* dout,
+               float* grads) {
+  extern __shared__ __align__(16) unsigned char smraw[];
+  GradShared& s = *reinterpret_cast<GradShared*>(smraw);
+  cg::cluster_group cluster = cg::this_cluster();
+  dependencyRelease();
+  const int tile = blockIdx.x / GC, rank = (int)cluster.block_rank();
+  const int tid = threadIdx.x;
+  const Layout L = layout(params);
+  const size_t part = (size_t)batch * H;
+  // which gradient: its D and In with their first column and width, and where
+  // the tile goes
+  constexpr int PER = (H / GT) * (H / GT);
+  int layer, o0, i0 = 0, width = GT;
+  const float *Dg, *Ig;
+  int ild = H;
+  if (tile < 2 * PER) {
+    layer = tile < PER ? 3 : 2;
+    const int t = tile % PER;
+    o0 = t / (H / GT) * GT;
+    i0 = t % (H / GT) * GT;
+    Dg = layer == 3 ? ws + 2 * part : ws + 4 * part;  // layer 3: A3, made D3 below
+    Ig = layer == 3 ? ws + part : ws;
+  } else if (tile < 2 * PER + H / GT) {
+    layer = 1;
+    o0 = (tile - 2 * PER) * GT;
+    Dg = ws + 3 * part;
+    Ig = X;
+    ild = NFEAT;
+    width = NFEAT;
+  } else {
+    layer = 4;
+    o0 = 0;
+    Dg = Ig = ws + 2 * part;  // A3
+  }
+  const bool vec = aligned16(ws);
+  const int tx = tid % 16, ty = tid / 16;
+  float acc[4][4] = {};
+  float accB = 0.f;  // layer 4: output column tid < H, else its bias; others: bias o0 + tid
+  dependencyWait();
+  if (layer == 3) copyRows(s.W4, H, L.W4, H, 1, H, aligned16(params));
+  for (int b0 = rank * GROWS; b0 < batch; b0 += GC * GROWS) {
+    const int rows = min(GROWS, batch - b0);
+    if (layer == 4) {
+      // one row of gradients: thread j sums column j, thread H the bias
+      if (tid <= H)
+#pragma unroll 8
+        for (int r = 0; r < rows; ++r) {
+          const float d = dout[b0 + r];
+          accB = tid < H ? __fmaf_rn(d, Dg[(size_t)(b0 + r) * H + tid], accB) : accB + d;
+        }
+      continue;
+    }
+    copyRows(s.D, GLD, Dg + (size_t)b0 * H + o0, H, rows, GT, vec);
+    copyRows(s.In, GLD, Ig + (size_t)b0 * ild + i0, ild, rows, width, vec && layer != 1);
+    if (layer == 3) copyRows(s.dout, GROWS, dout + b0, GROWS, 1, rows, false);
+    copyCommit();
+    copyWait<0>();
+    __syncthreads();
+    if (layer == 3) {
+      for (int i = tid; i < rows * GT; i += MLP_THREADS) {
+        const int r = i / GT, c = i % GT;
+        s.D[r * GLD + c] = outputGrad(s.D[r * GLD + c], s.dout[r], s.W4[o0 + c]);
+      }
+      __syncthreads();
+    }
+    if (tx * 4 < width)
+#pragma unroll 4
+      for (int r = 0; r < rows; ++r) {
+        const float4 d = *reinterpret_cast<const float4*>(s.D + r * GLD + ty * 4);
+        const float4 x = *reinterpret_cast<const float4*>(s.In + r * GLD + tx * 4);
+        const float dv[4] = {d.x, d.y, d.z, d.w}, xv[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) acc[i][j] = __fmaf_rn(dv[i], xv[j], acc[i][j]);
+      }
+    if (i0 == 0 && tid < GT)
+      for (int r = 0; r < rows; ++r) accB += s.D[r * GLD + tid];
+    __syncthreads();  // the next chunk reuses the buffers
+  }
+  // partial sums to shared memory (layer 4: one row of H columns and the bias)
+  float* partial = s.D;
+  if (layer == 4) {
+    if (tid <= H) partial[tid] = accB;
+  } else {
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      *reinterpret_cast<float4*>(partial + (ty * 4 + i) * GLD + tx * 4) =
+          make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+    if (tid < GT) s.bias[tid] = accB;
+  }
+  cluster.sync();
+  // CTA `rank` adds the eight partial sums of its share, in rank order
+  auto total = [&](float* at) {
+    float v = 0.f;
+#pragma unroll
+    for (int c = 0; c < GC; ++c) v += *cluster.map_shared_rank(at, c);
+    return v;
+  };
+  const Layout G = layout(grads);
+  if (layer == 4) {
+    for (int j = rank * MLP_THREADS + tid; j <= H; j += GC * MLP_THREADS) {
+      const float v = total(partial + j);
+      *const_cast<float*>(j < H ? G.W4 + j : G.b4) = v;
+    }
+  } else {
+    float* gW = const_cast<float*>(layer == 3 ? G.W3 : layer == 2 ? G.W2 : G.W1);
+    float* gb = const_cast<float*>(layer == 3 ? G.b3 : layer == 2 ? G.b2 : G.b1);
+    const int ld = layer == 1 ? NFEAT : H;
+    constexpr int OUT = GT / GC;  // rows of the tile
+    for (int i = tid; i < OUT * width; i += MLP_THREADS) {
+      const int o = rank * OUT + i / width, c = i % width;
+      gW[(size_t)(o0 + o) * ld + i0 + c] = total(partial + o * GLD + c);
+    }
+    if (i0 == 0 && tid < OUT) gb[o0 + rank * OUT + tid] = total(s.bias + rank * OUT + tid);
+  }
+  cluster.sync();  // no CTA leaves while another reads its shared memory
 }
 
 // dout[b] = 2 (out[b] - y[b]) / batch; *loss += sum (out - y)^2 / batch.
@@ -125,6 +498,8 @@ __global__ void mseGradKernel(const float* out, const float* y, int batch, float
                               float* loss) {
   __shared__ float red[256];
   float s = 0.f;
+  dependencyRelease();
+  dependencyWait();
   for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < batch; b += gridDim.x * blockDim.x) {
     const float d = out[b] - y[b];
     dout[b] = 2.f * d / batch;
@@ -142,6 +517,8 @@ __global__ void mseGradKernel(const float* out, const float* y, int batch, float
 // Adam (Kingma & Ba, 2015) with bias correction.
 __global__ void adamKernel(float* p, const float* g, float* m, float* v, int n, float lr,
                            float b1, float b2, float eps, float c1, float c2) {
+  dependencyRelease();
+  dependencyWait();
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const float gi = g[i];
     const float mi = b1 * m[i] + (1.f - b1) * gi;
@@ -157,21 +534,18 @@ int gridFor(size_t n) {
   return (int)(g > 4096 ? 4096 : (g < 1 ? 1 : g));
 }
 
-struct Layout {
-  const float *W1, *b1, *W2, *b2, *W3, *b3, *W4, *b4;
-};
-
-Layout layout(const float* p) {
-  Layout L;
-  L.W1 = p;
-  L.b1 = L.W1 + H * NFEAT;
-  L.W2 = L.b1 + H;
-  L.b2 = L.W2 + H * H;
-  L.W3 = L.b2 + H;
-  L.b3 = L.W3 + H * H;
-  L.W4 = L.b3 + H;
-  L.b4 = L.W4 + H;
-  return L;
+// Launches kernel<R> for the rows a CTA takes; shared: its structure by R.
+template <typename K8, typename K16, typename K32, typename... Args>
+cudaError_t launchRowsOf(int batch, cudaStream_t s, size_t sm8, size_t sm16, size_t sm32, K8 k8,
+                         K16 k16, K32 k32, Args... args) {
+  int dev = 0, sms = 0;
+  if (!currentDevice(dev, sms)) return cudaErrorInvalidDevice;
+  const int R = rowsPerCta(batch, sms);
+  const size_t smem = R == 8 ? sm8 : R == 16 ? sm16 : sm32;
+  const auto kernel = R == 8 ? k8 : R == 16 ? k16 : k32;
+  if (cachedOccupancy((const void*)kernel, MLP_THREADS, (int)smem) < 1)
+    return cudaErrorInvalidConfiguration;
+  return launchDependent(kernel, (unsigned)((batch + R - 1) / R), MLP_THREADS, smem, s, args...);
 }
 
 }  // namespace
@@ -189,21 +563,11 @@ int librett_c_mlp_forward(const float* params, const float* X, int batch, float*
                           void* stream) {
   using namespace lt;
   if (!params || !X || !ws || !out || batch < 1) return LIBRETT_INVALID_PARAMETER;
-  cudaStream_t s = (cudaStream_t)stream;
-  const Layout L = layout(params);
-  float* A1 = ws;
-  float* A2 = A1 + (size_t)batch * H;
-  float* A3 = A2 + (size_t)batch * H;
-  const int g = gridFor((size_t)batch * H);
-  if (sgemm(false, true, batch, H, NFEAT, 1.f, X, NFEAT, L.W1, NFEAT, 0.f, A1, H, s)) return LIBRETT_INTERNAL_ERROR;
-  biasActKernel<<<g, 256, 0, s>>>(A1, L.b1, batch, H, 1);
-  if (sgemm(false, true, batch, H, H, 1.f, A1, H, L.W2, H, 0.f, A2, H, s)) return LIBRETT_INTERNAL_ERROR;
-  biasActKernel<<<g, 256, 0, s>>>(A2, L.b2, batch, H, 1);
-  if (sgemm(false, true, batch, H, H, 1.f, A2, H, L.W3, H, 0.f, A3, H, s)) return LIBRETT_INTERNAL_ERROR;
-  biasActKernel<<<g, 256, 0, s>>>(A3, L.b3, batch, H, 1);
-  if (sgemm(false, true, batch, 1, H, 1.f, A3, H, L.W4, H, 0.f, out, 1, s)) return LIBRETT_INTERNAL_ERROR;
-  biasActKernel<<<gridFor(batch), 256, 0, s>>>(out, L.b4, batch, 1, 0);
-  return cudaGetLastError() == cudaSuccess ? LIBRETT_SUCCESS : LIBRETT_INTERNAL_ERROR;
+  const cudaError_t err = launchRowsOf(
+      batch, (cudaStream_t)stream, sizeof(ForwardShared<8>), sizeof(ForwardShared<16>),
+      sizeof(ForwardShared<32>), mlpForwardKernel<8>, mlpForwardKernel<16>, mlpForwardKernel<32>,
+      params, X, batch, ws, out);
+  return err == cudaSuccess ? LIBRETT_SUCCESS : LIBRETT_INTERNAL_ERROR;
 }
 
 int librett_c_mlp_backward(const float* params, const float* X, int batch, float* ws,
@@ -211,58 +575,31 @@ int librett_c_mlp_backward(const float* params, const float* X, int batch, float
   using namespace lt;
   if (!params || !X || !ws || !dout || !grads || batch < 1) return LIBRETT_INVALID_PARAMETER;
   cudaStream_t s = (cudaStream_t)stream;
-  const Layout L = layout(params);
-  float* gW1 = grads;
-  float* gb1 = gW1 + H * NFEAT;
-  float* gW2 = gb1 + H;
-  float* gb2 = gW2 + H * H;
-  float* gW3 = gb2 + H;
-  float* gb3 = gW3 + H * H;
-  float* gW4 = gb3 + H;
-  float* gb4 = gW4 + H;
-  const float* A1 = ws;
-  const float* A2 = A1 + (size_t)batch * H;
-  const float* A3 = A2 + (size_t)batch * H;
-  float* dA = ws + 3 * (size_t)batch * H;
-  float* dB = dA + (size_t)batch * H;
-  const size_t n = (size_t)batch * H;
-  const int g = gridFor(n);
-  // output layer
-  if (sgemm(true, false, 1, H, batch, 1.f, dout, 1, A3, H, 0.f, gW4, H, s)) return LIBRETT_INTERNAL_ERROR;
-  colSumKernel<<<1, 256, 0, s>>>(dout, batch, 1, gb4);
-  if (sgemm(false, false, batch, H, 1, 1.f, dout, 1, L.W4, H, 0.f, dA, H, s)) return LIBRETT_INTERNAL_ERROR;
-  reluMaskKernel<<<g, 256, 0, s>>>(dA, A3, n);
-  // layer 3
-  if (sgemm(true, false, H, H, batch, 1.f, dA, H, A2, H, 0.f, gW3, H, s)) return LIBRETT_INTERNAL_ERROR;
-  colSumKernel<<<H, 256, 0, s>>>(dA, batch, H, gb3);
-  if (sgemm(false, false, batch, H, H, 1.f, dA, H, L.W3, H, 0.f, dB, H, s)) return LIBRETT_INTERNAL_ERROR;
-  reluMaskKernel<<<g, 256, 0, s>>>(dB, A2, n);
-  // layer 2
-  if (sgemm(true, false, H, H, batch, 1.f, dB, H, A1, H, 0.f, gW2, H, s)) return LIBRETT_INTERNAL_ERROR;
-  colSumKernel<<<H, 256, 0, s>>>(dB, batch, H, gb2);
-  if (sgemm(false, false, batch, H, H, 1.f, dB, H, L.W2, H, 0.f, dA, H, s)) return LIBRETT_INTERNAL_ERROR;
-  reluMaskKernel<<<g, 256, 0, s>>>(dA, A1, n);
-  // layer 1
-  if (sgemm(true, false, H, NFEAT, batch, 1.f, dA, H, X, NFEAT, 0.f, gW1, NFEAT, s)) return LIBRETT_INTERNAL_ERROR;
-  colSumKernel<<<H, 256, 0, s>>>(dA, batch, H, gb1);
-  return cudaGetLastError() == cudaSuccess ? LIBRETT_SUCCESS : LIBRETT_INTERNAL_ERROR;
+  cudaError_t err = launchRowsOf(
+      batch, s, sizeof(BackwardShared<8>), sizeof(BackwardShared<16>), sizeof(BackwardShared<32>),
+      mlpBackwardRows<8>, mlpBackwardRows<16>, mlpBackwardRows<32>, params, batch, ws, dout);
+  if (err == cudaSuccess)
+    err = launchDependent(mlpWeightGrads, GTILES * GC, MLP_THREADS, sizeof(GradShared), s, params, X,
+                          batch, (const float*)ws, dout, grads);
+  return err == cudaSuccess ? LIBRETT_SUCCESS : LIBRETT_INTERNAL_ERROR;
 }
 
 int librett_c_mlp_mse_grad(const float* out, const float* y, int batch, float* dout, float* loss,
                            void* stream) {
   if (!out || !y || !dout || batch < 1) return LIBRETT_INVALID_PARAMETER;
-  lt::mseGradKernel<<<lt::gridFor(batch), 256, 0, (cudaStream_t)stream>>>(out, y, batch, dout,
-                                                                            loss);
-  return cudaGetLastError() == cudaSuccess ? LIBRETT_SUCCESS : LIBRETT_INTERNAL_ERROR;
+  const cudaError_t err = lt::launchDependent(lt::mseGradKernel, (unsigned)lt::gridFor(batch), 256, 0,
+                                              (cudaStream_t)stream, out, y, batch, dout, loss);
+  return err == cudaSuccess ? LIBRETT_SUCCESS : LIBRETT_INTERNAL_ERROR;
 }
 
 int librett_c_mlp_adam(float* params, const float* grads, float* m, float* v, int n, float lr,
                        float beta1, float beta2, float eps, int step, void* stream) {
   if (!params || !grads || !m || !v || n < 1 || step < 1) return LIBRETT_INVALID_PARAMETER;
   const float c1 = 1.f - powf(beta1, (float)step), c2 = 1.f - powf(beta2, (float)step);
-  lt::adamKernel<<<lt::gridFor(n), 256, 0, (cudaStream_t)stream>>>(params, grads, m, v, n, lr,
-                                                                     beta1, beta2, eps, c1, c2);
-  return cudaGetLastError() == cudaSuccess ? LIBRETT_SUCCESS : LIBRETT_INTERNAL_ERROR;
+  const cudaError_t err =
+      lt::launchDependent(lt::adamKernel, (unsigned)lt::gridFor(n), 256, 0, (cudaStream_t)stream, params,
+                          grads, m, v, n, lr, beta1, beta2, eps, c1, c2);
+  return err == cudaSuccess ? LIBRETT_SUCCESS : LIBRETT_INTERNAL_ERROR;
 }
 
 }  // extern "C"
