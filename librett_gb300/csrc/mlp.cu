@@ -74,6 +74,24 @@ __device__ __forceinline__ void copyWait() {
   asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
 }
 
+// A whole H x H matrix into dst (row stride dld).  Every CTA copies the same
+// matrix at the same time: each starts at another row, so that they do not all
+// ask the same L2 slice.
+__device__ __forceinline__ void copyMatrix(float* dst, int dld, const float* src, bool vec) {
+  const int start = (int)(blockIdx.x * 8);
+  if (vec) {
+    for (int i = threadIdx.x; i < H * H / 4; i += blockDim.x) {
+      const int r = (i / (H / 4) + start) % H, c = i % (H / 4) * 4;
+      copyAsync16(dst + r * dld + c, src + r * H + c);
+    }
+  } else {
+    for (int i = threadIdx.x; i < H * H; i += blockDim.x) {
+      const int r = (i / H + start) % H, c = i % H;
+      copyAsync4(dst + r * dld + c, src + r * H + c);
+    }
+  }
+}
+
 // rows x cols of src (row stride sld) into dst (row stride dld) by cp.async, in
 // 16-byte units when vec (cols, sld and dld multiples of 4, src 16-byte aligned).
 __device__ __forceinline__ void copyRows(float* dst, int dld, const float* src, int sld, int rows,
@@ -229,9 +247,9 @@ mlpForwardKernel(const float* params, const float* X, int batch,
   copyRows(s.b3, H, L.b3, H, 1, H, vec);
   copyRows(s.W4, H, L.W4, H, 1, H, vec);
   copyCommit();
-  copyRows(s.W2, LD, L.W2, H, H, H, vec);
+  copyMatrix(s.W2, LD, L.W2, vec);
   copyCommit();
-  copyRows(s.W3, LD, L.W3, H, H, H, vec);
+  copyMatrix(s.W3, LD, L.W3, vec);
   copyCommit();
   float* A1 = ws + (size_t)r0 * H;
   float* A2 = A1 + (size_t)batch * H;
@@ -275,7 +293,14 @@ mlpForwardKernel(const float* params, const float* X, int batch,
     const float* a = s.A + threadIdx.x * LD;
     float v = 0.f;
 #pragma unroll 8
-    for (int k = 0; k < H; ++k) v = __fmaf_rn(a[k], s.W4[k], v);
+    for (int k = 0; k < H; k += 4) {
+      const float4 av = *reinterpret_cast<const float4*>(a + k);
+      const float4 wv = *reinterpret_cast<const float4*>(s.W4 + k);
+      v = __fmaf_rn(av.x, wv.x, v);
+      v = __fmaf_rn(av.y, wv.y, v);
+      v = __fmaf_rn(av.z, wv.z, v);
+      v = __fmaf_rn(av.w, wv.w, v);
+    }
     out[r0 + threadIdx.x] = v + *L.b4;
   }
 }
@@ -292,24 +317,14 @@ struct BackwardShared {
   float D[R * LD], E[R * LD];
 };
 
-// The product masked with the layer's activation; to shared memory (the next
-// product's input) and to global memory.
-template <int R>
-__device__ __forceinline__ void maskGrad(const float (&acc)[Place<R>::TM][Place<R>::TN],
-                                         const float* act, float* shared, float* global, int rows) {
+// A thread's outputs' places in an activation or gradient of H columns.
+template <int R, typename F>
+__device__ __forceinline__ void forOutputs(F f) {
   using P = Place<R>;
 #pragma unroll
   for (int i = 0; i < P::TM; ++i)
 #pragma unroll
-    for (int j = 0; j < P::TN; ++j) {
-      const int r = P::row() + i, c = P::col() + j * P::COLS;
-      float v = 0.f;
-      if (r < rows) {
-        v = act[(size_t)r * H + c] > 0.f ? acc[i][j] : 0.f;
-        global[(size_t)r * H + c] = v;
-      }
-      if (shared) shared[r * LD + c] = v;
-    }
+    for (int j = 0; j < P::TN; ++j) f(i, j, P::row() + i, P::col() + j * P::COLS);
 }
 
 // D2 = (D3 W3) masked by A2 and D1 = (D2 W2) masked by A1, with D3 = dout W4
@@ -326,9 +341,9 @@ mlpBackwardRows(const float* params, int batch, float* ws,
   const Layout L = layout(params);
   const bool vec = aligned16(params);
   dependencyWait();
-  copyRows(s.W3, H, L.W3, H, H, H, vec);
+  copyMatrix(s.W3, H, L.W3, vec);
   copyCommit();
-  copyRows(s.W2, H, L.W2, H, H, H, vec);
+  copyMatrix(s.W2, H, L.W2, vec);
   copyCommit();
   const size_t part = (size_t)batch * H;
   const float* A1 = ws + (size_t)r0 * H;
@@ -340,26 +355,39 @@ mlpBackwardRows(const float* params, int batch, float* ws,
     const int r = i / H, c = i % H;
     s.D[r * LD + c] = r < rows ? outputGrad(A3[i], dout[r0 + r], L.W4[c]) : 0.f;
   }
+  // the masks of both products, read while the weights are on their way
+  bool on2[P::TM][P::TN], on1[P::TM][P::TN];
+  forOutputs<R>([&](int i, int j, int r, int c) {
+    on2[i][j] = r < rows && A2[(size_t)r * H + c] > 0.f;
+    on1[i][j] = r < rows && A1[(size_t)r * H + c] > 0.f;
+  });
   copyWait<1>();
   __syncthreads();
   {
     float acc[P::TM][P::TN] = {};
     layerTimesCols<R>(s.D, s.W3, acc);
-    maskGrad<R>(acc, A2, s.E, D2, rows);
+    forOutputs<R>([&](int i, int j, int r, int c) {
+      const float v = on2[i][j] ? acc[i][j] : 0.f;
+      s.E[r * LD + c] = v;
+      if (r < rows) D2[(size_t)r * H + c] = v;
+    });
   }
   copyWait<0>();
   __syncthreads();
   {
     float acc[P::TM][P::TN] = {};
     layerTimesCols<R>(s.E, s.W2, acc);
-    maskGrad<R>(acc, A1, nullptr, D1, rows);
+    forOutputs<R>([&](int i, int j, int r, int c) {
+      if (r < rows) D1[(size_t)r * H + c] = on1[i][j] ? acc[i][j] : 0.f;
+    });
   }
 }
 
 // Weight gradients: gW[o][i] = sum over rows of D[row][o] * In[row][i] and gb[o]
 // = sum of D[row][o], in tiles of GT x GT.  A cluster of GC CTAs shares a tile;
-// CTA c takes GROWS-row chunks c, c + GC, ... of the batch.
-constexpr int GT = 64, GC = 8, GROWS = 64;
+// CTA c takes GROWS-row chunks c, c + GC, ... of the batch, each half of its
+// threads every other row.
+constexpr int GT = 64, GC = 8, GROWS = 128, GTHREADS = 512;
 constexpr int GLD = GT + 4;
 // tiles: W3 and W2 four each, W1 two (NFEAT <= GT), the output layer one
 constexpr int GTILES = 2 * (H / GT) * (H / GT) + H / GT + 1;
@@ -370,8 +398,9 @@ struct GradShared {
   float dout[GROWS], W4[H];
   float bias[GT];
 };
+static_assert(GROWS * GLD >= 2 * GT * GLD, "both halves' partial tiles fit");
 
-__global__ void __cluster_dims__(GC, 1, 1) __launch_bounds__(MLP_THREADS)
+__global__ void __cluster_dims__(GC, 1, 1) __launch_bounds__(GTHREADS)
 mlpWeightGrads(const float* params, const float* X, int batch,
                const float* ws, const float* dout,
                float* grads) {
@@ -409,9 +438,9 @@ mlpWeightGrads(const float* params, const float* X, int batch,
     Dg = Ig = ws + 2 * part;  // A3
   }
   const bool vec = aligned16(ws);
-  const int tx = tid % 16, ty = tid / 16;
-  float acc[4][4] = {};
-  float accB = 0.f;  // layer 4: output column tid < H, else its bias; others: bias o0 + tid
+  const int half = tid / (GTHREADS / 2), tx = tid % 16, ty = tid / 16 % 16;
+  float acc[4][4] = {}, accD[4] = {};  // the tile; the bias
+  float accB = 0.f;                    // layer 4: output column tid < H, else its bias
   dependencyWait();
   if (layer == 3) copyRows(s.W4, H, L.W4, H, 1, H, aligned16(params));
   for (int b0 = rank * GROWS; b0 < batch; b0 += GC * GROWS) {
@@ -433,7 +462,7 @@ mlpWeightGrads(const float* params, const float* X, int batch,
     copyWait<0>();
     __syncthreads();
     if (layer == 3) {
-      for (int i = tid; i < rows * GT; i += MLP_THREADS) {
+      for (int i = tid; i < rows * GT; i += GTHREADS) {
         const int r = i / GT, c = i % GT;
         s.D[r * GLD + c] = outputGrad(s.D[r * GLD + c], s.dout[r], s.W4[o0 + c]);
       }
@@ -441,17 +470,17 @@ mlpWeightGrads(const float* params, const float* X, int batch,
     }
     if (tx * 4 < width)
 #pragma unroll 4
-      for (int r = 0; r < rows; ++r) {
+      for (int r = half; r < rows; r += 2) {
         const float4 d = *reinterpret_cast<const float4*>(s.D + r * GLD + ty * 4);
         const float4 x = *reinterpret_cast<const float4*>(s.In + r * GLD + tx * 4);
         const float dv[4] = {d.x, d.y, d.z, d.w}, xv[4] = {x.x, x.y, x.z, x.w};
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
+        for (int i = 0; i < 4; ++i) {
+          accD[i] += dv[i];
 #pragma unroll
           for (int j = 0; j < 4; ++j) acc[i][j] = __fmaf_rn(dv[i], xv[j], acc[i][j]);
+        }
       }
-    if (i0 == 0 && tid < GT)
-      for (int r = 0; r < rows; ++r) accB += s.D[r * GLD + tid];
     __syncthreads();  // the next chunk reuses the buffers
   }
   // partial sums to shared memory (layer 4: one row of H columns and the bias)
@@ -459,11 +488,23 @@ mlpWeightGrads(const float* params, const float* X, int batch,
   if (layer == 4) {
     if (tid <= H) partial[tid] = accB;
   } else {
+    if (half == 1) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
-      *reinterpret_cast<float4*>(partial + (ty * 4 + i) * GLD + tx * 4) =
-          make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
-    if (tid < GT) s.bias[tid] = accB;
+      for (int i = 0; i < 4; ++i)
+        *reinterpret_cast<float4*>(partial + (GT + ty * 4 + i) * GLD + tx * 4) =
+            make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+      if (tx == 0) *reinterpret_cast<float4*>(s.bias + ty * 4) = make_float4(accD[0], accD[1], accD[2], accD[3]);
+    }
+    __syncthreads();
+    if (half == 0) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float4 o = *reinterpret_cast<const float4*>(partial + (GT + ty * 4 + i) * GLD + tx * 4);
+        *reinterpret_cast<float4*>(partial + (ty * 4 + i) * GLD + tx * 4) =
+            make_float4(acc[i][0] + o.x, acc[i][1] + o.y, acc[i][2] + o.z, acc[i][3] + o.w);
+        if (tx == 0) s.bias[ty * 4 + i] += accD[i];
+      }
+    }
   }
   cluster.sync();
   // CTA `rank` adds the eight partial sums of its share, in rank order
@@ -475,7 +516,7 @@ mlpWeightGrads(const float* params, const float* X, int batch,
   };
   const Layout G = layout(grads);
   if (layer == 4) {
-    for (int j = rank * MLP_THREADS + tid; j <= H; j += GC * MLP_THREADS) {
+    for (int j = rank * GTHREADS + tid; j <= H; j += GC * GTHREADS) {
       const float v = total(partial + j);
       *const_cast<float*>(j < H ? G.W4 + j : G.b4) = v;
     }
@@ -484,7 +525,7 @@ mlpWeightGrads(const float* params, const float* X, int batch,
     float* gb = const_cast<float*>(layer == 3 ? G.b3 : layer == 2 ? G.b2 : G.b1);
     const int ld = layer == 1 ? NFEAT : H;
     constexpr int OUT = GT / GC;  // rows of the tile
-    for (int i = tid; i < OUT * width; i += MLP_THREADS) {
+    for (int i = tid; i < OUT * width; i += GTHREADS) {
       const int o = rank * OUT + i / width, c = i % width;
       gW[(size_t)(o0 + o) * ld + i0 + c] = total(partial + o * GLD + c);
     }
@@ -579,8 +620,10 @@ int librett_c_mlp_backward(const float* params, const float* X, int batch, float
       batch, s, sizeof(BackwardShared<8>), sizeof(BackwardShared<16>), sizeof(BackwardShared<32>),
       mlpBackwardRows<8>, mlpBackwardRows<16>, mlpBackwardRows<32>, params, batch, ws, dout);
   if (err == cudaSuccess)
-    err = launchDependent(mlpWeightGrads, GTILES * GC, MLP_THREADS, sizeof(GradShared), s, params, X,
-                          batch, (const float*)ws, dout, grads);
+    err = cachedOccupancy((const void*)mlpWeightGrads, GTHREADS, (int)sizeof(GradShared)) < 1
+              ? cudaErrorInvalidConfiguration
+              : launchDependent(mlpWeightGrads, GTILES * GC, GTHREADS, sizeof(GradShared), s, params, X,
+                                batch, (const float*)ws, dout, grads);
   return err == cudaSuccess ? LIBRETT_SUCCESS : LIBRETT_INTERNAL_ERROR;
 }
 
