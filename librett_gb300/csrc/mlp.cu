@@ -32,7 +32,7 @@
 
 #include <cmath>
 
-#include "kernels.cuh"
+#include "tile_kernel.cuh"
 #include "librett.h"
 #include "librett_c.h"
 #include "plans.h"
@@ -74,38 +74,49 @@ __device__ __forceinline__ void copyWait() {
   asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
 }
 
-// A whole H x H matrix into dst (row stride dld).  Every CTA copies the same
-// matrix at the same time: each starts at another row, so that they do not all
-// ask the same L2 slice.
-__device__ __forceinline__ void copyMatrix(float* dst, int dld, const float* src, bool vec) {
-  const int start = (int)(blockIdx.x * 8);
-  if (vec) {
-    for (int i = threadIdx.x; i < H * H / 4; i += blockDim.x) {
-      const int r = (i / (H / 4) + start) % H, c = i % (H / 4) * 4;
-      copyAsync16(dst + r * dld + c, src + r * H + c);
-    }
-  } else {
-    for (int i = threadIdx.x; i < H * H; i += blockDim.x) {
-      const int r = (i / H + start) % H, c = i % H;
-      copyAsync4(dst + r * dld + c, src + r * H + c);
-    }
-  }
+// Weights come by bulk copies that complete on an mbarrier (16 bytes per thread
+// and cp.async moved 25 bytes a cycle into an SM), where the parameters are
+// 16-byte aligned.  The waits are bounded like the transpose kernels': a copy
+// that does not arrive makes the CTA return without results, NaN as output.
+struct Arrival {
+  unsigned long long bar;
+};
+
+__device__ __forceinline__ uint32_t sharedAddr(const void* p) {
+  return (uint32_t)__cvta_generic_to_shared(p);
+}
+
+// Called by one thread: one arrival, `bytes` to come.
+__device__ __forceinline__ void expect(Arrival& a, uint32_t bytes) {
+  mbarArriveExpectTx(sharedAddr(&a.bar), bytes);
+}
+
+__device__ __forceinline__ void bulkFloats(float* dst, const float* src, int n, Arrival& a) {
+  bulkLoad(sharedAddr(dst), src, (uint32_t)(n * 4), sharedAddr(&a.bar));
+}
+
+__device__ __forceinline__ bool arrived(Arrival& a) {
+  return mbarWaitBounded(sharedAddr(&a.bar), 0, BULK_WAIT_NS);
 }
 
 // rows x cols of src (row stride sld) into dst (row stride dld) by cp.async, in
 // 16-byte units when vec (cols, sld and dld multiples of 4, src 16-byte aligned).
 __device__ __forceinline__ void copyRows(float* dst, int dld, const float* src, int sld, int rows,
                                          int cols, bool vec) {
-  if (vec) {
-    const int c4 = cols / 4;
-    for (int i = threadIdx.x; i < rows * c4; i += blockDim.x) {
-      const int r = i / c4, c = (i - r * c4) * 4;
-      copyAsync16(dst + r * dld + c, src + (size_t)r * sld + c);
-    }
-  } else {
-    for (int i = threadIdx.x; i < rows * cols; i += blockDim.x) {
-      const int r = i / cols, c = i - r * cols;
+  const int per = vec ? 4 : 1, units = cols / per;
+  // one division per thread: (r, c) then advances by blockDim.x units
+  int r = (int)threadIdx.x / units, c = (int)threadIdx.x - r * units;
+  const int dr = (int)blockDim.x / units, dc = (int)blockDim.x - dr * units;
+  while (r < rows) {
+    if (vec)
+      copyAsync16(dst + r * dld + 4 * c, src + (size_t)r * sld + 4 * c);
+    else
       copyAsync4(dst + r * dld + c, src + (size_t)r * sld + c);
+    r += dr;
+    c += dc;
+    if (c >= units) {
+      c -= units;
+      ++r;
     }
   }
 }
@@ -146,60 +157,74 @@ struct Place {
   __device__ static int row() { return threadIdx.x / COLS * TM; }
 };
 
-// acc += in[rows][0..K) * w[cols][0..K)^T, both padded rows of LD; products in
-// input order.
+// acc += sum over k of in[row][k] * w(k)[col], products in input order; w(k, j)
+// gives weights k .. k + 3 of column j.  The operands of the next four inputs
+// are read ahead of this four's products: with two warps per scheduler the
+// reads' latency otherwise bounds the loop.
+template <int R, typename W4>
+__device__ __forceinline__ void layerProducts(const float* in, W4 w4,
+                                              float (&acc)[Place<R>::TM][Place<R>::TN]) {
+  using P = Place<R>;
+  const float* a = in + P::row() * LD;
+  float4 w[P::TN], x[P::TM];
+  auto read = [&](int k) {
+#pragma unroll
+    for (int j = 0; j < P::TN; ++j) w[j] = w4(k, j);
+#pragma unroll
+    for (int i = 0; i < P::TM; ++i) x[i] = *reinterpret_cast<const float4*>(a + i * LD + k);
+  };
+  read(0);
+#pragma unroll 4
+  for (int k = 0; k < H; k += 4) {
+    float4 cw[P::TN], cx[P::TM];
+#pragma unroll
+    for (int j = 0; j < P::TN; ++j) cw[j] = w[j];
+#pragma unroll
+    for (int i = 0; i < P::TM; ++i) cx[i] = x[i];
+    if (k + 4 < H) read(k + 4);
+#pragma unroll
+    for (int i = 0; i < P::TM; ++i)
+#pragma unroll
+      for (int j = 0; j < P::TN; ++j) acc[i][j] = __fmaf_rn(cx[i].x, cw[j].x, acc[i][j]);
+#pragma unroll
+    for (int i = 0; i < P::TM; ++i)
+#pragma unroll
+      for (int j = 0; j < P::TN; ++j) acc[i][j] = __fmaf_rn(cx[i].y, cw[j].y, acc[i][j]);
+#pragma unroll
+    for (int i = 0; i < P::TM; ++i)
+#pragma unroll
+      for (int j = 0; j < P::TN; ++j) acc[i][j] = __fmaf_rn(cx[i].z, cw[j].z, acc[i][j]);
+#pragma unroll
+    for (int i = 0; i < P::TM; ++i)
+#pragma unroll
+      for (int j = 0; j < P::TN; ++j) acc[i][j] = __fmaf_rn(cx[i].w, cw[j].w, acc[i][j]);
+  }
+}
+
+// With the weights in padded rows of LD, one per output.
 template <int R>
 __device__ __forceinline__ void layerTimesRows(const float* in, const float* w,
                                                float (&acc)[Place<R>::TM][Place<R>::TN]) {
   using P = Place<R>;
-  const float* a = in + P::row() * LD;
   const float* b = w + P::col() * LD;
-#pragma unroll 4
-  for (int k = 0; k < H; k += 4) {
-    float4 wv[P::TN];
-#pragma unroll
-    for (int j = 0; j < P::TN; ++j)
-      wv[j] = *reinterpret_cast<const float4*>(b + j * P::COLS * LD + k);
-#pragma unroll
-    for (int i = 0; i < P::TM; ++i) {
-      const float4 av = *reinterpret_cast<const float4*>(a + i * LD + k);
-#pragma unroll
-      for (int j = 0; j < P::TN; ++j) {
-        acc[i][j] = __fmaf_rn(av.x, wv[j].x, acc[i][j]);
-        acc[i][j] = __fmaf_rn(av.y, wv[j].y, acc[i][j]);
-        acc[i][j] = __fmaf_rn(av.z, wv[j].z, acc[i][j]);
-        acc[i][j] = __fmaf_rn(av.w, wv[j].w, acc[i][j]);
-      }
-    }
-  }
+  layerProducts<R>(
+      in, [&](int k, int j) { return *reinterpret_cast<const float4*>(b + j * P::COLS * LD + k); },
+      acc);
 }
 
-// acc += in[rows][0..H) * w[0..H)[cols]: w in rows of H, one per input.
+// With the weights in rows of H, one per input.
 template <int R>
 __device__ __forceinline__ void layerTimesCols(const float* in, const float* w,
                                                float (&acc)[Place<R>::TM][Place<R>::TN]) {
   using P = Place<R>;
-  const float* a = in + P::row() * LD;
   const float* b = w + P::col();
-#pragma unroll 4
-  for (int k = 0; k < H; k += 4) {
-    float wv[4][P::TN];
-#pragma unroll
-    for (int q = 0; q < 4; ++q)
-#pragma unroll
-      for (int j = 0; j < P::TN; ++j) wv[q][j] = b[(k + q) * H + j * P::COLS];
-#pragma unroll
-    for (int i = 0; i < P::TM; ++i) {
-      const float4 av = *reinterpret_cast<const float4*>(a + i * LD + k);
-#pragma unroll
-      for (int j = 0; j < P::TN; ++j) {
-        acc[i][j] = __fmaf_rn(av.x, wv[0][j], acc[i][j]);
-        acc[i][j] = __fmaf_rn(av.y, wv[1][j], acc[i][j]);
-        acc[i][j] = __fmaf_rn(av.z, wv[2][j], acc[i][j]);
-        acc[i][j] = __fmaf_rn(av.w, wv[3][j], acc[i][j]);
-      }
-    }
-  }
+  layerProducts<R>(
+      in,
+      [&](int k, int j) {
+        const float* q = b + k * H + j * P::COLS;
+        return make_float4(q[0], q[H], q[2 * H], q[3 * H]);
+      },
+      acc);
 }
 
 template <int R>
@@ -209,6 +234,7 @@ struct ForwardShared {
   float A[R * LD], B[R * LD];
   float W1[H * NFEAT];
   float b1[H], b2[H], b3[H], W4[H];
+  Arrival first, second, third;  // W1 and X's CTA-wide part; W2; W3
 };
 
 // Bias, ReLU; the activation to shared memory and to global memory.
@@ -239,24 +265,45 @@ mlpForwardKernel(const float* params, const float* X, int batch,
   const int r0 = blockIdx.x * R, rows = min(R, batch - r0);
   const Layout L = layout(params);
   const bool vec = aligned16(params);
+  if (threadIdx.x == 0) {
+    mbarInit(sharedAddr(&s.first.bar), 1);
+    mbarInit(sharedAddr(&s.second.bar), 1);
+    mbarInit(sharedAddr(&s.third.bar), 1);
+    mbarInitFence();
+  }
+  __syncthreads();
   dependencyWait();
+  if (vec) {
+    if (threadIdx.x == 0) {
+      expect(s.first, H * NFEAT * 4);
+      bulkFloats(s.W1, L.W1, H * NFEAT, s.first);
+      expect(s.second, H * H * 4);
+      expect(s.third, H * H * 4);
+    }
+    __syncthreads();  // the counts are armed before a copy completes
+    if (threadIdx.x < H) {
+      bulkFloats(s.W2 + threadIdx.x * LD, L.W2 + threadIdx.x * H, H, s.second);
+      bulkFloats(s.W3 + threadIdx.x * LD, L.W3 + threadIdx.x * H, H, s.third);
+    }
+  } else {
+    copyRows(s.W1, H * NFEAT, L.W1, 0, 1, H * NFEAT, false);
+    copyRows(s.W2, LD, L.W2, H, H, H, false);
+    copyRows(s.W3, LD, L.W3, H, H, H, false);
+  }
   copyRows(s.X, XLD, X + (size_t)r0 * NFEAT, NFEAT, rows, NFEAT, false);
-  copyRows(s.W1, H * NFEAT, L.W1, H * NFEAT, 1, H * NFEAT, vec && H * NFEAT % 4 == 0);
-  copyRows(s.b1, H, L.b1, H, 1, H, vec);
-  copyRows(s.b2, H, L.b2, H, 1, H, vec);
-  copyRows(s.b3, H, L.b3, H, 1, H, vec);
-  copyRows(s.W4, H, L.W4, H, 1, H, vec);
+  copyRows(s.b1, H, L.b1, 0, 1, H, vec);
+  copyRows(s.b2, H, L.b2, 0, 1, H, vec);
+  copyRows(s.b3, H, L.b3, 0, 1, H, vec);
+  copyRows(s.W4, H, L.W4, 0, 1, H, vec);
   copyCommit();
-  copyMatrix(s.W2, LD, L.W2, vec);
-  copyCommit();
-  copyMatrix(s.W3, LD, L.W3, vec);
-  copyCommit();
+  bool ok = true;  // every copy arrived
   float* A1 = ws + (size_t)r0 * H;
   float* A2 = A1 + (size_t)batch * H;
   float* A3 = A2 + (size_t)batch * H;
   // rows past the batch: any finite input
   for (int i = rows * XLD + threadIdx.x; i < R * XLD; i += MLP_THREADS) s.X[i] = 0.f;
-  copyWait<2>();
+  copyWait<0>();
+  if (vec) ok = arrived(s.first);
   __syncthreads();
   {
     float acc[P::TM][P::TN] = {};
@@ -274,14 +321,14 @@ mlpForwardKernel(const float* params, const float* X, int batch,
     }
     activate<R>(acc, s.b1, s.A, A1, rows);
   }
-  copyWait<1>();
+  if (vec) ok = arrived(s.second) && ok;
   __syncthreads();
   {
     float acc[P::TM][P::TN] = {};
     layerTimesRows<R>(s.A, s.W2, acc);
     activate<R>(acc, s.b2, s.B, A2, rows);
   }
-  copyWait<0>();
+  if (vec) ok = arrived(s.third) && ok;
   __syncthreads();
   {
     float acc[P::TM][P::TN] = {};
@@ -301,7 +348,7 @@ mlpForwardKernel(const float* params, const float* X, int batch,
       v = __fmaf_rn(av.z, wv.z, v);
       v = __fmaf_rn(av.w, wv.w, v);
     }
-    out[r0 + threadIdx.x] = v + *L.b4;
+    out[r0 + threadIdx.x] = ok ? v + *L.b4 : nanf("");
   }
 }
 
@@ -315,6 +362,7 @@ template <int R>
 struct BackwardShared {
   float W3[H * H], W2[H * H];
   float D[R * LD], E[R * LD];
+  Arrival first, second;  // W3, W2
 };
 
 // A thread's outputs' places in an activation or gradient of H columns.
@@ -340,11 +388,27 @@ mlpBackwardRows(const float* params, int batch, float* ws,
   const int r0 = blockIdx.x * R, rows = min(R, batch - r0);
   const Layout L = layout(params);
   const bool vec = aligned16(params);
+  if (threadIdx.x == 0) {
+    mbarInit(sharedAddr(&s.first.bar), 1);
+    mbarInit(sharedAddr(&s.second.bar), 1);
+    mbarInitFence();
+  }
+  __syncthreads();
   dependencyWait();
-  copyMatrix(s.W3, H, L.W3, vec);
-  copyCommit();
-  copyMatrix(s.W2, H, L.W2, vec);
-  copyCommit();
+  if (vec) {
+    if (threadIdx.x == 0) {
+      constexpr int PIECE = H * H / 4;
+      expect(s.first, H * H * 4);
+      for (int i = 0; i < H * H; i += PIECE) bulkFloats(s.W3 + i, L.W3 + i, PIECE, s.first);
+      expect(s.second, H * H * 4);
+      for (int i = 0; i < H * H; i += PIECE) bulkFloats(s.W2 + i, L.W2 + i, PIECE, s.second);
+    }
+  } else {
+    copyRows(s.W3, H * H, L.W3, 0, 1, H * H, false);
+    copyRows(s.W2, H * H, L.W2, 0, 1, H * H, false);
+    copyCommit();
+  }
+  bool ok = true;  // every copy arrived
   const size_t part = (size_t)batch * H;
   const float* A1 = ws + (size_t)r0 * H;
   const float* A2 = A1 + part;
@@ -361,24 +425,27 @@ mlpBackwardRows(const float* params, int batch, float* ws,
     on2[i][j] = r < rows && A2[(size_t)r * H + c] > 0.f;
     on1[i][j] = r < rows && A1[(size_t)r * H + c] > 0.f;
   });
-  copyWait<1>();
+  if (vec)
+    ok = arrived(s.first);
+  else
+    copyWait<0>();
   __syncthreads();
   {
     float acc[P::TM][P::TN] = {};
     layerTimesCols<R>(s.D, s.W3, acc);
     forOutputs<R>([&](int i, int j, int r, int c) {
-      const float v = on2[i][j] ? acc[i][j] : 0.f;
+      const float v = !ok ? nanf("") : on2[i][j] ? acc[i][j] : 0.f;
       s.E[r * LD + c] = v;
       if (r < rows) D2[(size_t)r * H + c] = v;
     });
   }
-  copyWait<0>();
+  if (vec) ok = arrived(s.second) && ok;
   __syncthreads();
   {
     float acc[P::TM][P::TN] = {};
     layerTimesCols<R>(s.E, s.W2, acc);
     forOutputs<R>([&](int i, int j, int r, int c) {
-      if (r < rows) D1[(size_t)r * H + c] = on1[i][j] ? acc[i][j] : 0.f;
+      if (r < rows) D1[(size_t)r * H + c] = !ok ? nanf("") : on1[i][j] ? acc[i][j] : 0.f;
     });
   }
 }
@@ -391,6 +458,7 @@ constexpr int GT = 64, GC = 8, GROWS = 128, GTHREADS = 512;
 constexpr int GLD = GT + 4;
 // tiles: W3 and W2 four each, W1 two (NFEAT <= GT), the output layer one
 constexpr int GTILES = 2 * (H / GT) * (H / GT) + H / GT + 1;
+static_assert(H == 2 * GT, "layer 4 reads its activation as two halves");
 static_assert(NFEAT <= GT, "one tile covers the features");
 
 struct GradShared {
@@ -435,32 +503,35 @@ mlpWeightGrads(const float* params, const float* X, int batch,
   } else {
     layer = 4;
     o0 = 0;
-    Dg = Ig = ws + 2 * part;  // A3
+    Dg = ws + 2 * part;  // A3
+    Ig = Dg + GT;
   }
   const bool vec = aligned16(ws);
   const int half = tid / (GTHREADS / 2), tx = tid % 16, ty = tid / 16 % 16;
   float acc[4][4] = {}, accD[4] = {};  // the tile; the bias
-  float accB = 0.f;                    // layer 4: output column tid < H, else its bias
+  float acc4 = 0.f;  // layer 4: column tid % H over every fourth row; its bias in accD[0]
   dependencyWait();
   if (layer == 3) copyRows(s.W4, H, L.W4, H, 1, H, aligned16(params));
   for (int b0 = rank * GROWS; b0 < batch; b0 += GC * GROWS) {
     const int rows = min(GROWS, batch - b0);
-    if (layer == 4) {
-      // one row of gradients: thread j sums column j, thread H the bias
-      if (tid <= H)
-#pragma unroll 8
-        for (int r = 0; r < rows; ++r) {
-          const float d = dout[b0 + r];
-          accB = tid < H ? __fmaf_rn(d, Dg[(size_t)(b0 + r) * H + tid], accB) : accB + d;
-        }
-      continue;
-    }
     copyRows(s.D, GLD, Dg + (size_t)b0 * H + o0, H, rows, GT, vec);
     copyRows(s.In, GLD, Ig + (size_t)b0 * ild + i0, ild, rows, width, vec && layer != 1);
-    if (layer == 3) copyRows(s.dout, GROWS, dout + b0, GROWS, 1, rows, false);
+    if (layer >= 3) copyRows(s.dout, GROWS, dout + b0, GROWS, 1, rows, false);
     copyCommit();
     copyWait<0>();
     __syncthreads();
+    if (layer == 4) {
+      // one row of gradients: D holds activation columns 0 .. GT - 1, In the rest
+      const int j = tid % H;
+      const float* a = j < GT ? s.D + j : s.In + j - GT;
+#pragma unroll 8
+      for (int r = tid / H; r < rows; r += GTHREADS / H) {
+        acc4 = __fmaf_rn(s.dout[r], a[r * GLD], acc4);
+        accD[0] += s.dout[r];
+      }
+      __syncthreads();
+      continue;
+    }
     if (layer == 3) {
       for (int i = tid; i < rows * GT; i += GTHREADS) {
         const int r = i / GT, c = i % GT;
@@ -486,7 +557,15 @@ mlpWeightGrads(const float* params, const float* X, int batch,
   // partial sums to shared memory (layer 4: one row of H columns and the bias)
   float* partial = s.D;
   if (layer == 4) {
-    if (tid <= H) partial[tid] = accB;
+    partial[tid] = acc4;
+    if (tid % H == 0) s.bias[tid / H] = accD[0];
+    __syncthreads();
+    float v = 0.f;
+    if (tid <= H)
+#pragma unroll
+      for (int k = 0; k < GTHREADS / H; ++k) v += tid < H ? partial[k * H + tid] : s.bias[k];
+    __syncthreads();
+    if (tid <= H) partial[tid] = v;
   } else {
     if (half == 1) {
 #pragma unroll
