@@ -12,7 +12,7 @@
 //                      layer waits for its own;
 //   mlpBackwardRows    a CTA takes R rows back through layers 3 and 2 (the
 //                      gradients of their inputs, D2 and D1);
-//   mlpWeightGrads     a cluster of 8 CTAs per 64 x 64 tile of a weight
+//   mlpWeightGrads     a cluster of 8 CTAs per 32 x 64 tile of a weight
 //                      gradient, each summing an eighth of the rows, combined
 //                      through distributed shared memory in a fixed order.
 // A layer-by-layer version (a 64 x 64-tiled SGEMM, bias, mask and column-sum
@@ -31,6 +31,7 @@
 #include <cuda_runtime.h>
 
 #include <cmath>
+#include <type_traits>
 
 #include "tile_kernel.cuh"
 #include "librett.h"
@@ -415,9 +416,17 @@ mlpBackwardRows(const float* params, int batch, float* ws,
   const float* A3 = A2 + part;
   float* D1 = ws + 3 * part + (size_t)r0 * H;
   float* D2 = D1 + part;
-  for (int i = threadIdx.x; i < R * H; i += MLP_THREADS) {
-    const int r = i / H, c = i % H;
-    s.D[r * LD + c] = r < rows ? outputGrad(A3[i], dout[r0 + r], L.W4[c]) : 0.f;
+  constexpr int PER = R * H / MLP_THREADS;  // elements of D3 a thread makes
+  float a3[PER];
+#pragma unroll
+  for (int q = 0; q < PER; ++q) {
+    const int i = threadIdx.x + q * MLP_THREADS;
+    a3[q] = i / H < rows ? A3[i] : 0.f;
+  }
+#pragma unroll
+  for (int q = 0; q < PER; ++q) {
+    const int i = threadIdx.x + q * MLP_THREADS, r = i / H, c = i % H;
+    s.D[r * LD + c] = r < rows ? outputGrad(a3[q], dout[r0 + r], L.W4[c]) : 0.f;
   }
   // the masks of both products, read while the weights are on their way
   bool on2[P::TM][P::TN], on1[P::TM][P::TN];
@@ -451,142 +460,155 @@ mlpBackwardRows(const float* params, int batch, float* ws,
 }
 
 // Weight gradients: gW[o][i] = sum over rows of D[row][o] * In[row][i] and gb[o]
-// = sum of D[row][o], in tiles of GT x GT.  A cluster of GC CTAs shares a tile;
-// CTA c takes GROWS-row chunks c, c + GC, ... of the batch, each half of its
-// threads every other row.
-constexpr int GT = 64, GC = 8, GROWS = 128, GTHREADS = 512;
-constexpr int GLD = GT + 4;
-// tiles: W3 and W2 four each, W1 two (NFEAT <= GT), the output layer one
-constexpr int GTILES = 2 * (H / GT) * (H / GT) + H / GT + 1;
-static_assert(H == 2 * GT, "layer 4 reads its activation as two halves");
-static_assert(NFEAT <= GT, "one tile covers the features");
+// = sum of D[row][o], in tiles of GO x GI.  A cluster of GC CTAs shares a tile;
+// CTA c takes GROWS-row chunks c, c + GC, ... of the batch (the next chunk on its
+// way while one is summed), each GPARTS-th of its threads every GPARTS-th row.
+// A thread sums 4 x 8 products per row for three 16-byte reads, so the kernel is
+// bound by the FMA pipe; 22 tiles x 8 CTAs cover the device.
+constexpr int GO = 32, GI = 64, GC = 8, GROWS = 128, GTHREADS = 256;
+constexpr int GPART = (GO / 4) * (GI / 8), GPARTS = GTHREADS / GPART;
+constexpr int DLD = GO + 4, ILD = GI + 4;
+constexpr int GW_TILES = (H / GO) * (H / GI);  // of W3 and of W2
+constexpr int GTILES = 2 * GW_TILES + H / GO + H / GI;
+static_assert(NFEAT <= GI, "one tile width covers the features");
 
 struct GradShared {
-  float D[GROWS * GLD], In[GROWS * GLD];  // a chunk; then the CTA's partial tile in D
-  float dout[GROWS], W4[H];
-  float bias[GT];
+  struct Chunk {
+    float D[GROWS * DLD], In[GROWS * ILD], dout[GROWS];
+  } chunk[2];
+  float W4[H];
+  float bias[GPARTS][GO];
 };
-static_assert(GROWS * GLD >= 2 * GT * GLD, "both halves' partial tiles fit");
+constexpr int GPARTIAL = GO * ILD;  // floats of a part's tile, in the chunks' place
+static_assert(GPARTS * GPARTIAL * sizeof(float) <= sizeof(GradShared::chunk), "parts' tiles fit");
 
 __global__ void __cluster_dims__(GC, 1, 1) __launch_bounds__(GTHREADS)
-mlpWeightGrads(const float* params, const float* X, int batch,
-               const float* ws, const float* dout,
+mlpWeightGrads(const float* params, const float* X, int batch, const float* ws, const float* dout,
                float* grads) {
   extern __shared__ __align__(16) unsigned char smraw[];
   GradShared& s = *reinterpret_cast<GradShared*>(smraw);
   cg::cluster_group cluster = cg::this_cluster();
   dependencyRelease();
-  const int tile = blockIdx.x / GC, rank = (int)cluster.block_rank();
-  const int tid = threadIdx.x;
+  const int tile = blockIdx.x / GC, rank = (int)cluster.block_rank(), tid = threadIdx.x;
   const Layout L = layout(params);
   const size_t part = (size_t)batch * H;
   // which gradient: its D and In with their first column and width, and where
   // the tile goes
-  constexpr int PER = (H / GT) * (H / GT);
-  int layer, o0, i0 = 0, width = GT;
-  const float *Dg, *Ig;
-  int ild = H;
-  if (tile < 2 * PER) {
-    layer = tile < PER ? 3 : 2;
-    const int t = tile % PER;
-    o0 = t / (H / GT) * GT;
-    i0 = t % (H / GT) * GT;
+  int layer, o0 = 0, i0 = 0, width = GI, ild = H;
+  const float *Dg = ws, *Ig;
+  if (tile < 2 * GW_TILES) {
+    layer = tile < GW_TILES ? 3 : 2;
+    const int t = tile % GW_TILES;
+    o0 = t / (H / GI) * GO;
+    i0 = t % (H / GI) * GI;
     Dg = layer == 3 ? ws + 2 * part : ws + 4 * part;  // layer 3: A3, made D3 below
     Ig = layer == 3 ? ws + part : ws;
-  } else if (tile < 2 * PER + H / GT) {
+  } else if (tile < 2 * GW_TILES + H / GO) {
     layer = 1;
-    o0 = (tile - 2 * PER) * GT;
+    o0 = (tile - 2 * GW_TILES) * GO;
     Dg = ws + 3 * part;
     Ig = X;
-    ild = NFEAT;
-    width = NFEAT;
+    ild = width = NFEAT;
   } else {
-    layer = 4;
-    o0 = 0;
-    Dg = ws + 2 * part;  // A3
-    Ig = Dg + GT;
+    layer = 4;  // one row of gradients: D is dout
+    i0 = (tile - 2 * GW_TILES - H / GO) * GI;
+    Ig = ws + 2 * part;
   }
-  const bool vec = aligned16(ws);
-  const int half = tid / (GTHREADS / 2), tx = tid % 16, ty = tid / 16 % 16;
-  float acc[4][4] = {}, accD[4] = {};  // the tile; the bias
-  float acc4 = 0.f;  // layer 4: column tid % H over every fourth row; its bias in accD[0]
+  const bool vec = aligned16(ws), bias = i0 == 0;
+  const int sub = tid / GPART, tx = tid % 8, ty = tid / 8 % (GO / 4);
+  float acc[4][8] = {}, accD[4] = {};  // the tile: columns 4 tx + j, then 32 + 4 tx + j; the bias
   dependencyWait();
-  if (layer == 3) copyRows(s.W4, H, L.W4, H, 1, H, aligned16(params));
-  for (int b0 = rank * GROWS; b0 < batch; b0 += GC * GROWS) {
+  if (layer == 3) copyRows(s.W4, H, L.W4, 0, 1, H, aligned16(params));
+  auto fetch = [&](int b0, GradShared::Chunk& c) {
     const int rows = min(GROWS, batch - b0);
-    copyRows(s.D, GLD, Dg + (size_t)b0 * H + o0, H, rows, GT, vec);
-    copyRows(s.In, GLD, Ig + (size_t)b0 * ild + i0, ild, rows, width, vec && layer != 1);
-    if (layer >= 3) copyRows(s.dout, GROWS, dout + b0, GROWS, 1, rows, false);
+    if (layer != 4) copyRows(c.D, DLD, Dg + (size_t)b0 * H + o0, H, rows, GO, vec);
+    copyRows(c.In, ILD, Ig + (size_t)b0 * ild + i0, ild, rows, width, vec && layer != 1);
+    if (layer >= 3) copyRows(c.dout, GROWS, dout + b0, 0, 1, rows, false);
     copyCommit();
-    copyWait<0>();
-    __syncthreads();
-    if (layer == 4) {
-      // one row of gradients: D holds activation columns 0 .. GT - 1, In the rest
-      const int j = tid % H;
-      const float* a = j < GT ? s.D + j : s.In + j - GT;
-#pragma unroll 8
-      for (int r = tid / H; r < rows; r += GTHREADS / H) {
-        acc4 = __fmaf_rn(s.dout[r], a[r * GLD], acc4);
-        accD[0] += s.dout[r];
-      }
-      __syncthreads();
-      continue;
+  };
+  const int first = rank * GROWS, stride = GC * GROWS;
+  if (first < batch) fetch(first, s.chunk[0]);
+  int buf = 0;
+  for (int b0 = first; b0 < batch; b0 += stride, buf ^= 1) {
+    const int rows = min(GROWS, batch - b0);
+    GradShared::Chunk& c = s.chunk[buf];
+    if (b0 + stride < batch) {
+      fetch(b0 + stride, s.chunk[buf ^ 1]);
+      copyWait<1>();
+    } else {
+      copyWait<0>();
     }
+    __syncthreads();
     if (layer == 3) {
-      for (int i = tid; i < rows * GT; i += GTHREADS) {
-        const int r = i / GT, c = i % GT;
-        s.D[r * GLD + c] = outputGrad(s.D[r * GLD + c], s.dout[r], s.W4[o0 + c]);
+#pragma unroll 4
+      for (int i = tid; i < rows * GO; i += GTHREADS) {
+        float& d = c.D[i / GO * DLD + i % GO];
+        d = outputGrad(d, c.dout[i / GO], s.W4[o0 + i % GO]);
       }
       __syncthreads();
     }
-    if (tx * 4 < width)
+    if (layer == 4) {
+      const float* x = c.In + tid % GI;
+#pragma unroll 8
+      for (int r = tid / GI; r < rows; r += GTHREADS / GI) {
+        acc[0][0] = __fmaf_rn(c.dout[r], x[r * ILD], acc[0][0]);
+        accD[0] += c.dout[r];
+      }
+    } else if (tx * 4 < width) {
+      auto sum = [&](auto withBias) {
 #pragma unroll 4
-      for (int r = half; r < rows; r += 2) {
-        const float4 d = *reinterpret_cast<const float4*>(s.D + r * GLD + ty * 4);
-        const float4 x = *reinterpret_cast<const float4*>(s.In + r * GLD + tx * 4);
-        const float dv[4] = {d.x, d.y, d.z, d.w}, xv[4] = {x.x, x.y, x.z, x.w};
+        for (int r = sub; r < rows; r += GPARTS) {
+          const float4 d = *reinterpret_cast<const float4*>(c.D + r * DLD + ty * 4);
+          const float4 x = *reinterpret_cast<const float4*>(c.In + r * ILD + tx * 4);
+          const float4 y = *reinterpret_cast<const float4*>(c.In + r * ILD + GI / 2 + tx * 4);
+          const float dv[4] = {d.x, d.y, d.z, d.w};
+          const float xv[8] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          accD[i] += dv[i];
+          for (int i = 0; i < 4; ++i) {
+            if (decltype(withBias)::value) accD[i] += dv[i];
 #pragma unroll
-          for (int j = 0; j < 4; ++j) acc[i][j] = __fmaf_rn(dv[i], xv[j], acc[i][j]);
+            for (int j = 0; j < 8; ++j) acc[i][j] = __fmaf_rn(dv[i], xv[j], acc[i][j]);
+          }
         }
-      }
-    __syncthreads();  // the next chunk reuses the buffers
+      };
+      if (bias && tx == 0)
+        sum(std::true_type{});
+      else
+        sum(std::false_type{});
+    }
+    __syncthreads();  // the chunk after the next reuses this buffer
   }
-  // partial sums to shared memory (layer 4: one row of H columns and the bias)
-  float* partial = s.D;
+  // the parts' sums to shared memory, added in part order
+  float* partial = s.chunk[0].D;  // the chunks' place, from its start
   if (layer == 4) {
-    partial[tid] = acc4;
-    if (tid % H == 0) s.bias[tid / H] = accD[0];
-    __syncthreads();
-    float v = 0.f;
-    if (tid <= H)
-#pragma unroll
-      for (int k = 0; k < GTHREADS / H; ++k) v += tid < H ? partial[k * H + tid] : s.bias[k];
-    __syncthreads();
-    if (tid <= H) partial[tid] = v;
+    partial[tid] = acc[0][0];
+    if (tid % GI == 0) s.bias[tid / GI][0] = accD[0];
   } else {
-    if (half == 1) {
+    float* at = partial + sub * GPARTIAL + ty * 4 * ILD + tx * 4;
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
-        *reinterpret_cast<float4*>(partial + (GT + ty * 4 + i) * GLD + tx * 4) =
-            make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
-      if (tx == 0) *reinterpret_cast<float4*>(s.bias + ty * 4) = make_float4(accD[0], accD[1], accD[2], accD[3]);
+    for (int i = 0; i < 4; ++i) {
+      *reinterpret_cast<float4*>(at + i * ILD) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+      *reinterpret_cast<float4*>(at + i * ILD + GI / 2) =
+          make_float4(acc[i][4], acc[i][5], acc[i][6], acc[i][7]);
+      if (tx == 0) s.bias[sub][ty * 4 + i] = accD[i];
     }
-    __syncthreads();
-    if (half == 0) {
+  }
+  __syncthreads();
+  const int outs = layer == 4 ? GI : GO * ILD, apart = layer == 4 ? GI : GPARTIAL;
+  for (int i = tid; i < outs; i += GTHREADS) {
+    float v = partial[i];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const float4 o = *reinterpret_cast<const float4*>(partial + (GT + ty * 4 + i) * GLD + tx * 4);
-        *reinterpret_cast<float4*>(partial + (ty * 4 + i) * GLD + tx * 4) =
-            make_float4(acc[i][0] + o.x, acc[i][1] + o.y, acc[i][2] + o.z, acc[i][3] + o.w);
-        if (tx == 0) s.bias[ty * 4 + i] += accD[i];
-      }
-    }
+    for (int k = 1; k < GPARTS; ++k) v += partial[k * apart + i];
+    partial[i] = v;
+  }
+  if (tid < GO) {
+    float v = s.bias[0][tid];
+#pragma unroll
+    for (int k = 1; k < GPARTS; ++k) v += s.bias[k][tid];
+    s.bias[0][tid] = v;
   }
   cluster.sync();
-  // CTA `rank` adds the eight partial sums of its share, in rank order
+  // CTA `rank` adds the eight CTAs' sums of its share, in rank order
   auto total = [&](float* at) {
     float v = 0.f;
 #pragma unroll
@@ -595,20 +617,17 @@ mlpWeightGrads(const float* params, const float* X, int batch,
   };
   const Layout G = layout(grads);
   if (layer == 4) {
-    for (int j = rank * GTHREADS + tid; j <= H; j += GC * GTHREADS) {
-      const float v = total(partial + j);
-      *const_cast<float*>(j < H ? G.W4 + j : G.b4) = v;
-    }
+    constexpr int OUT = GI / GC;
+    if (tid < OUT) const_cast<float*>(G.W4)[i0 + rank * OUT + tid] = total(partial + rank * OUT + tid);
+    if (bias && rank == 0 && tid == OUT) *const_cast<float*>(G.b4) = total(&s.bias[0][0]);
   } else {
     float* gW = const_cast<float*>(layer == 3 ? G.W3 : layer == 2 ? G.W2 : G.W1);
     float* gb = const_cast<float*>(layer == 3 ? G.b3 : layer == 2 ? G.b2 : G.b1);
-    const int ld = layer == 1 ? NFEAT : H;
-    constexpr int OUT = GT / GC;  // rows of the tile
-    for (int i = tid; i < OUT * width; i += GTHREADS) {
-      const int o = rank * OUT + i / width, c = i % width;
-      gW[(size_t)(o0 + o) * ld + i0 + c] = total(partial + o * GLD + c);
-    }
-    if (i0 == 0 && tid < OUT) gb[o0 + rank * OUT + tid] = total(s.bias + rank * OUT + tid);
+    constexpr int OUT = GO / GC;  // rows of the tile
+    const int o = rank * OUT + tid / GI, c = tid % GI;
+    static_assert(OUT * GI == GTHREADS, "one output a thread");
+    if (c < width) gW[(size_t)(o0 + o) * ild + i0 + c] = total(partial + o * ILD + c);
+    if (bias && tid < OUT) gb[o0 + rank * OUT + tid] = total(&s.bias[0][rank * OUT + tid]);
   }
   cluster.sync();  // no CTA leaves while another reads its shared memory
 }
