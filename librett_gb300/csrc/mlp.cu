@@ -571,7 +571,7 @@ mlpWeightGrads(const float* params, const float* X, int batch, const float* ws, 
           }
         }
       };
-      if (bias && tx == 0)
+      if (bias)
         sum(std::true_type{});
       else
         sum(std::false_type{});
