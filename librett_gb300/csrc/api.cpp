@@ -614,7 +614,7 @@ int librett_c_slot_check(int rank, const int* dim, const int* permutation, size_
   int ext[lt::MAXR], step[lt::MAXR];
   const bool few = lt::loadRanks(tp, ext, step) <= 2;
   bool ok = false;
-  switch (lt::storeRankClass(tp.nTR)) {
+  switch (lt::storeRankClass(tp)) {
     case 2: ok = go(slotsMatch<2, 2>); break;
     case 3: ok = few ? go(slotsMatch<2, 3>) : go(slotsMatch<3, 3>); break;
     case 4: ok = few ? go(slotsMatch<2, 4>) : go(slotsMatch<4, 4>); break;

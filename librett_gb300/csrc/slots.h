@@ -16,7 +16,7 @@
 // Narrow units are bound by instruction issue: float32 (127, 63, 65, 33) perm
 // (3, 1, 2, 0), which moves in 4-byte units on both sides, issued 74 warp
 // instructions per 32 elements with every element decoded on its own and 45
-// with slot sums (39.9 -> 30.9 us).
+// with slot sums (39.9 -> 30.9 us; 28.7 us with dependent launches as well).
 //
 // Unused high ranks have ext 2^16 (in-tile indices are smaller, so their
 // lower neighbour never carries into them) and step 0.  Sums are unsigned: a
@@ -203,8 +203,21 @@ void makeStoreSlots(const TileParams& tp, int esize, StoreSlots<NS, NR>& s) {
                             s.corrJ, s.lim, s.offJ);
 }
 
+// Grid ranks whose chunks fit the parameter block of rank class c.  The block
+// is copied into every launch, so the classes of few tile ranks carry only as
+// many grid ranks as a problem of rank 7 can have (96 KiB of float32 in a loop
+// of executes: @@ us a call with room for 16 in every class, @@ us here).
+constexpr int GRID_FEW = 7;
+constexpr int gridCapacity(int rankClass) { return rankClass < ARITH_MAX_NTR ? GRID_FEW : MAXR; }
+
 // Rank counts the kernels are instantiated for: tiles of 1..6 ranks run as
-// 2, 3, 4 or 6 (high ranks unused).
-inline int storeRankClass(int nTR) { return nTR <= 2 ? 2 : nTR <= 4 ? nTR : 6; }
+// 2, 3, 4 or 6 (high ranks unused), and as 6 with more than GRID_FEW grid
+// ranks (a tensor of eight ranks or more); 0 for tiles with offset tables.
+inline int storeRankClass(const TileParams& tp) {
+  const int r = arithRanks(tp);
+  if (r == 0) return 0;
+  if (tp.nGR > GRID_FEW) return ARITH_MAX_NTR;
+  return r <= 2 ? 2 : r <= 4 ? r : ARITH_MAX_NTR;
+}
 
 }  // namespace lt

@@ -451,10 +451,12 @@ struct FlatParams {
   LoadSlots<NL, NI> ld;
   StoreSlots<NS, NTR> st;
   int nGR;           // grid ranks, as in TileParams
-  FastDiv grDiv[MAXR];
-  long long grSin[MAXR], grSout[MAXR], grLastIn[MAXR], grLastOut[MAXR];
+  static constexpr int NG = gridCapacity(NTR);
+  FastDiv grDiv[NG];
+  long long grSin[NG], grSout[NG], grLastIn[NG], grLastOut[NG];
 };
 
+// tp.nGR <= gridCapacity(NTR), as storeRankClass gives.
 template <int ES, int LV, int SV, int NL, int NI, int NTR>
 FlatParams<ES, LV, SV, NL, NI, NTR> makeFlatParams(const TileParams& tp) {
   FlatParams<ES, LV, SV, NL, NI, NTR> p;
