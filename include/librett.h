@@ -93,8 +93,8 @@ librettResult librettExecute(librettHandle handle, void* idata, void* odata);
 
 /* ---- Grouped execution (no LibreTT counterpart) ----
  * Many plans, each with its own input and output, executed as one CUDA
- * graph: members are bucketed by kernel shape, each bucket is one launch over
- * a device-resident descriptor table.  Creation plans, allocates (stream-
+ * graph: members are bucketed by kernel shape, most buckets share one launch
+ * (or two) over a device-resident descriptor table.  Creation plans, allocates (stream-
  * ordered on `stream`), writes the tables and instantiates the graph
  * (synchronising `stream` once); execution is one graph launch on `stream`;
  * destruction frees in stream order.  The member plans may be destroyed once

@@ -222,8 +222,8 @@ int librett_c_group_create_policy(librettGroupHandle* group, int count,
                                   const librettHandle* plans, void* const* idata,
                                   void* const* odata, void* stream, const int* policy);
 int librett_c_group_tune(librettGroupHandle group);
-/* Bucket `index` of the group's graph, in launch order (the small ones that
- * share the mixed launch last): shape[6] = element
+/* Bucket `index` of the group's graph (those that share a mixed launch keep
+ * their own entry; a group may have more buckets than launches): shape[6] = element
  * bytes, load unit, store unit (elements), load units per thread, dynamic
  * shared memory bytes, loads (0/1/2 as in the policy); its members, tiles
  * and algorithmic bytes. */

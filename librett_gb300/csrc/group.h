@@ -3,18 +3,19 @@
 // kernel per librettExecute call, src/librett.cpp:372-385).
 //
 // Every member runs as a flat tile plan.  Members are bucketed by kernel
-// shape (element size, load unit, store unit, load units per thread); each
-// bucket is one launch over a device-resident descriptor table in which CTA
-// b reads its tile (tensor index and corner offsets) and that tensor's
-// descriptor (pointers, run tables).
+// shape (element size, load unit, store unit, load units per thread).  The
+// members of the cp.async buckets whose tiles have a box (box.h) then move into
+// at most two mixed launches, one tile per CTA in any unit (k_groupmix.cu); the
+// other buckets keep a launch each over a device-resident descriptor table in
+// which CTA b reads its tile (tensor index and corner offsets) and that
+// tensor's descriptor (pointers, run tables).
 //
 // Which flat tile a member gets, and whether its bucket loads through
 // registers or cp.async, is a policy per member class (size and element
-// size); an autotuner
-// (librettGroupTune) times the policies on the group's own buffers and keeps
-// the fastest combination, cached by the batch's signature.  Buckets are
-// also split by shared-memory size (4 KiB classes), so that a CTA reserves
-// little more than its own tile needs.
+// size); an autotuner (librettGroupTune) times the policies on the group's own
+// buffers and keeps the fastest combination, cached by the batch's signature.
+// Launches are also split by the CTAs per SM that their members' shared memory
+// allows, so that a large tile costs the others no occupancy.
 #pragma once
 
 #include <cuda_runtime.h>
