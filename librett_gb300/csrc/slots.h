@@ -205,8 +205,8 @@ void makeStoreSlots(const TileParams& tp, int esize, StoreSlots<NS, NR>& s) {
 
 // Grid ranks whose chunks fit the parameter block of rank class c.  The block
 // is copied into every launch, so the classes of few tile ranks carry only as
-// many grid ranks as a problem of rank 7 can have (96 KiB of float32 in a loop
-// of executes: @@ us a call with room for 16 in every class, @@ us here).
+// many grid ranks as a problem of rank 7 can have (float32 (64, 48, 32) in
+// a loop of executes: 2.90 us a call with room for 16 in every class, 2.72 here).
 constexpr int GRID_FEW = 7;
 constexpr int gridCapacity(int rankClass) { return rankClass < ARITH_MAX_NTR ? GRID_FEW : MAXR; }
 
