@@ -380,6 +380,7 @@ class ResultSlot {
   ~ResultSlot() {
     if (p_ == nullptr) return;
     if (own_) {
+      const Uncaptured relaxed;
       cudaFreeHost(p_);
       return;
     }
@@ -398,7 +399,15 @@ class ResultSlot {
 
  private:
   static constexpr size_t PAGE = 4096, SLOT = 64;  // bytes
+  // Allocating is no error, and ends no capture, while another thread captures
+  // a stream.
+  struct Uncaptured {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    Uncaptured() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~Uncaptured() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  };
   static void* allocate(size_t bytes) {
+    const Uncaptured relaxed;
     void* p = nullptr;
     const unsigned flags = cudaHostAllocMapped | cudaHostAllocPortable;
     return cudaHostAlloc(&p, bytes, flags) == cudaSuccess ? p : nullptr;
