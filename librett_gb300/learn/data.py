@@ -7,8 +7,11 @@ uniformly random permutation.
 
 Timing of one candidate: plan it (librett_c_plan_candidate), one untimed
 launch, then three batches of R back-to-back launches between CUDA events on
-the plan's stream (R chosen so a batch lasts about 100 us, 1 <= R <= 64); the
-time is the median batch time / R.
+the plan's stream (R chosen so a batch lasts about 200 us, 1 <= R <= 64); the
+time is the median batch time / R.  A batch is one librett_c_execute_batch call:
+from a Python loop the launches of small problems come too slowly to tell their
+candidates apart.  Its launches go round up to 8 places of 1 GiB buffers, so that
+tensors of 10 MB or more come from memory, not from the L2 cache.
 
 Usage (on a GPU):
     python -m librett_gb300.learn.data --problems 6000 --seed 7 --out data.npz
@@ -75,20 +78,25 @@ def features(dims, perm, es, candidate, num_sms=152):
     return np.frombuffer(buf, dtype=np.float32).copy()
 
 
-def time_candidate(dims, perm, es, candidate, stream, din, dout, ev):
+def time_candidate(dims, perm, es, candidate, stream, din, dout, ev, room=0):
+    """room: bytes of the buffers at din and dout (0: one problem's)"""
     import torch
 
     plan = L.Plan(dims, perm, es, stream, candidate=candidate)
     try:
         nbytes = int(np.prod(dims)) * es
         est = 2.0 * nbytes / 5e12 + 4e-6
-        reps = int(min(64, max(1, np.ceil(100e-6 / est))))
+        reps = int(min(64, max(1, np.ceil(200e-6 / est))))
         plan.execute(din, dout)
+        step = -(-nbytes // 256) * 256
+        at = [k % max(1, min(8, room // step)) * step for k in range(reps)]
+        batch = L._handle_arrays([plan] * reps, [din + o for o in at], [dout + o for o in at])
         ts = []
         for _ in range(3):
             ev[0].record(stream)
-            for _ in range(reps):
-                plan.execute(din, dout)
+            rc = _lib.load().librett_c_execute_batch(*batch)
+            if rc != L.LIBRETT_SUCCESS:
+                raise L.LibrettError(rc, "librett_c_execute_batch")
             ev[1].record(stream)
             ev[1].synchronize()
             ts.append(ev[0].elapsed_time(ev[1]) / reps / 1e3)
@@ -102,7 +110,7 @@ def collect(probs, num_sms, log_every=200):
     import torch
 
     stream = torch.cuda.current_stream()
-    maxb = max(int(np.prod(d)) * es for d, _, es in probs)
+    maxb = max(1 << 30, max(int(np.prod(d)) * es for d, _, es in probs))
     a = torch.empty(maxb, dtype=torch.uint8, device="cuda")
     b = torch.empty(maxb, dtype=torch.uint8, device="cuda")
     a.random_(0, 256)
@@ -114,7 +122,7 @@ def collect(probs, num_sms, log_every=200):
         h = L.describe(dims, perm, es, num_sms=num_sms)
         for c in range(h["num_candidates"]):
             X.append(features(dims, perm, es, c, num_sms))
-            T.append(time_candidate(dims, perm, es, c, stream, a.data_ptr(), b.data_ptr(), ev))
+            T.append(time_candidate(dims, perm, es, c, stream, a.data_ptr(), b.data_ptr(), ev, maxb))
             P.append(i)
             C.append(c)
         heur.append(h["candidate"])  # the analytic model's pick (selector forced to analytic)
