@@ -393,8 +393,9 @@ bool loadSelectorModel(const char* path, std::string* why) {
 // Tiles whose candidates the learned model ranks: the analytic model's
 // cheapest few.  A short list of 4 tiles cost no measurable throughput
 // against ranking every candidate (random-shape suite geomean 6399.5 vs
-// 6399.0 GB/s on one GB300, held-out regret 1.53% vs 1.43%), while the
-// network runs on about half of them; 3 cost 0.5% on the suite.
+// 6399.0 GB/s on one GB300), while the network runs on about half of them; 3
+// cost 0.5% on the suite.  On the present timings, held out: 3.06 % regret, 2.23 %
+// ranking every candidate, 3.71 % with 3 tiles.
 int shortlistSize() {
   static const int k = [] {
     const char* e = std::getenv("LIBRETT_SELECTOR_SHORTLIST");
@@ -405,7 +406,7 @@ int shortlistSize() {
 }
 
 // Of the short-listed tiles, the cheapest SHORTLIST_TWINS also bring their
-// bulk-copy twin.  Held out (1,000 problems): twins of all 4 tiles 2.02 %
+// bulk-copy twin.  Held out (1,000 problems, an earlier model): twins of all 4 tiles 2.02 %
 // regret over 6.2 candidates, of the first 2 tiles 2.14 % over 5.0, of
 // none 2.66 % over 3.7; on the random-shape suite (1 GiB problems) twins of
 // only 2 tiles cost 0.4 % of throughput on one GB300, so all 4 keep them.
@@ -413,8 +414,8 @@ constexpr int SHORTLIST_TWINS = 4;
 // A twin joins only when the tile's input runs hold at least this many bytes:
 // in the timings, bulk copies of shorter runs rarely beat their per-unit
 // twin (128-255 bytes: 18 of 3528 tiles, 16 % slower at the median; 256-511:
-// 183 of 5613).  With the model trained on every candidate, the held-out
-// regret is 2.16 % over 4.62 candidates against 2.09 % over 6.20 without
+// 183 of 5613).  With an earlier model trained on every candidate, the held-out
+// regret was 2.16 % over 4.62 candidates against 2.09 % over 6.20 without
 // the rule and 2.13 % over 4.99 with 1 KiB (1,800 problems of 2^28 bytes
 // and more: 1.03 % against 0.99 %).  On one GB300 machine, 2 KiB against 1 KiB:
 // librettPlan 16.2-16.3 against 16.6-16.7 us, the random-shape suite
