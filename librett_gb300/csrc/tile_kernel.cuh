@@ -813,30 +813,6 @@ tileKernelBulkTables(const __grid_constant__ TileParams p,
   storeTileFlat<ES, SV>(p, stOff, stSm, pf, s, out + bout);
 }
 
-// Shared load where live (predicated as above); the result is undefined
-// where not live.
-template <int BYTES>
-__device__ __forceinline__ typename Word<BYTES>::T ldSharedIf(bool live, uint32_t addr) {
-  typename Word<BYTES>::T v;
-  if constexpr (BYTES == 4) {
-    asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %2, 0;\n @p ld.shared.b32 %0, [%1];\n}\n"
-                 : "=r"(v)
-                 : "r"(addr), "r"((int)live));
-  } else if constexpr (BYTES == 8) {
-    asm volatile(
-        "{\n .reg .pred p;\n setp.ne.b32 p, %3, 0;\n @p ld.shared.v2.b32 {%0, %1}, [%2];\n}\n"
-        : "=r"(v.x), "=r"(v.y)
-        : "r"(addr), "r"((int)live));
-  } else {
-    asm volatile(
-        "{\n .reg .pred p;\n setp.ne.b32 p, %5, 0;\n"
-        " @p ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];\n}\n"
-        : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
-        : "r"(addr), "r"((int)live));
-  }
-  return v;
-}
-
 template <int BYTES>
 __device__ __forceinline__ typename Word<BYTES>::T ldShared(uint32_t addr) {
   typename Word<BYTES>::T v;
