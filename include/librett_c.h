@@ -250,7 +250,8 @@ int librett_c_group_run_check(int rank, const int* dim, const int* permutation, 
 /* Host-only self-check of the table-free tile kernels' addressing for
  * flat-tile candidate `candidate` (in element units when element_units != 0):
  * the sums of thread and slot parts must reproduce the per-unit offset tables
- * for every unit of the tile.  Returns LIBRETT_SUCCESS when they do,
+ * for every unit of the tile, and where the tile is loaded by spans, those must
+ * bring every element to where the store side reads it.  Returns LIBRETT_SUCCESS when they do,
  * LIBRETT_INTERNAL_ERROR on a mismatch, LIBRETT_INVALID_DEVICE when the tile
  * has more ranks than those kernels take, LIBRETT_INVALID_PARAMETER for a bad
  * problem or candidate. */

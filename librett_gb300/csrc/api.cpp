@@ -588,6 +588,56 @@ bool slotsMatch(const lt::TileParams& tp, int esize, const int* ldOff, const int
   return true;
 }
 
+// Replays span loads for a tensor that starts at `start` modulo 16: the blocks
+// stay inside shared memory and apart from each other, bring every element to the
+// address that its digits name, and the store side reads it from there.
+template <int NI, int NTR>
+bool spanMatches(const lt::TileParams& tp, const lt::SpanLayout& L, int start, const int* ldOff,
+                 const int* stOff) {
+  constexpr int NS = lt::spanSlots(lt::TILE_MAX_SLOTS), ES = lt::SPAN_ES;
+  lt::StoreSlots<NS, NI> blocks;
+  lt::StoreSlots<lt::TILE_MAX_SLOTS, NTR> st;
+  lt::makeSpanSlots(L, blocks);
+  lt::makeStoreSlots(tp, L.stepJ, st);
+  if (L.units > NS * lt::TILE_THREADS) return false;
+  std::unordered_map<int, int64_t> at;  // shared word -> global element
+  int d[NTR > NI ? NTR : NI];
+  for (int u = 0; u < L.units; ++u) {
+    const int t = u % lt::TILE_THREADS, k = u / lt::TILE_THREADS;
+    uint32_t offT, jT, off, j;
+    lt::storeThreadOffset(blocks, (uint32_t)t, d, offT, jT);
+    lt::storeSlotOffset(blocks, k, offT, jT, d, off, j);
+    const int64_t a = (start + (int64_t)(int)off * ES) & ~int64_t(15);
+    const int sa = (start + (int)j) & ~15;
+    if (sa < 0 || sa + 16 > L.smBytes) return false;
+    for (int i = 0; i < 16; i += ES)
+      if (!at.emplace(sa + i, a + i - start).second) return false;
+  }
+  std::unordered_map<int, int64_t> in;  // input-order element -> global element
+  for (int u = 0; u < tp.nIn; ++u) in[u] = ldOff[u];
+  int step[lt::MAXR];
+  for (int i = 0; i < tp.nTR; ++i) step[i] = tp.toInTile[i];
+  for (int w = 0; w < tp.nOut; ++w) {
+    const int t = w % lt::TILE_THREADS, k = w / lt::TILE_THREADS;
+    uint32_t offT, jT, off, j;
+    lt::storeThreadOffset(st, (uint32_t)(t * tp.sv), d, offT, jT);
+    lt::storeSlotOffset(st, k, offT, jT, d, off, j);
+    if ((int)off != stOff[w]) return false;
+    for (int m = 0; m < tp.sv; ++m) {
+      uint32_t jm = j + (uint32_t)(m * L.stepJ[0]), o2;
+      if (tp.storeStraddle) lt::storeThreadOffset(st, (uint32_t)(w * tp.sv + m), d, o2, jm);
+      int x = w * tp.sv + m, e = 0;  // the element's input-order index
+      for (int i = 0; i < tp.nTR; ++i) {
+        e += x % tp.toE[i] * step[i];
+        x /= tp.toE[i];
+      }
+      auto it = at.find(start + (int)jm);
+      if (it == at.end() || it->second != (int64_t)in[e] * ES) return false;
+    }
+  }
+  return true;
+}
+
 }  // namespace
 
 extern "C" {
@@ -619,6 +669,20 @@ int librett_c_slot_check(int rank, const int* dim, const int* permutation, size_
     case 3: ok = few ? go(slotsMatch<2, 3>) : go(slotsMatch<3, 3>); break;
     case 4: ok = few ? go(slotsMatch<2, 4>) : go(slotsMatch<4, 4>); break;
     default: ok = few ? go(slotsMatch<2, 6>) : go(slotsMatch<6, 6>); break;
+  }
+  lt::SpanLayout span;
+  if (ok && lt::makeSpan(tp, es, span)) {
+    auto spans = [&](auto match) {
+      for (int start = 0; start < 16 && ok; start += es)
+        ok = match(tp, span, start, ldOff.data(), stOff.data());
+      return ok;
+    };
+    switch (lt::storeRankClass(tp)) {
+      case 2: ok = spans(spanMatches<2, 2>); break;
+      case 3: ok = few ? spans(spanMatches<2, 3>) : spans(spanMatches<3, 3>); break;
+      case 4: ok = few ? spans(spanMatches<2, 4>) : spans(spanMatches<4, 4>); break;
+      default: ok = few ? spans(spanMatches<2, 6>) : spans(spanMatches<6, 6>); break;
+    }
   }
   return ok ? LIBRETT_SUCCESS : LIBRETT_INTERNAL_ERROR;
 }

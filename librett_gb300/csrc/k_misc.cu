@@ -471,7 +471,7 @@ cudaError_t launchPlan(const PlanDesc& pd, const DeviceTables* dt, const void* i
       if ((pd.tile.lv > 1 || pd.tile.sv > 1) && align % 16 != 0) {
         // 16-byte units need 16-byte aligned tensors; fall back to element
         // units, in the flat pipeline (16.8M float32 elements one element
-        // off alignment: 26.9 us, against 51.0 in the register-staged
+        // off alignment: 25.6 us, against 51.0 in the register-staged
         // pipeline, which builds its tables in every CTA and holds 3 CTAs per
         // SM), or the register-staged one for tiles of more ranks than the
         // table-free kernels take

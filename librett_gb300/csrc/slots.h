@@ -14,7 +14,7 @@
 // with operands in the parameter block.
 //
 // Narrow units are bound by instruction issue: float32 (127, 63, 65, 33) perm
-// (3, 1, 2, 0), which moves in 4-byte units on both sides, issued 74 warp
+// (3, 1, 2, 0), which moved in 4-byte units on both sides, issued 74 warp
 // instructions per 32 elements with every element decoded on its own and 45
 // with slot sums (39.9 -> 30.9 us; 28.7 us with dependent launches as well).
 //
@@ -193,14 +193,96 @@ void makeLoadSlots(const TileParams& tp, LoadSlots<NS, NR>& s) {
                             s.off);
 }
 
+// stepJ: shared bytes between elements along each tile rank, in output order.
 template <int NS, int NR>
-void makeStoreSlots(const TileParams& tp, int esize, StoreSlots<NS, NR>& s) {
-  int stepJ[MAXR];
-  for (int i = 0; i < tp.nTR; ++i) stepJ[i] = tp.toInTile[i] * esize;
+void makeStoreSlots(const TileParams& tp, const int* stepJ, StoreSlots<NS, NR>& s) {
   detail::fillSlots<NS, NR>(tp.nTR, tp.toE, tp.toSout, TILE_THREADS * tp.sv, s.mul, s.ext, s.step,
                             s.corr, s.lim, s.off);
   detail::fillSlots<NS, NR>(tp.nTR, tp.toE, stepJ, TILE_THREADS * tp.sv, s.mul, s.ext, s.stepJ,
                             s.corrJ, s.lim, s.offJ);
+}
+
+template <int NS, int NR>
+void makeStoreSlots(const TileParams& tp, int esize, StoreSlots<NS, NR>& s) {
+  int stepJ[MAXR];
+  for (int i = 0; i < tp.nTR; ++i) stepJ[i] = tp.toInTile[i] * esize;
+  makeStoreSlots(tp, stepJ, s);
+}
+
+// Span loads of a tile whose input moves in element units: the contiguous runs
+// of its input come as the aligned 16-byte blocks around them (tileKernelSpan).
+// A run lies in shared memory at the same address modulo 16 as in global memory,
+// for every tile: a rank's shared step is congruent to its global step modulo 16,
+// so that shared addresses stay sums of digits times steps, and runs lie far
+// enough apart for the blocks around them.
+struct SpanLayout {
+  int perRun, units;  // blocks of a run, of the tile
+  int n;              // load ranks (loadRanks), the first of them the run
+  int ext[MAXR], step[MAXR], stepS[MAXR];  // extents; global (elements) and shared (bytes) steps
+  int stepJ[MAXR];    // shared step of each tile rank in output order
+  int smBytes;
+};
+
+// 4-byte elements in runs of 128 bytes or more.  float32 (r, 4000, 53) perm (2, 1,
+// 0), runs of r elements, in element units and in spans: r = 33 12.77 and 12.52 us,
+// 45 16.6 and 15.7, 61 22.1 and 20.2, 65 23.3 and 22.2, 126 (runs of 63) 43.5 and
+// 41.3.  Shorter runs read more than an eighth of their bytes again.  8-byte
+// elements have half the load instructions to save and lost: float64 (127, 63, 65,
+// 33) perm (3, 1, 2, 0) 46.5 and 47.7, (2, 4, 105, 294, 92) off alignment 55.2 and 61.5.
+constexpr int SPAN_ES = 4, SPAN_MIN_BYTES = 128, SPAN_MAX_SMEM = 48 * 1024;
+
+// Load slots of a tile of at most NL elements per thread: a run of
+// SPAN_MIN_BYTES or more takes at most 1/8 more blocks than its bytes fill.
+LT_HD constexpr int spanSlots(int NL) { return NL * SPAN_ES / 16 + 1; }
+
+inline bool makeSpan(const TileParams& tp, int esize, SpanLayout& L) {
+  if (esize != SPAN_ES || tp.lv != 1 || tp.nTR < 1 || tp.trSin[0] != 1) return false;
+  L.n = loadRanks(tp, L.ext, L.step);
+  const int bytes = L.ext[0] * esize;
+  if (bytes < SPAN_MIN_BYTES) return false;
+  L.perRun = (16 - esize + bytes + 15) / 16;
+  L.units = tp.tileVol / L.ext[0] * L.perRun;
+  int room = L.perRun * 16 + 15;  // of the ranks so far, wherever a block starts
+  L.stepS[0] = esize;
+  for (int r = 1; r < L.n; ++r) {
+    const int want = (int)((int64_t)L.step[r] * esize % 16);
+    L.stepS[r] = room + (want - room % 16 + 16) % 16;
+    // an odd number of 16-byte units at least: lanes that step along this rank
+    // then meet in 4 of 32 banks' worth at most, not in one bank
+    if (L.stepS[r] % 32 == 0) L.stepS[r] += 16;
+    room = L.ext[r] * L.stepS[r];
+  }
+  L.smBytes = (room + 16 + 15) / 16 * 16;  // and the tile's own start modulo 16
+  if (L.smBytes > SPAN_MAX_SMEM) return false;
+  // tile ranks merged into a load rank continue each other
+  int trStep[MAXR];
+  for (int t = 0, r = -1, left = 1; t < tp.nTR; ++t) {
+    if (left == 1) {
+      ++r;
+      left = L.ext[r];
+      trStep[t] = L.stepS[r];
+    } else {
+      trStep[t] = trStep[t - 1] * tp.trE[t - 1];
+    }
+    left /= tp.trE[t];
+  }
+  for (int i = 0; i < tp.nTR; ++i) L.stepJ[i] = trStep[tp.trOut[i]];
+  return true;
+}
+
+// Global offsets (elements) and shared addresses (bytes) of the blocks, before
+// both are rounded down to 16 bytes.
+template <int NS, int NR>
+void makeSpanSlots(const SpanLayout& L, StoreSlots<NS, NR>& s) {
+  int ext[MAXR], step[MAXR], stepS[MAXR];
+  for (int r = 0; r < L.n; ++r) {
+    ext[r] = r == 0 ? L.perRun : L.ext[r];
+    step[r] = r == 0 ? 16 / SPAN_ES : L.step[r];
+    stepS[r] = r == 0 ? 16 : L.stepS[r];
+  }
+  detail::fillSlots<NS, NR>(L.n, ext, step, TILE_THREADS, s.mul, s.ext, s.step, s.corr, s.lim, s.off);
+  detail::fillSlots<NS, NR>(L.n, ext, stepS, TILE_THREADS, s.mul, s.ext, s.stepJ, s.corrJ, s.lim,
+                            s.offJ);
 }
 
 // Grid ranks whose chunks fit the parameter block of rank class c.  The block
