@@ -33,7 +33,10 @@ __device__ __forceinline__ uint32_t fdiv(uint32_t n, const FastDiv& f) {
 // an ordinary launch) and calls dependencyRelease first, which lets its own
 // successor do the same as soon as all its CTAs run.  Loads that the compiler
 // may treat as invariant (const __restrict__ pointers) can be moved above the
-// wait, so such kernels load through ldGlobal.
+// wait, so such kernels load through ldGlobal.  A non-coherent load
+// (ld.global.nc, __ldg) is defined for memory that nobody writes while the
+// kernel runs; the predecessors still write these inputs then, so they are read by
+// ordinary loads only.  Tables fixed before the launch may be read either way.
 __device__ __forceinline__ void dependencyRelease() {
   asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
 }
@@ -46,11 +49,11 @@ template <int BYTES>
 __device__ __forceinline__ typename Word<BYTES>::T ldGlobal(const void* p) {
   typename Word<BYTES>::T v;
   if constexpr (BYTES == 4)
-    asm volatile("ld.global.nc.b32 %0, [%1];\n" : "=r"(v) : "l"(p) : "memory");
+    asm volatile("ld.global.b32 %0, [%1];\n" : "=r"(v) : "l"(p) : "memory");
   else if constexpr (BYTES == 8)
-    asm volatile("ld.global.nc.v2.b32 {%0, %1}, [%2];\n" : "=r"(v.x), "=r"(v.y) : "l"(p) : "memory");
+    asm volatile("ld.global.v2.b32 {%0, %1}, [%2];\n" : "=r"(v.x), "=r"(v.y) : "l"(p) : "memory");
   else
-    asm volatile("ld.global.nc.v4.b32 {%0, %1, %2, %3}, [%4];\n"
+    asm volatile("ld.global.v4.b32 {%0, %1, %2, %3}, [%4];\n"
                  : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
                  : "l"(p)
                  : "memory");
