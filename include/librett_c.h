@@ -195,6 +195,16 @@ int librett_c_mlp_forward(const float* params, const float* X, int batch, float*
                           void* stream);
 int librett_c_mlp_backward(const float* params, const float* X, int batch, float* ws,
                            const float* dout, float* grads, void* stream);
+/* Test hook for the network kernels' bounded waits: runs the forward rows
+ * (waits 0..2) or, with backward != 0, the backward rows (waits 0..1; out is
+ * then dout, X unused) once with `extra_bytes` (1..4096) more transaction bytes
+ * armed on that wait than its copies bring.  Every CTA gives up after its time
+ * limit (about 1 s, then up to 1 s more a wait for its copies) with NaN as its
+ * results: out and the workspace's three activations, or its two gradients.
+ * Synchronises the stream.  params must be 16-byte aligned, batch at most 4096.
+ * Nothing faults: the copies complete, only the armed count is never reached. */
+int librett_c_mlp_wait_test(int backward, int wait, unsigned extra_bytes, const float* params,
+                            const float* X, int batch, float* ws, float* out, void* stream);
 int librett_c_mlp_mse_grad(const float* out, const float* y, int batch, float* dout, float* loss,
                            void* stream);
 int librett_c_mlp_adam(float* params, const float* grads, float* m, float* v, int n, float lr,

@@ -109,6 +109,8 @@ C_FUNCTIONS = [
     ("librett_c_mlp_workspace_floats", ctypes.c_int, [ctypes.c_int]),
     ("librett_c_mlp_forward", ctypes.c_int, [_P, _P, ctypes.c_int, _P, _P, _P]),
     ("librett_c_mlp_backward", ctypes.c_int, [_P, _P, ctypes.c_int, _P, _P, _P, _P]),
+    ("librett_c_mlp_wait_test", ctypes.c_int,
+     [ctypes.c_int, ctypes.c_int, ctypes.c_uint, _P, _P, ctypes.c_int, _P, _P, _P]),
     ("librett_c_mlp_mse_grad", ctypes.c_int, [_P, _P, ctypes.c_int, _P, _P, _P]),
     ("librett_c_mlp_adam", ctypes.c_int,
      [_P, _P, _P, _P, ctypes.c_int, ctypes.c_float, ctypes.c_float, ctypes.c_float,

@@ -77,10 +77,17 @@ __device__ __forceinline__ void copyWait() {
 
 // Weights come by bulk copies that complete on an mbarrier (16 bytes per thread
 // and cp.async moved 25 bytes a cycle into an SM), where the parameters are
-// 16-byte aligned.  The waits are bounded like the transpose kernels': a copy
-// that does not arrive makes the CTA return without results, NaN as output.
+// 16-byte aligned.  The waits are bounded like the transpose kernels': when a
+// copy does not arrive in time, the CTA writes NaN for all of its results, waits
+// once more (bounded) for its copies in flight, and returns.
 struct Arrival {
   unsigned long long bar;
+};
+
+// Test hook: bytes armed beyond what the copies bring, per wait (zeros in every
+// other launch).
+struct ExtraBytes {
+  int wait[3];
 };
 
 __device__ __forceinline__ uint32_t sharedAddr(const void* p) {
@@ -98,6 +105,16 @@ __device__ __forceinline__ void bulkFloats(float* dst, const float* src, int n, 
 
 __device__ __forceinline__ bool arrived(Arrival& a) {
   return mbarWaitBounded(sharedAddr(&a.bar), 0, BULK_WAIT_NS);
+}
+
+// The bounded wait of a CTA that gives up: its copies write its shared memory.
+__device__ __forceinline__ void outlast(Arrival& a) {
+  mbarWaitBounded(sharedAddr(&a.bar), 0, BULK_WAIT_NS);
+}
+
+// NaN for n floats at p, by the CTA.
+__device__ __forceinline__ void fillNaN(float* p, int n) {
+  for (int i = threadIdx.x; i < n; i += blockDim.x) p[i] = nanf("");
 }
 
 // rows x cols of src (row stride sld) into dst (row stride dld) by cp.async, in
@@ -258,7 +275,7 @@ __device__ __forceinline__ void activate(const float (&acc)[Place<R>::TM][Place<
 template <int R>
 __global__ void __launch_bounds__(MLP_THREADS)
 mlpForwardKernel(const float* params, const float* X, int batch,
-                 float* ws, float* out) {
+                 float* ws, float* out, ExtraBytes extra) {
   using P = Place<R>;
   extern __shared__ __align__(16) unsigned char smraw[];
   ForwardShared<R>& s = *reinterpret_cast<ForwardShared<R>*>(smraw);
@@ -276,10 +293,10 @@ mlpForwardKernel(const float* params, const float* X, int batch,
   dependencyWait();
   if (vec) {
     if (threadIdx.x == 0) {
-      expect(s.first, H * NFEAT * 4);
+      expect(s.first, H * NFEAT * 4 + extra.wait[0]);
       bulkFloats(s.W1, L.W1, H * NFEAT, s.first);
-      expect(s.second, H * H * 4);
-      expect(s.third, H * H * 4);
+      expect(s.second, H * H * 4 + extra.wait[1]);
+      expect(s.third, H * H * 4 + extra.wait[2]);
     }
     __syncthreads();  // the counts are armed before a copy completes
     if (threadIdx.x < H) {
@@ -297,15 +314,22 @@ mlpForwardKernel(const float* params, const float* X, int batch,
   copyRows(s.b3, H, L.b3, 0, 1, H, vec);
   copyRows(s.W4, H, L.W4, 0, 1, H, vec);
   copyCommit();
-  bool ok = true;  // every copy arrived
   float* A1 = ws + (size_t)r0 * H;
   float* A2 = A1 + (size_t)batch * H;
   float* A3 = A2 + (size_t)batch * H;
+  auto giveUp = [&] {
+    fillNaN(A1, rows * H);
+    fillNaN(A2, rows * H);
+    fillNaN(A3, rows * H);
+    fillNaN(out + r0, rows);
+    outlast(s.first);
+    outlast(s.second);
+    outlast(s.third);
+  };
   // rows past the batch: any finite input
   for (int i = rows * XLD + threadIdx.x; i < R * XLD; i += MLP_THREADS) s.X[i] = 0.f;
   copyWait<0>();
-  if (vec) ok = arrived(s.first);
-  __syncthreads();
+  if (!__syncthreads_and(!vec || arrived(s.first))) return giveUp();
   {
     float acc[P::TM][P::TN] = {};
     const float* a = s.X + P::row() * XLD;
@@ -322,15 +346,13 @@ mlpForwardKernel(const float* params, const float* X, int batch,
     }
     activate<R>(acc, s.b1, s.A, A1, rows);
   }
-  if (vec) ok = arrived(s.second) && ok;
-  __syncthreads();
+  if (!__syncthreads_and(!vec || arrived(s.second))) return giveUp();
   {
     float acc[P::TM][P::TN] = {};
     layerTimesRows<R>(s.A, s.W2, acc);
     activate<R>(acc, s.b2, s.B, A2, rows);
   }
-  if (vec) ok = arrived(s.third) && ok;
-  __syncthreads();
+  if (!__syncthreads_and(!vec || arrived(s.third))) return giveUp();
   {
     float acc[P::TM][P::TN] = {};
     layerTimesRows<R>(s.B, s.W3, acc);
@@ -349,7 +371,7 @@ mlpForwardKernel(const float* params, const float* X, int batch,
       v = __fmaf_rn(av.z, wv.z, v);
       v = __fmaf_rn(av.w, wv.w, v);
     }
-    out[r0 + threadIdx.x] = ok ? v + *L.b4 : nanf("");
+    out[r0 + threadIdx.x] = v + *L.b4;
   }
 }
 
@@ -381,7 +403,7 @@ __device__ __forceinline__ void forOutputs(F f) {
 template <int R>
 __global__ void __launch_bounds__(MLP_THREADS)
 mlpBackwardRows(const float* params, int batch, float* ws,
-                const float* dout) {
+                const float* dout, ExtraBytes extra) {
   using P = Place<R>;
   extern __shared__ __align__(16) unsigned char smraw[];
   BackwardShared<R>& s = *reinterpret_cast<BackwardShared<R>*>(smraw);
@@ -399,9 +421,9 @@ mlpBackwardRows(const float* params, int batch, float* ws,
   if (vec) {
     if (threadIdx.x == 0) {
       constexpr int PIECE = H * H / 4;
-      expect(s.first, H * H * 4);
+      expect(s.first, H * H * 4 + extra.wait[0]);
       for (int i = 0; i < H * H; i += PIECE) bulkFloats(s.W3 + i, L.W3 + i, PIECE, s.first);
-      expect(s.second, H * H * 4);
+      expect(s.second, H * H * 4 + extra.wait[1]);
       for (int i = 0; i < H * H; i += PIECE) bulkFloats(s.W2 + i, L.W2 + i, PIECE, s.second);
     }
   } else {
@@ -409,13 +431,18 @@ mlpBackwardRows(const float* params, int batch, float* ws,
     copyRows(s.W2, H * H, L.W2, 0, 1, H * H, false);
     copyCommit();
   }
-  bool ok = true;  // every copy arrived
   const size_t part = (size_t)batch * H;
   const float* A1 = ws + (size_t)r0 * H;
   const float* A2 = A1 + part;
   const float* A3 = A2 + part;
   float* D1 = ws + 3 * part + (size_t)r0 * H;
   float* D2 = D1 + part;
+  auto giveUp = [&] {
+    fillNaN(D1, rows * H);
+    fillNaN(D2, rows * H);
+    outlast(s.first);
+    outlast(s.second);
+  };
   constexpr int PER = R * H / MLP_THREADS;  // elements of D3 a thread makes
   float a3[PER];
 #pragma unroll
@@ -434,27 +461,23 @@ mlpBackwardRows(const float* params, int batch, float* ws,
     on2[i][j] = r < rows && A2[(size_t)r * H + c] > 0.f;
     on1[i][j] = r < rows && A1[(size_t)r * H + c] > 0.f;
   });
-  if (vec)
-    ok = arrived(s.first);
-  else
-    copyWait<0>();
-  __syncthreads();
+  if (!vec) copyWait<0>();
+  if (!__syncthreads_and(!vec || arrived(s.first))) return giveUp();
   {
     float acc[P::TM][P::TN] = {};
     layerTimesCols<R>(s.D, s.W3, acc);
     forOutputs<R>([&](int i, int j, int r, int c) {
-      const float v = !ok ? nanf("") : on2[i][j] ? acc[i][j] : 0.f;
+      const float v = on2[i][j] ? acc[i][j] : 0.f;
       s.E[r * LD + c] = v;
       if (r < rows) D2[(size_t)r * H + c] = v;
     });
   }
-  if (vec) ok = arrived(s.second) && ok;
-  __syncthreads();
+  if (!__syncthreads_and(!vec || arrived(s.second))) return giveUp();
   {
     float acc[P::TM][P::TN] = {};
     layerTimesCols<R>(s.E, s.W2, acc);
     forOutputs<R>([&](int i, int j, int r, int c) {
-      if (r < rows) D1[(size_t)r * H + c] = !ok ? nanf("") : on1[i][j] ? acc[i][j] : 0.f;
+      if (r < rows) D1[(size_t)r * H + c] = on1[i][j] ? acc[i][j] : 0.f;
     });
   }
 }
@@ -687,6 +710,20 @@ cudaError_t launchRowsOf(int batch, cudaStream_t s, size_t sm8, size_t sm16, siz
   return launchDependent(kernel, (unsigned)((batch + R - 1) / R), MLP_THREADS, smem, s, args...);
 }
 
+cudaError_t forwardRows(const float* params, const float* X, int batch, float* ws, float* out,
+                        cudaStream_t s, const ExtraBytes& extra) {
+  return launchRowsOf(batch, s, sizeof(ForwardShared<8>), sizeof(ForwardShared<16>),
+                      sizeof(ForwardShared<32>), mlpForwardKernel<8>, mlpForwardKernel<16>,
+                      mlpForwardKernel<32>, params, X, batch, ws, out, extra);
+}
+
+cudaError_t backwardRows(const float* params, int batch, float* ws, const float* dout,
+                         cudaStream_t s, const ExtraBytes& extra) {
+  return launchRowsOf(batch, s, sizeof(BackwardShared<8>), sizeof(BackwardShared<16>),
+                      sizeof(BackwardShared<32>), mlpBackwardRows<8>, mlpBackwardRows<16>,
+                      mlpBackwardRows<32>, params, batch, ws, dout, extra);
+}
+
 }  // namespace
 }  // namespace lt
 
@@ -702,10 +739,7 @@ int librett_c_mlp_forward(const float* params, const float* X, int batch, float*
                           void* stream) {
   using namespace lt;
   if (!params || !X || !ws || !out || batch < 1) return LIBRETT_INVALID_PARAMETER;
-  const cudaError_t err = launchRowsOf(
-      batch, (cudaStream_t)stream, sizeof(ForwardShared<8>), sizeof(ForwardShared<16>),
-      sizeof(ForwardShared<32>), mlpForwardKernel<8>, mlpForwardKernel<16>, mlpForwardKernel<32>,
-      params, X, batch, ws, out);
+  const cudaError_t err = forwardRows(params, X, batch, ws, out, (cudaStream_t)stream, {});
   return err == cudaSuccess ? LIBRETT_SUCCESS : LIBRETT_INTERNAL_ERROR;
 }
 
@@ -714,15 +748,29 @@ int librett_c_mlp_backward(const float* params, const float* X, int batch, float
   using namespace lt;
   if (!params || !X || !ws || !dout || !grads || batch < 1) return LIBRETT_INVALID_PARAMETER;
   cudaStream_t s = (cudaStream_t)stream;
-  cudaError_t err = launchRowsOf(
-      batch, s, sizeof(BackwardShared<8>), sizeof(BackwardShared<16>), sizeof(BackwardShared<32>),
-      mlpBackwardRows<8>, mlpBackwardRows<16>, mlpBackwardRows<32>, params, batch, ws, dout);
+  cudaError_t err = backwardRows(params, batch, ws, dout, s, {});
   if (err == cudaSuccess)
     err = cachedOccupancy((const void*)mlpWeightGrads, GTHREADS, (int)sizeof(GradShared)) < 1
               ? cudaErrorInvalidConfiguration
               : launchDependent(mlpWeightGrads, GTILES * GC, GTHREADS, sizeof(GradShared), s, params, X,
                                 batch, (const float*)ws, dout, grads);
   return err == cudaSuccess ? LIBRETT_SUCCESS : LIBRETT_INTERNAL_ERROR;
+}
+
+int librett_c_mlp_wait_test(int backward, int wait, unsigned extra_bytes, const float* params,
+                            const float* X, int batch, float* ws, float* out, void* stream) {
+  using namespace lt;
+  if (!params || (!backward && !X) || !ws || !out || batch < 1 || batch > 4096 ||
+      (uintptr_t)params % 16 || wait < 0 || wait >= (backward ? 2 : 3) || extra_bytes == 0 ||
+      extra_bytes > 4096)
+    return LIBRETT_INVALID_PARAMETER;
+  ExtraBytes extra = {};
+  extra.wait[wait] = (int)extra_bytes;
+  cudaStream_t s = (cudaStream_t)stream;
+  const cudaError_t err = backward ? backwardRows(params, batch, ws, out, s, extra)
+                                   : forwardRows(params, X, batch, ws, out, s, extra);
+  return err == cudaSuccess && cudaStreamSynchronize(s) == cudaSuccess ? LIBRETT_SUCCESS
+                                                                       : LIBRETT_INTERNAL_ERROR;
 }
 
 int librett_c_mlp_mse_grad(const float* out, const float* y, int batch, float* dout, float* loss,
