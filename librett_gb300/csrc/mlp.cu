@@ -601,6 +601,7 @@ mlpWeightGrads(const float* params, const float* X, int batch, const float* ws, 
     }
     __syncthreads();  // the chunk after the next reuses this buffer
   }
+  cpAsyncWaitAll();  // W4's copy, in a CTA that had no rows
   // the parts' sums to shared memory, added in part order
   float* partial = s.chunk[0].D;  // the chunks' place, from its start
   if (layer == 4) {

@@ -39,3 +39,13 @@ def test_dependent_kernels_wait():
         for body in _code(path).split("__global__")[1:]:
             if "dependencyRelease()" in body:
                 assert re.search(r"dependencyWait\(\)|bulkIssue<|groupTileBody<", body), path.name
+
+
+def test_copies_are_waited_for():
+    """mlpWeightGrads: a CTA may have no rows (batches of 896 or fewer), so the wait
+    for the copies it starts before its loop over rows stands behind the loop."""
+    body = _code(CSRC / "mlp.cu").split("mlpWeightGrads(", 1)[1].split("__global__", 1)[0]
+    start = body.index("copyRows(s.W4")
+    loop = body.index("for (int b0 = first; b0 < batch; b0 += stride")
+    end = body.index("float* partial = ")
+    assert start < loop < body.index("cpAsyncWaitAll()") < end
