@@ -13,7 +13,9 @@
 // kernel takes 121 us (4-byte output units: two thirds of the issue slots).
 // The check shares no addressing with the single-plan kernels (slots.h).
 #include <cuda_runtime.h>
+#include <unistd.h>
 
+#include <cstdlib>
 #include <cstring>
 #include <mutex>
 #include <vector>
@@ -377,66 +379,91 @@ int verifyTiles(const Fused& f, int sms, const void* in, const void* out, Verify
 // A call's result: two zeroed words of mapped host memory that the kernel adds
 // to and the host reads after its synchronisation, so that a call makes no
 // device allocation, memset or copy (together 150 us a call, with the default
-// pool giving its memory back at every synchronisation).  The slots come from
-// one page, kept until the process exits; a call beyond them allocates its own.
+// pool giving its memory back at every synchronisation).  The slots lie in one page
+// of the process's own memory, registered with CUDA by the first call and again by
+// the first one after a cudaDeviceReset, which ends the registration; a call
+// beyond the page's slots allocates its own.
 class ResultSlot {
  public:
   ResultSlot() {
     {
       std::lock_guard<std::mutex> lk(mutex());
       std::vector<unsigned long long*>& f = freeSlots();
-      static bool made = false;
-      if (!made) {
-        made = true;
-        if (void* page = allocate(PAGE))
-          for (size_t k = 0; k < PAGE / SLOT; ++k)
-            f.push_back(reinterpret_cast<unsigned long long*>(static_cast<char*>(page) + k * SLOT));
-      }
-      if (!f.empty()) {
+      static const bool made = addPage(f);
+      if (made && !f.empty()) {
         p_ = f.back();
         f.pop_back();
       }
     }
-    if (p_ == nullptr) {
-      p_ = static_cast<unsigned long long*>(allocate(SLOT));
-      own_ = true;
+    if (p_ != nullptr) d_ = pageAddress();
+    if (d_ == nullptr) {
+      giveBack();
+      own_ = p_ = allocate();
+      d_ = address();
     }
     if (p_ != nullptr) p_[0] = p_[1] = 0;
   }
   ~ResultSlot() {
-    if (p_ == nullptr) return;
-    if (own_) {
+    if (own_ != nullptr) {
       const Uncaptured relaxed;
-      cudaFreeHost(p_);
-      return;
+      cudaFreeHost(own_);
+    } else {
+      giveBack();
     }
-    std::lock_guard<std::mutex> lk(mutex());
-    freeSlots().push_back(p_);
   }
   ResultSlot(const ResultSlot&) = delete;
   ResultSlot& operator=(const ResultSlot&) = delete;
   volatile unsigned long long* host() const { return p_; }
   // Its address on the current device, nullptr when there is none.
-  unsigned long long* device() const {
-    void* d = nullptr;
-    if (p_ == nullptr || cudaHostGetDevicePointer(&d, p_, 0) != cudaSuccess) return nullptr;
-    return static_cast<unsigned long long*>(d);
-  }
+  unsigned long long* device() const { return d_; }
 
  private:
-  static constexpr size_t PAGE = 4096, SLOT = 64;  // bytes
-  // Allocating is no error, and ends no capture, while another thread captures
-  // a stream.
+  static constexpr size_t SLOTS = 64, SLOT = 64;  // bytes of a slot
+  // Allocating and registering is no error, and ends no capture, while another
+  // thread captures a stream.
   struct Uncaptured {
     cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
     Uncaptured() { cudaThreadExchangeStreamCaptureMode(&mode); }
     ~Uncaptured() { cudaThreadExchangeStreamCaptureMode(&mode); }
   };
-  static void* allocate(size_t bytes) {
+  static unsigned long long* allocate() {
     const Uncaptured relaxed;
     void* p = nullptr;
     const unsigned flags = cudaHostAllocMapped | cudaHostAllocPortable;
-    return cudaHostAlloc(&p, bytes, flags) == cudaSuccess ? p : nullptr;
+    if (cudaHostAlloc(&p, SLOT, flags) == cudaSuccess) return static_cast<unsigned long long*>(p);
+    cudaGetLastError();
+    return nullptr;
+  }
+  // Whole pages of their own, so that no other registration touches them.
+  static bool addPage(std::vector<unsigned long long*>& f) {
+    const long unit = sysconf(_SC_PAGESIZE);
+    pageBytes() = (SLOTS * SLOT + unit - 1) / unit * unit;
+    if (posix_memalign(&page(), (size_t)unit, pageBytes()) != 0) return false;
+    for (size_t k = 0; k < SLOTS; ++k)
+      f.push_back(reinterpret_cast<unsigned long long*>(static_cast<char*>(page()) + k * SLOT));
+    return true;
+  }
+  unsigned long long* address() const {
+    void* d = nullptr;
+    if (p_ == nullptr) return nullptr;
+    if (cudaHostGetDevicePointer(&d, p_, 0) == cudaSuccess) return static_cast<unsigned long long*>(d);
+    cudaGetLastError();  // not registered
+    return nullptr;
+  }
+  unsigned long long* pageAddress() const {
+    if (unsigned long long* d = address()) return d;
+    const Uncaptured relaxed;
+    // (an error when another thread was faster)
+    if (cudaHostRegister(page(), pageBytes(), cudaHostRegisterMapped | cudaHostRegisterPortable) !=
+        cudaSuccess)
+      cudaGetLastError();
+    return address();
+  }
+  void giveBack() {
+    if (p_ == nullptr) return;
+    std::lock_guard<std::mutex> lk(mutex());
+    freeSlots().push_back(p_);
+    p_ = nullptr;
   }
   static std::mutex& mutex() {
     static std::mutex m;
@@ -446,8 +473,15 @@ class ResultSlot {
     static auto* f = new std::vector<unsigned long long*>();  // lives until the process exits
     return *f;
   }
-  unsigned long long* p_ = nullptr;
-  bool own_ = false;
+  static void*& page() {
+    static void* p = nullptr;
+    return p;
+  }
+  static size_t& pageBytes() {
+    static size_t n = 0;
+    return n;
+  }
+  unsigned long long *p_ = nullptr, *own_ = nullptr, *d_ = nullptr;
 };
 
 }  // namespace
@@ -476,14 +510,15 @@ extern "C" int librett_c_verify(int rank, const int* dim, const int* permutation
       smem > 0 ? lt::verifyKernelOf(reinterpret_cast<const lt::TileBlock*>(tiles.block)->store) : nullptr;
   const int occ =
       kernel ? lt::cachedOccupancy((const void*)kernel, lt::TILE_THREADS, smem) : 0;
-  cudaError_t err;
+  cudaError_t err = cudaErrorInvalidConfiguration;
   if (occ > 0) {
     const uint32_t wave = (uint32_t)(sms * occ);
     kernel<<<tiles.numTiles < wave ? tiles.numTiles : wave, lt::TILE_THREADS, smem, s>>>(tiles, d);
     err = cudaGetLastError();
-  } else {
-    err = lt::verifyElements(f, sms, idata, odata, d, s);
   }
+  // (a launch is refused, too, when a device reset took the kernel's shared-memory limit)
+  if (err == cudaErrorInvalidConfiguration || err == cudaErrorInvalidValue)
+    err = lt::verifyElements(f, sms, idata, odata, d, s);
   // also after an error: a launch may have been made
   const cudaError_t done = cudaStreamSynchronize(s);
   if (err != cudaSuccess || done != cudaSuccess) return LIBRETT_INTERNAL_ERROR;
