@@ -280,6 +280,16 @@ int librett_c_slot_check(int rank, const int* dim, const int* permutation, size_
 int librett_c_group_box_check(int rank, const int* dim, const int* permutation, size_t sizeofType,
                               int num_sms, int candidate, int variant);
 
+/* Host-only self-check of librett_c_verify's addressing: the map of its tile must
+ * be the transpose formula's (each check repeats that on the device and goes
+ * element by element where it fails), and the elements that its tiles own must add
+ * up to the tensor.  mistake 1..9 plants one first: the check must then fail.
+ * Returns LIBRETT_SUCCESS when the addressing holds, LIBRETT_INTERNAL_ERROR when it
+ * does not, LIBRETT_INVALID_DEVICE where the problem has no tile, or the mistake no
+ * place in it, LIBRETT_INVALID_PARAMETER for a bad problem or mistake. */
+int librett_c_verify_map_check(int rank, const int* dim, const int* permutation, size_t sizeofType,
+                               int num_sms, int element_units, int mistake);
+
 /* Host-only self-check of the bulk-copy pipeline for candidate `candidate`
  * of the planner's candidate list (candidate set 1): every segment the
  * kernel copies with one cp.async.bulk must be contiguous in global memory

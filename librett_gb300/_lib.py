@@ -143,10 +143,10 @@ C_FUNCTIONS = [
     ("librett_c_slot_check", ctypes.c_int,
      [ctypes.c_int, ctypes.POINTER(ctypes.c_int), ctypes.POINTER(ctypes.c_int), ctypes.c_size_t,
       ctypes.c_int, ctypes.c_int, ctypes.c_int]),
-    ("librett_c_group_box_check", ctypes.c_int,
+    ("librett_c_verify_map_check", ctypes.c_int,
      [ctypes.c_int, ctypes.POINTER(ctypes.c_int), ctypes.POINTER(ctypes.c_int), ctypes.c_size_t,
       ctypes.c_int, ctypes.c_int, ctypes.c_int]),
-    ("librett_c_slot_check", ctypes.c_int,
+    ("librett_c_group_box_check", ctypes.c_int,
      [ctypes.c_int, ctypes.POINTER(ctypes.c_int), ctypes.POINTER(ctypes.c_int), ctypes.c_size_t,
       ctypes.c_int, ctypes.c_int, ctypes.c_int]),
     ("librett_c_bulk_check", ctypes.c_int,

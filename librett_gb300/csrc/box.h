@@ -136,4 +136,37 @@ LT_HD int boxDecode(const BoxRank* rank, int p, uint32_t x, uint32_t& off, uint3
   return (int)x;
 }
 
+struct Place {  // of a thread on one side
+  uint32_t off, sm;
+  int slots;  // it takes part in
+};
+
+LT_HD Place placeAt(const unsigned char* block, const BoxHead& h, uint32_t thread) {
+  Place t;
+  const BoxRank* rank = reinterpret_cast<const BoxRank*>(block + h.rankAt);
+  const int top = boxDecode(rank, h.p, thread * h.unit, t.off, t.sm);
+  t.slots = (int)thread >= h.active ? 0 : h.nFull + (top < h.rem ? h.nRagged : 0);
+  return t;
+}
+
+// Shared addresses of the SV elements of a thread's store unit, the first at
+// sm0.
+template <int SV>
+LT_HD void elementsAt(const unsigned char* block, const TileBlock& g, uint32_t thread, uint32_t sm0,
+                      uint32_t (&sm)[SV]) {
+  sm[0] = sm0;
+#pragma unroll
+  for (int m = 1; m < SV; ++m) sm[m] = sm0 + (uint32_t)m * g.elemStep;
+  if (SV > 1 && g.straddle) {
+    const BoxRank* rank = reinterpret_cast<const BoxRank*>(block + g.st.rankAt);
+    uint32_t off, first, j;
+    boxDecode(rank, g.st.p, thread * SV, off, first);
+#pragma unroll
+    for (int m = 1; m < SV; ++m) {
+      boxDecode(rank, g.st.p, thread * SV + m, off, j);
+      sm[m] = sm0 + j - first;
+    }
+  }
+}
+
 }  // namespace lt

@@ -7,17 +7,8 @@
 
 namespace lt {
 
-struct Place {  // of a thread on one side
-  uint32_t off, sm;
-  int slots;  // it takes part in
-};
-
 __device__ __forceinline__ Place placeOf(const unsigned char* block, const BoxHead& h) {
-  Place t;
-  const BoxRank* rank = reinterpret_cast<const BoxRank*>(block + h.rankAt);
-  const int top = boxDecode(rank, h.p, threadIdx.x * h.unit, t.off, t.sm);
-  t.slots = (int)threadIdx.x >= h.active ? 0 : h.nFull + (top < h.rem ? h.nRagged : 0);
-  return t;
+  return placeAt(block, h, threadIdx.x);
 }
 
 // Runs f(slots...) for slots 0 .. n - 1 (n may differ between threads), PER (1,
@@ -50,24 +41,10 @@ __device__ __forceinline__ void loadTile(const unsigned char* block, const BoxHe
   });
 }
 
-// Shared addresses of the SV elements of a thread's store unit, the first at
-// sm0.
 template <int SV>
 __device__ __forceinline__ void elementsOf(const unsigned char* block, const TileBlock& g,
                                            uint32_t sm0, uint32_t (&sm)[SV]) {
-  sm[0] = sm0;
-#pragma unroll
-  for (int m = 1; m < SV; ++m) sm[m] = sm0 + (uint32_t)m * g.elemStep;
-  if (SV > 1 && g.straddle) {
-    const BoxRank* rank = reinterpret_cast<const BoxRank*>(block + g.st.rankAt);
-    uint32_t off, first, j;
-    boxDecode(rank, g.st.p, threadIdx.x * SV, off, first);
-#pragma unroll
-    for (int m = 1; m < SV; ++m) {
-      boxDecode(rank, g.st.p, threadIdx.x * SV + m, off, j);
-      sm[m] = sm0 + j - first;
-    }
-  }
+  elementsAt<SV>(block, g, threadIdx.x, sm0, sm);
 }
 
 }  // namespace lt

@@ -7,17 +7,22 @@
 //
 // The input is read a tile at a time through shared memory (box.h), because the
 // elements that consecutive output elements name lie far apart: gathering them
-// one by one from global memory (verifyKernel, kept for tiles without a box)
+// one by one from global memory (verifyKernel, kept for problems without a sound tile)
 // fetched 32 bytes for 4 and took 745 us for 66.8M float32 elements (64, 128,
 // 96, 85) perm (3, 1, 0, 2), where the two tensors' bytes take 80 us; this
 // kernel takes 121 us (4-byte output units: two thirds of the issue slots).
-// The check shares no addressing with the single-plan kernels (slots.h).
+// The tile's addressing is the grouped kernel's, the grid and the proof that the
+// addressing is the transpose formula's are this file's own: each check replays its
+// tile's map (verify_map.h), and where that fails, which no problem is
+// known to do, the check is made element by element.
 #include <cuda_runtime.h>
 #include <unistd.h>
 
+#include <algorithm>
 #include <cstdlib>
 #include <cstring>
 #include <mutex>
+#include <utility>
 #include <vector>
 
 #include "box_kernel.cuh"
@@ -25,6 +30,7 @@
 #include "librett_c.h"
 #include "plan.h"
 #include "plans.h"
+#include "verify_map.h"
 
 namespace lt {
 namespace {
@@ -141,6 +147,8 @@ struct VerifyTiles {
   // no rank above).
   uint32_t overlap[MAXR];
   FastDiv outStep[MAXR], outDim[MAXR];
+  int smBytes;  // of the tile, behind the block
+  TileMap map;
   uint4 block[TILE_BLOCK_MAX / 16];
 };
 
@@ -153,12 +161,11 @@ constexpr uint32_t VERIFY_LIST = 64;  // tiles with differences a CTA lists
 
 // Corners of a tile; returns the grid ranks along which it overlaps its neighbour,
 // as bits.
-__device__ __forceinline__ uint32_t tileCorner(const VerifyTiles& p, uint32_t tile, long long& bin,
-                                               long long& bout) {
+LT_HD uint32_t tileCorner(const VerifyTiles& p, uint32_t tile, long long& bin, long long& bout) {
   bin = bout = 0;
   uint32_t rem = tile, shared = 0;
   for (int r = 0; r < p.nGR; ++r) {
-    const uint32_t q = fdiv(rem, p.grDiv[r]);
+    const uint32_t q = mapDiv(rem, p.grDiv[r]);
     const uint32_t c = rem - q * p.grDiv[r].d;
     rem = q;
     const bool last = c + 1 == p.grDiv[r].d;
@@ -209,6 +216,8 @@ verifyTilesKernel(const __grid_constant__ VerifyTiles p, unsigned long long* res
     found = {0ull, ~0ull};
     numListed = 0;
   }
+  dependencyRelease();  // of the map's kernel
+  dependencyWait();     // at once: launched ordinarily
   for (int c = threadIdx.x; c < p.blockBytes / 16; c += blockDim.x)
     reinterpret_cast<uint4*>(smraw)[c] = p.block[c];
   __syncthreads();
@@ -318,17 +327,96 @@ verifyTilesKernel(const __grid_constant__ VerifyTiles p, unsigned long long* res
   if (threadIdx.x == 0) report(found.bad, found.first, result);
 }
 
+// Replays the tile's map (verify_map.h), one CTA, next to the check itself: it is
+// launched dependently behind that and touches none of the tensors.  Inside the
+// check's kernel, as its last CTA's first work, it cost the others registers (135 ->
+// 149 us for 256 MB); behind it 1 to 3 us of any check.
+template <int ES, int SV>
+__global__ void __launch_bounds__(TILE_THREADS)
+verifyMapKernel(const __grid_constant__ VerifyTiles p, unsigned long long* result) {
+  extern __shared__ __align__(16) unsigned char smraw[];
+  __shared__ int count[3];  // loaded, compared, marked
+  uint32_t* cell = reinterpret_cast<uint32_t*>(smraw + p.blockBytes);
+  const uint32_t smBytes = (uint32_t)p.smBytes;
+  for (uint32_t i = threadIdx.x; i < smBytes / 4; i += TILE_THREADS) cell[i] = CELL_EMPTY;
+  for (int c = threadIdx.x; c < p.blockBytes / 16; c += TILE_THREADS)
+    reinterpret_cast<uint4*>(smraw)[c] = p.block[c];
+  if (threadIdx.x < 3) count[threadIdx.x] = 0;
+  __syncthreads();
+  int loaded = 0, compared = 0, marked = 0;
+  bool ok = mapLoads(smraw, threadIdx.x, smBytes, loaded,
+                     [&](uint32_t at, uint32_t v) { cell[at / 4] = v; });
+  __syncthreads();
+  ok = mapStores<ES, SV>(p.map, smraw, threadIdx.x, smBytes, compared,
+                         [&](uint32_t at) { return cell[at / 4]; }) && ok;
+  __syncthreads();
+  mapMark<ES, SV>(smraw, threadIdx.x, smBytes, [&](uint32_t at) { cell[at / 4] = CELL_USED; });
+  __syncthreads();
+  for (uint32_t i = threadIdx.x; i < smBytes / 4; i += TILE_THREADS)
+    marked += cell[i] == CELL_USED ? 1 : 0;
+  loaded = __reduce_add_sync(~0u, loaded);
+  compared = __reduce_add_sync(~0u, compared);
+  marked = __reduce_add_sync(~0u, marked);
+  if (threadIdx.x % 32 == 0) {
+    atomicAdd(&count[0], loaded);
+    atomicAdd(&count[1], compared);
+    atomicAdd(&count[2], marked);
+  }
+  ok = __syncthreads_and(ok) != 0;
+  ok = ok && count[0] == p.map.vol && count[1] == p.map.vol && count[2] == p.map.vol;
+  if (!ok && threadIdx.x == 0) atomicAdd_system(result + 2, 1ull);
+  dependencyWait();
+}
+
+
 using VerifyKernel = void (*)(const VerifyTiles, unsigned long long*);
 
-VerifyKernel verifyKernelOf(int store) {
+// The check's kernel and its map's.
+struct VerifyKernels {
+  VerifyKernel tiles = nullptr, map = nullptr;
+};
+
+VerifyKernels verifyKernelsOf(int store) {
   switch (store) {
-    case blockStore(4, 4): return verifyTilesKernel<4, 4>;
-    case blockStore(4, 1): return verifyTilesKernel<4, 1>;
-    case blockStore(8, 2): return verifyTilesKernel<8, 2>;
-    case blockStore(8, 1): return verifyTilesKernel<8, 1>;
-    case blockStore(16, 1): return verifyTilesKernel<16, 1>;
-    default: return nullptr;
+#define LT_VERIFY(ES, SV) \
+  case blockStore(ES, SV): return {verifyTilesKernel<ES, SV>, verifyMapKernel<ES, SV>};
+    LT_VERIFY(4, 4)
+    LT_VERIFY(4, 1)
+    LT_VERIFY(8, 2)
+    LT_VERIFY(8, 1)
+    LT_VERIFY(16, 1)
+#undef LT_VERIFY
+    default: return {};
   }
+}
+
+// Launches the check over tiles and the replay of their map; an error where one of
+// them cannot be launched (the check may have been).
+cudaError_t checkTiles(const VerifyTiles& tiles, int sms, int smem, unsigned long long* d,
+                       cudaStream_t s) {
+  const VerifyKernels k = verifyKernelsOf(reinterpret_cast<const TileBlock*>(tiles.block)->store);
+  if (k.tiles == nullptr) return cudaErrorInvalidConfiguration;
+  const int occ = cachedOccupancy((const void*)k.tiles, TILE_THREADS, smem);
+  if (occ < 1 || cachedOccupancy((const void*)k.map, TILE_THREADS, smem) < 1)
+    return cudaErrorInvalidConfiguration;
+  k.tiles<<<std::min(tiles.numTiles, (uint32_t)(sms * occ)), TILE_THREADS, smem, s>>>(tiles, d);
+  const cudaError_t err = cudaGetLastError();
+  return err != cudaSuccess ? err : launchDependent(k.map, 1, TILE_THREADS, smem, s, tiles, d);
+}
+
+// Adds a grid rank: chunks of ext along dim, the last one ending at dim.
+void addGridRank(int64_t dim, int64_t ext, int64_t sin, int64_t sout, VerifyTiles& p) {
+  const int g = p.nGR++;
+  p.grDiv[g] = makeFastDiv((uint32_t)((dim + ext - 1) / ext));
+  p.grSin[g] = ext * sin;
+  p.grSout[g] = ext * sout;
+  p.grLastIn[g] = (dim - ext) * sin;
+  p.grLastOut[g] = (dim - ext) * sout;
+  // extents of 2 and more have strides below 2^31 (the tile's span is)
+  p.overlap[g] = dim % ext != 0 ? (uint32_t)(ext - dim % ext) : 0;
+  if (p.overlap[g] == 0) return;
+  p.outStep[g] = makeFastDiv((uint32_t)sout);
+  p.outDim[g] = dim < (int64_t(1) << 31) ? makeFastDiv((uint32_t)dim) : FastDiv{};
 }
 
 // Fills p for a check of in against out; the kernel's shared memory returned,
@@ -349,26 +437,24 @@ int verifyTiles(const Fused& f, int sms, const void* in, const void* out, Verify
   const TileParams& tp = pd.tile;
   static thread_local BoxParams b;
   if (!makeBox(tp, f.esize, b, false)) return 0;
-  p.numTiles = tp.numTiles;
-  p.nGR = tp.nGR;
+  // The grid from the extents; the tile only says in which order its ranks go.
+  int64_t tiles = 1;
+  p.nGR = 0;
+  uint32_t seen = 0;
   for (int g = 0; g < tp.nGR; ++g) {
-    p.grDiv[g] = tp.grDiv[g];
-    p.grSin[g] = tp.grSin[g];
-    p.grSout[g] = tp.grSout[g];
-    p.grLastIn[g] = tp.grLastIn[g];
-    p.grLastOut[g] = tp.grLastOut[g];
-    int r = 0;  // the rank: input strides of a chunk differ between ranks
-    while (r < f.rank && (pd.extent[r] * f.sin[r] != tp.grSin[g] ||
-                          pd.extent[r] * f.sout[r] != tp.grSout[g] || f.dim[r] <= pd.extent[r]))
-      ++r;
-    if (r == f.rank) return 0;
-    // extents of 2 and more have a stride below 2^31 (the tile's span is)
-    const int64_t ragged = f.dim[r] % pd.extent[r];
-    p.overlap[g] = ragged != 0 ? (uint32_t)(pd.extent[r] - ragged) : 0;
-    if (p.overlap[g] == 0) continue;
-    p.outStep[g] = makeFastDiv((uint32_t)f.sout[r]);
-    p.outDim[g] = f.dim[r] < (int64_t(1) << 31) ? makeFastDiv((uint32_t)f.dim[r]) : FastDiv{};
+    int r = 0;  // input strides of a chunk differ between ranks
+    while (r < f.rank && (pd.extent[r] * f.sin[r] != tp.grSin[g] || pd.extent[r] >= f.dim[r])) ++r;
+    if (r == f.rank || (seen >> r & 1) != 0) return 0;
+    seen |= 1u << r;
+    addGridRank(f.dim[r], pd.extent[r], f.sin[r], f.sout[r], p);
+    tiles *= p.grDiv[g].d;
+    if (tiles >= (int64_t(1) << 31)) return 0;
   }
+  for (int r = 0; r < f.rank; ++r)  // every other rank lies in the tile whole
+    if ((seen >> r & 1) == 0 && pd.extent[r] != f.dim[r]) return 0;
+  p.numTiles = (uint32_t)tiles;
+  p.smBytes = b.smBytes;
+  p.map = makeTileMap(f, pd.extent);
   const std::vector<unsigned char> block =
       packBlock(b, f.esize, in, const_cast<void*>(out));
   p.blockBytes = (int)block.size();
@@ -376,7 +462,8 @@ int verifyTiles(const Fused& f, int sms, const void* in, const void* out, Verify
   return p.blockBytes + b.smBytes;
 }
 
-// A call's result: two zeroed words of mapped host memory that the kernel adds
+// A call's result: three zeroed words (wrong elements, the complement of the first
+// one's index, whether the tile's map failed) of mapped host memory that the kernel adds
 // to and the host reads after its synchronisation, so that a call makes no
 // device allocation, memset or copy (together 150 us a call, with the default
 // pool giving its memory back at every synchronisation).  The slots lie in one page
@@ -401,7 +488,7 @@ class ResultSlot {
       own_ = p_ = allocate();
       d_ = address();
     }
-    if (p_ != nullptr) p_[0] = p_[1] = 0;
+    if (p_ != nullptr) clear();
   }
   ~ResultSlot() {
     if (own_ != nullptr) {
@@ -414,6 +501,7 @@ class ResultSlot {
   ResultSlot(const ResultSlot&) = delete;
   ResultSlot& operator=(const ResultSlot&) = delete;
   volatile unsigned long long* host() const { return p_; }
+  void clear() { p_[0] = p_[1] = p_[2] = 0; }
   // Its address on the current device, nullptr when there is none.
   unsigned long long* device() const { return d_; }
 
@@ -487,6 +575,139 @@ class ResultSlot {
 }  // namespace
 }  // namespace lt
 
+namespace lt {
+namespace {
+
+// mapIsSound on the host.
+template <int ES, int SV>
+bool mapIsSoundHost(const VerifyTiles& p, const unsigned char* block) {
+  std::vector<uint32_t> cells(p.smBytes / 4, CELL_EMPTY);
+  int loaded = 0, compared = 0;
+  bool ok = true;
+  const uint32_t smBytes = (uint32_t)p.smBytes;
+  for (uint32_t t = 0; t < TILE_THREADS; ++t)
+    ok = mapLoads(block, t, smBytes, loaded, [&](uint32_t at, uint32_t v) { cells[at / 4] = v; }) && ok;
+  for (uint32_t t = 0; t < TILE_THREADS; ++t)
+    ok = mapStores<ES, SV>(p.map, block, t, smBytes, compared,
+                           [&](uint32_t at) { return cells[at / 4]; }) && ok;
+  for (uint32_t t = 0; t < TILE_THREADS; ++t)
+    mapMark<ES, SV>(block, t, smBytes, [&](uint32_t at) { cells[at / 4] = CELL_USED; });
+  const int marked = (int)std::count(cells.begin(), cells.end(), CELL_USED);
+  return ok && loaded == p.map.vol && compared == p.map.vol && marked == p.map.vol;
+}
+
+bool mapIsSoundHost(const VerifyTiles& p) {
+  const unsigned char* block = reinterpret_cast<const unsigned char*>(p.block);
+  switch (reinterpret_cast<const TileBlock*>(block)->store) {
+    case blockStore(4, 4): return mapIsSoundHost<4, 4>(p, block);
+    case blockStore(4, 1): return mapIsSoundHost<4, 1>(p, block);
+    case blockStore(8, 2): return mapIsSoundHost<8, 2>(p, block);
+    case blockStore(8, 1): return mapIsSoundHost<8, 1>(p, block);
+    default: return mapIsSoundHost<16, 1>(p, block);
+  }
+}
+
+// Every tile's corner is the formula's, and the elements that the tiles own add up
+// to the tensor.
+bool gridIsSound(const Fused& f, const VerifyTiles& p) {
+  uint64_t owned = 0;
+  for (uint32_t tile = 0; tile < p.numTiles; ++tile) {
+    long long bin, bout;
+    uint32_t shared = tileCorner(p, tile, bin, bout);
+    long long rem = bout, src = 0;
+    uint64_t mine = 1;
+    uint32_t ranks = 0;
+    for (int i = 0; i < f.rank; ++i) {
+      const int r = f.perm[i];
+      const long long c = rem % f.dim[r];
+      if (c + p.map.ext[i] > f.dim[r]) return false;
+      src += c * f.sin[r];
+      rem /= f.dim[r];
+      // the rank's first digits, where the tile before owns them
+      uint64_t digits = p.map.ext[i];
+      for (int g = 0; g < p.nGR; ++g)
+        if ((shared >> g & 1) != 0 && p.outStep[g].d == (uint64_t)f.sout[r]) {
+          digits -= p.overlap[g];
+          ranks |= 1u << g;
+        }
+      mine *= digits;
+    }
+    if (src != bin || rem != 0 || ranks != shared) return false;
+    owned += mine;
+  }
+  return owned == (uint64_t)f.vol;
+}
+
+// Plants mistake 1 .. 9 in a check's addressing; false where it has no place.
+bool plant(int mistake, VerifyTiles& p) {
+  unsigned char* block = reinterpret_cast<unsigned char*>(p.block);
+  TileBlock& g = *reinterpret_cast<TileBlock*>(block);
+  BoxSlot* ld = reinterpret_cast<BoxSlot*>(block + g.ld.slotAt);
+  BoxSlot* st = reinterpret_cast<BoxSlot*>(block + g.st.slotAt);
+  BoxRank* rank = reinterpret_cast<BoxRank*>(block + g.ld.rankAt);
+  switch (mistake) {
+    case 1:  // two slots' input, exchanged: every element still arrives somewhere
+      if (g.ld.nFull < 2) return false;
+      std::swap(ld[0].off, ld[1].off);
+      return true;
+    case 2:  // two slots' places in shared memory, exchanged
+      if (g.st.nFull < 2) return false;
+      std::swap(st[0].sm, st[1].sm);
+      return true;
+    case 3:  // the output of a slot
+      if (g.st.nFull < 2) return false;
+      st[0].off = st[1].off;
+      return true;
+    case 4:  // a step of the input
+      rank[0].step += 1;
+      return g.ld.active > 1 && (g.ld.p == 0 || (int)rank[0].ext > g.ld.unit);
+    case 5:  // elements left out
+      if (g.st.nFull < 1) return false;
+      g.st.nFull -= 1;
+      return true;
+    case 6:  // elements left out on both sides
+      if (g.ld.nFull < 1) return false;
+      g.ld.active -= 1;
+      g.st.active -= 1;
+      return true;
+    case 7:  // a corner
+      if (p.nGR < 1) return false;
+      p.grSin[0] += 1;
+      return p.grDiv[0].d > 2;
+    case 8:  // a tile left out
+      p.numTiles -= 1;
+      return p.numTiles > 0;
+    case 9:  // an overlap counted twice
+      for (int r = 0; r < p.nGR; ++r)
+        if (p.overlap[r] > 0) {
+          p.overlap[r] -= 1;
+          return true;
+        }
+      return false;
+    default: return false;
+  }
+}
+
+}  // namespace
+}  // namespace lt
+
+extern "C" int librett_c_verify_map_check(int rank, const int* dim, const int* permutation,
+                                          size_t sizeofType, int num_sms, int element_units,
+                                          int mistake) {
+  if (lt::checkInput(rank, dim, permutation, sizeofType) != 0 || mistake < 0 || mistake > 9)
+    return LIBRETT_INVALID_PARAMETER;
+  lt::Fused f;
+  lt::fuseRanks(rank, dim, permutation, (int)sizeofType, f);
+  static thread_local lt::VerifyTiles tiles;
+  const uintptr_t at = element_units ? 4096 + sizeofType % 16 : 4096;  // addresses, not followed
+  if (lt::verifyTiles(f, num_sms > 0 ? num_sms : 152, reinterpret_cast<const void*>(at),
+                      reinterpret_cast<const void*>(2 * at), tiles) <= 0 ||
+      (mistake > 0 && !lt::plant(mistake, tiles)))
+    return LIBRETT_INVALID_DEVICE;
+  return lt::mapIsSoundHost(tiles) && lt::gridIsSound(f, tiles) ? LIBRETT_SUCCESS
+                                                                 : LIBRETT_INTERNAL_ERROR;
+}
+
 extern "C" int librett_c_verify(int rank, const int* dim, const int* permutation,
                                 size_t sizeofType, const void* idata, const void* odata,
                                 void* stream, unsigned long long* mismatches,
@@ -506,21 +727,18 @@ extern "C" int librett_c_verify(int rank, const int* dim, const int* permutation
   if (d == nullptr) return LIBRETT_INTERNAL_ERROR;
   static thread_local lt::VerifyTiles tiles;
   const int smem = lt::verifyTiles(f, sms, idata, odata, tiles);
-  const lt::VerifyKernel kernel =
-      smem > 0 ? lt::verifyKernelOf(reinterpret_cast<const lt::TileBlock*>(tiles.block)->store) : nullptr;
-  const int occ =
-      kernel ? lt::cachedOccupancy((const void*)kernel, lt::TILE_THREADS, smem) : 0;
-  cudaError_t err = cudaErrorInvalidConfiguration;
-  if (occ > 0) {
-    const uint32_t wave = (uint32_t)(sms * occ);
-    kernel<<<tiles.numTiles < wave ? tiles.numTiles : wave, lt::TILE_THREADS, smem, s>>>(tiles, d);
-    err = cudaGetLastError();
-  }
-  // (a launch is refused, too, when a device reset took the kernel's shared-memory limit)
-  if (err == cudaErrorInvalidConfiguration || err == cudaErrorInvalidValue)
-    err = lt::verifyElements(f, sms, idata, odata, d, s);
+  cudaError_t err = smem > 0 ? lt::checkTiles(tiles, sms, smem, d, s) : cudaErrorInvalidConfiguration;
   // also after an error: a launch may have been made
-  const cudaError_t done = cudaStreamSynchronize(s);
+  cudaError_t done = cudaStreamSynchronize(s);
+  // Element by element: without a tile, where its map is not the formula's, or where a
+  // launch was refused (as after a device reset, which takes a kernel's limit on
+  // shared memory)
+  const bool refused = err == cudaErrorInvalidConfiguration || err == cudaErrorInvalidValue;
+  if (done == cudaSuccess && (refused || (err == cudaSuccess && slot.host()[2] != 0))) {
+    slot.clear();
+    err = lt::verifyElements(f, sms, idata, odata, d, s);
+    done = cudaStreamSynchronize(s);
+  }
   if (err != cudaSuccess || done != cudaSuccess) return LIBRETT_INTERNAL_ERROR;
   const unsigned long long host[2] = {slot.host()[0], slot.host()[1]};
   *mismatches = host[0];
