@@ -354,8 +354,10 @@ std::vector<unsigned char> makeBlock(const Member& m, int* dataBytes) {
 
 // Moves the members of the cp.async buckets into mixed launches: one for
 // tiles that leave room for six CTAs per SM and one for larger tiles,
-// so that those do not cost the others occupancy.  Members whose tile has no
-// box keep their bucket.
+// so that those do not cost the others occupancy.  Members that a mixed launch
+// cannot take (a tile without a box, which no candidate is known to be; 2^31 tiles;
+// 128 MB of blocks) keep their bucket, with loads through registers: an
+// instantiation for cp.async of its own would be reached by nothing else.
 void mixBuckets(std::vector<Bucket>& buckets, const std::vector<Member>& members) {
   // narrow units, whose tiles take longest, first: the last CTAs end together
   std::stable_sort(buckets.begin(), buckets.end(), [](const Bucket& a, const Bucket& b) {
@@ -371,6 +373,7 @@ void mixBuckets(std::vector<Bucket>& buckets, const std::vector<Member>& members
       continue;
     }
     Bucket left = b, part[2] = {b, b};
+    left.loads = 0;
     for (Bucket* x : {&left, &part[0], &part[1]}) {
       x->members.clear();
       x->tiles = 0;

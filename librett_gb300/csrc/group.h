@@ -83,8 +83,8 @@ struct GroupTableJob {
 };
 
 // Launch of one bucket's kernel (defined per element size in k_tile*.cu);
-// loads: 0 registers, 1 cp.async (one tile per CTA), 2 cp.async with
-// persistent CTAs (grid = numSMs x occupancy, a grid stride over the tiles).
+// loads: 0 registers, 2 cp.async with persistent CTAs (grid = numSMs x occupancy,
+// a grid stride over the tiles).
 cudaError_t launchGroupTile4(int lv, int sv, int nl, int loads, const GroupTensor* tens,
                              const GroupTile* tiles, uint32_t numTiles, int smem,
                              cudaStream_t s, int numSMs);

@@ -926,8 +926,8 @@ __device__ __forceinline__ void stShared(uint32_t addr, const typename Word<BYTE
 // offsets come from the run split (GroupTensor): a small table entry per
 // run plus the position inside the run, so the tables stay in L1 even when
 // consecutive CTAs belong to different tensors; when they are small enough
-// the store-side tables are copied into shared memory with the data.  LOADS:
-// 0 stages the load units in registers; 1 copies them with cp.async straight
+// the store-side tables are copied into shared memory with the data.  The load
+// units are staged in registers or, with ASYNC, copied with cp.async straight
 // into shared memory (no data registers, so more CTAs fit an SM).  Every
 // access stays inside the member's input and output tensors.
 //
@@ -939,7 +939,7 @@ __device__ __forceinline__ void stShared(uint32_t addr, const typename Word<BYTE
 // padShift = 31 (none), so slot k's padded index is padT + k * padStep: one
 // multiply-add per slot.  Byte offsets are multiply-adds by a scale the
 // compiler cannot fold into shifts.
-template <int ES, int LV, int SV, int NL, int LOADS>
+template <int ES, int LV, int SV, int NL, bool ASYNC>
 __device__ __forceinline__ void groupTileBody(const GroupTensor* __restrict__ g, long long bin,
                                               long long bout) {
   using T = typename Word<ES>::T;
@@ -984,7 +984,7 @@ __device__ __forceinline__ void groupTileBody(const GroupTensor* __restrict__ g,
           runBase = offsetBytes(inM1, __ldg(offsetBytes(ldRow, (int)r, four)), esR);
         return reinterpret_cast<const LT*>(offsetBytes(runBase, a1, esR));
       };
-      if constexpr (LOADS >= 1) {
+      if constexpr (ASYNC) {
 #pragma unroll
         for (int k = 0; k < NL; ++k)
           if constexpr (STEP)  // the source is arithmetic only: predicate the copy
@@ -1121,9 +1121,10 @@ __device__ __forceinline__ const GroupTensor* groupTile(const GroupTensor* __res
   return tens + (int)(tile.x >> GROUP_TILE_SHIFT);
 }
 
-// One tile of a group bucket per CTA (LOADS 0: loads through registers,
-// 1: cp.async), or, with LOADS 2, persistent CTAs (grid = SMs x occupancy)
-// that walk the bucket's tile list with a grid stride, cp.async loads.
+// One tile of a group bucket per CTA, loads through registers (LOADS 0), or
+// persistent CTAs (grid = SMs x occupancy) that walk the bucket's tile list with a
+// grid stride, cp.async loads (LOADS 2).  One tile per CTA with cp.async is the mixed
+// launch (k_groupmix.cu).
 template <int ES, int LV, int SV, int NL, int LOADS>
 __global__ void __launch_bounds__(TILE_THREADS)
 groupTileKernel(const GroupTensor* __restrict__ tens, const GroupTile* __restrict__ tiles,
@@ -1133,12 +1134,12 @@ groupTileKernel(const GroupTensor* __restrict__ tens, const GroupTile* __restric
   if constexpr (LOADS == 2) {
     for (uint32_t t = blockIdx.x; t < numTiles; t += gridDim.x) {
       const GroupTensor* g = groupTile(tens, tiles, t, bin, bout);
-      groupTileBody<ES, LV, SV, NL, 1>(g, bin, bout);
+      groupTileBody<ES, LV, SV, NL, true>(g, bin, bout);
       __syncthreads();  // the next tile reuses the shared buffers
     }
   } else {
     const GroupTensor* g = groupTile(tens, tiles, blockIdx.x, bin, bout);
-    groupTileBody<ES, LV, SV, NL, LOADS>(g, bin, bout);
+    groupTileBody<ES, LV, SV, NL, false>(g, bin, bout);
   }
 }
 
