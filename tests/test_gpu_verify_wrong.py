@@ -60,3 +60,16 @@ def test_time_of_a_wrong_output(cuda, dims, perm, es):
     right = best((0, -1))
     out[::es // 4] ^= 1
     assert best((vol, 0)) < 5 * right
+
+
+@pytest.mark.parametrize("es", [4, 8, 16])
+def test_no_tile(cuda, es):
+    """A tensor of one element has no tile and goes element by element."""
+    import torch
+
+    inp = torch.arange(1, es + 1, dtype=torch.uint8, device="cuda")
+    out = inp.clone()
+    s = torch.cuda.current_stream()
+    assert L.verify([1], [0], es, inp.data_ptr(), out.data_ptr(), s) == (0, -1)
+    out[es - 1] ^= 1
+    assert L.verify([1], [0], es, inp.data_ptr(), out.data_ptr(), s) == (1, 0)
