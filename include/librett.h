@@ -88,15 +88,27 @@ librettResult librettDestroy(librettHandle handle);
 /*
  * Execute a plan out-of-place, asynchronously on the plan's stream
  * (LibreTT src/librett.h:121).  idata == odata -> LIBRETT_INVALID_PARAMETER.
+ *
+ * Order on the stream is the ordinary one: a transpose reads idata and writes
+ * odata after all work before it, and work behind it starts after it has ended.
+ * One thing differs from a plain launch: outside stream capture the kernels take
+ * part in programmatic dependent launch and release their successor early.  A
+ * kernel of the caller's that is itself launched with programmatic stream
+ * serialization directly behind a transpose (or a group) may start while that
+ * still runs, so it must call cudaGridDependencySynchronize (griddepcontrol.wait)
+ * before it touches idata's or odata's memory.  Every other launch, copy and event
+ * waits as before.
  */
 librettResult librettExecute(librettHandle handle, void* idata, void* odata);
 
 /* ---- Grouped execution (no LibreTT counterpart) ----
- * Many plans, each with its own input and output, executed as one CUDA
- * graph: members are bucketed by kernel shape, most buckets share one launch
- * (or two) over a device-resident descriptor table.  Creation plans, allocates (stream-
- * ordered on `stream`), writes the tables and instantiates the graph
- * (synchronising `stream` once); execution is one graph launch on `stream`;
+ * Many plans, each with its own input and output, executed at once: members are
+ * bucketed by kernel shape, most buckets share one launch (or two) over a
+ * device-resident descriptor table.  Creation plans, allocates (stream-ordered on
+ * `stream`), writes the tables and instantiates a graph of the launches
+ * (synchronising `stream` once); execution is one graph launch on `stream`, or,
+ * where the graph would hold a single launch, that launch (which releases its
+ * successor early, as described at librettExecute);
  * destruction frees in stream order.  The member plans may be destroyed once
  * the group exists (the group keeps what it needs).  Every member runs as a
  * flat tile inside its bucket (in element units when its pointers are not

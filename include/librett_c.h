@@ -77,7 +77,11 @@ int librett_c_plan_measure(librettHandle* handle, int rank, const int* dim,
                            const int* permutation, size_t sizeofType, void* stream,
                            const void* idata, void* odata);
 
-/* librettExecute (LibreTT src/librett.h:121). Asynchronous on the plan's stream. */
+/* librettExecute (LibreTT src/librett.h:121). Asynchronous on the plan's stream.
+ * A kernel of the caller's launched directly behind it with programmatic stream
+ * serialization must wait (griddepcontrol.wait) before it touches the tensors; see
+ * librett.h.  The same holds behind librett_c_transpose_noalloc, groups and the
+ * librett_c_mlp_* kernels. */
 int librett_c_execute(librettHandle handle, const void* idata, void* odata);
 
 /* librettDestroy (LibreTT src/librett.h:108). */
@@ -145,7 +149,8 @@ int librett_c_transpose_noalloc(int rank, const int* dim, const int* permutation
  * src/TensorTester.cpp:47-126): compares every element of odata with the
  * element of idata the transpose formula names, on the device, and returns
  * the number of mismatching elements and the smallest mismatching output
- * index (-1 if none).  Synchronises `stream`. */
+ * index (-1 if none).  Synchronises `stream`.  The tiles that it reads by are
+ * replayed against the formula in the same call. */
 int librett_c_verify(int rank, const int* dim, const int* permutation, size_t sizeofType,
                      const void* idata, const void* odata, void* stream,
                      unsigned long long* mismatches, long long* first_bad);

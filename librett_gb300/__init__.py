@@ -124,8 +124,8 @@ def transpose_noalloc(dim, permutation, sizeofType: int, stream, idata: int, oda
 
 
 class Group:
-    """Owning wrapper of a group of plans executed as one CUDA graph
-    (librett_c_group_*; no LibreTT counterpart)."""
+    """Owning wrapper of a group of plans executed at once, as one CUDA graph or
+    one launch (librett_c_group_*; no LibreTT counterpart)."""
 
     # policies per member size class (librett_c.h): tile + 4 * loads
     POLICY_SELECTOR, POLICY_WIDE, POLICY_WIDEST, POLICY_FILL = 0, 1, 2, 3

@@ -4,7 +4,7 @@
 // A launch of one bucket costs about 5 us whatever its work (graph node, first
 // descriptor reads, one tile), and a batch of small tensors has tens of buckets
 // of a few CTAs each.  500 tensors of 2^10 .. 2^16 elements: 33 launches on 8
-// graph branches 77.0 us, one mixed launch 18.6 us.  2,500 tensors of 2^10 ..
+// graph branches 77.0 us, one mixed launch 18.2 us.  2,500 tensors of 2^10 ..
 // 2^22 elements: 2567 us in buckets, 2406 us mixed (93 % of the copy rate); what
 // is left there is partly filled sectors of narrow runs.
 //

@@ -10,7 +10,7 @@
 // one by one from global memory (verifyKernel, kept for problems without a sound tile)
 // fetched 32 bytes for 4 and took 745 us for 66.8M float32 elements (64, 128,
 // 96, 85) perm (3, 1, 0, 2), where the two tensors' bytes take 80 us; this
-// kernel takes 121 us (4-byte output units: two thirds of the issue slots).
+// kernel takes 118 us (4-byte output units: two thirds of the issue slots).
 // The tile's addressing is the grouped kernel's, the grid and the proof that the
 // addressing is the transpose formula's are this file's own: each check replays its
 // tile's map (verify_map.h), and where that fails, which no problem is
