@@ -21,7 +21,9 @@
 #include <algorithm>
 #include <cstdlib>
 #include <cstring>
+#include <exception>
 #include <mutex>
+#include <new>
 #include <utility>
 #include <vector>
 
@@ -396,9 +398,13 @@ cudaError_t checkTiles(const VerifyTiles& tiles, int sms, int smem, unsigned lon
                        cudaStream_t s) {
   const VerifyKernels k = verifyKernelsOf(reinterpret_cast<const TileBlock*>(tiles.block)->store);
   if (k.tiles == nullptr) return cudaErrorInvalidConfiguration;
-  const int occ = cachedOccupancy((const void*)k.tiles, TILE_THREADS, smem);
-  if (occ < 1 || cachedOccupancy((const void*)k.map, TILE_THREADS, smem) < 1)
-    return cudaErrorInvalidConfiguration;
+  int occ = 0;
+  try {
+    if (cachedOccupancy((const void*)k.map, TILE_THREADS, smem) > 0)
+      occ = cachedOccupancy((const void*)k.tiles, TILE_THREADS, smem);
+  } catch (const std::exception&) {  // no host memory for its record
+  }
+  if (occ < 1) return cudaErrorInvalidConfiguration;
   k.tiles<<<std::min(tiles.numTiles, (uint32_t)(sms * occ)), TILE_THREADS, smem, s>>>(tiles, d);
   const cudaError_t err = cudaGetLastError();
   return err != cudaSuccess ? err : launchDependent(k.map, 1, TILE_THREADS, smem, s, tiles, d);
@@ -460,6 +466,16 @@ int verifyTiles(const Fused& f, int sms, const void* in, const void* out, Verify
   p.blockBytes = (int)block.size();
   std::memcpy(p.block, block.data(), block.size());
   return p.blockBytes + b.smBytes;
+}
+
+// As verifyTiles; 0 also where the host has no memory for the choice of a tile.
+int verifyTilesOrNone(const Fused& f, int sms, const void* in, const void* out,
+                      VerifyTiles& p) noexcept {
+  try {
+    return verifyTiles(f, sms, in, out, p);
+  } catch (const std::exception&) {
+    return 0;
+  }
 }
 
 // A call's result: three zeroed words (wrong elements, the complement of the first
@@ -526,6 +542,11 @@ class ResultSlot {
   static bool addPage(std::vector<unsigned long long*>& f) {
     const long unit = sysconf(_SC_PAGESIZE);
     pageBytes() = (SLOTS * SLOT + unit - 1) / unit * unit;
+    try {
+      f.reserve(SLOTS);  // for good: giving a slot back needs no memory
+    } catch (const std::exception&) {
+      return false;
+    }
     if (posix_memalign(&page(), (size_t)unit, pageBytes()) != 0) return false;
     for (size_t k = 0; k < SLOTS; ++k)
       f.push_back(reinterpret_cast<unsigned long long*>(static_cast<char*>(page()) + k * SLOT));
@@ -558,7 +579,10 @@ class ResultSlot {
     return m;
   }
   static std::vector<unsigned long long*>& freeSlots() {
-    static auto* f = new std::vector<unsigned long long*>();  // lives until the process exits
+    // lives until the process exits
+    alignas(std::vector<unsigned long long*>) static unsigned char place[sizeof(
+        std::vector<unsigned long long*>)];
+    static auto* f = new (place) std::vector<unsigned long long*>();
     return *f;
   }
   static void*& page() {
@@ -700,7 +724,7 @@ extern "C" int librett_c_verify_map_check(int rank, const int* dim, const int* p
   lt::fuseRanks(rank, dim, permutation, (int)sizeofType, f);
   static thread_local lt::VerifyTiles tiles;
   const uintptr_t at = element_units ? 4096 + sizeofType % 16 : 4096;  // addresses, not followed
-  if (lt::verifyTiles(f, num_sms > 0 ? num_sms : 152, reinterpret_cast<const void*>(at),
+  if (lt::verifyTilesOrNone(f, num_sms > 0 ? num_sms : 152, reinterpret_cast<const void*>(at),
                       reinterpret_cast<const void*>(2 * at), tiles) <= 0 ||
       (mistake > 0 && !lt::plant(mistake, tiles)))
     return LIBRETT_INVALID_DEVICE;
@@ -726,7 +750,7 @@ extern "C" int librett_c_verify(int rank, const int* dim, const int* permutation
   unsigned long long* d = slot.device();
   if (d == nullptr) return LIBRETT_INTERNAL_ERROR;
   static thread_local lt::VerifyTiles tiles;
-  const int smem = lt::verifyTiles(f, sms, idata, odata, tiles);
+  const int smem = lt::verifyTilesOrNone(f, sms, idata, odata, tiles);
   cudaError_t err = smem > 0 ? lt::checkTiles(tiles, sms, smem, d, s) : cudaErrorInvalidConfiguration;
   // also after an error: a launch may have been made
   cudaError_t done = cudaStreamSynchronize(s);

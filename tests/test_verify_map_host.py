@@ -1,12 +1,17 @@
 """The verifier's addressing on the host: the map of its tile is the transpose
 formula's, its tiles own every element once, and every planted mistake is seen."""
+import os
 import random
+import subprocess
+import sys
+from pathlib import Path
 
 import pytest
 
 import librett_gb300 as L
 from librett_gb300 import _lib
 
+ROOT = Path(__file__).resolve().parents[1]
 KNOWN = [([64, 48, 32], [2, 0, 1], 4), ([64, 128, 96, 85], [3, 1, 0, 2], 4),
          ([127, 63, 65, 33], [3, 1, 2, 0], 4), ([1000, 517], [1, 0], 8), ([200, 300, 400], [0, 2, 1], 8),
          ([4, 6, 819, 5, 25], [3, 0, 4, 2, 1], 16), ([70001], [0], 4), ([2] * 16, list(range(15, -1, -1)), 4),
@@ -60,3 +65,41 @@ def test_arguments():
     assert _check([4, 4], [1, 0], 3) == L.LIBRETT_INVALID_PARAMETER
     assert _check([4, 4], [1, 0], 4, 0, 10) == L.LIBRETT_INVALID_PARAMETER
     assert _check([4, 4], [1, 0], 4, 0, -1) == L.LIBRETT_INVALID_PARAMETER
+
+
+THROWING_NEW = r"""
+#include <cstdlib>
+#include <new>
+static bool armed;
+extern "C" void arm(int on) { armed = on != 0; }
+void* operator new(std::size_t n) {
+  void* p = armed ? nullptr : std::malloc(n ? n : 1);
+  if (p == nullptr) throw std::bad_alloc();
+  return p;
+}
+void operator delete(void* p) noexcept { std::free(p); }
+void operator delete(void* p, std::size_t) noexcept { std::free(p); }
+"""
+
+NO_MEMORY = r"""
+import ctypes, sys
+from librett_gb300 import _lib
+lib, own = _lib.load(), ctypes.CDLL(sys.argv[1])
+dims, perm = _lib.int_array([64, 48, 32]), _lib.int_array([2, 0, 1])
+own.arm(1)
+rc = lib.librett_c_verify_map_check(3, dims, perm, 4, 152, 0, 0)
+own.arm(0)
+print(rc, lib.librett_c_verify_map_check(3, dims, perm, 4, 152, 0, 0))
+"""
+
+
+def test_no_host_memory(tmp_path):
+    """Without host memory for the choice of a tile there is none (the check then goes
+    element by element); no exception leaves the C entry."""
+    src, own = tmp_path / "new.cpp", tmp_path / "new.so"
+    src.write_text(THROWING_NEW)
+    subprocess.run(["g++", "-shared", "-fPIC", "-O1", str(src), "-o", str(own)], check=True)
+    r = subprocess.run([sys.executable, "-c", NO_MEMORY, str(own)], cwd=ROOT, text=True,
+                       capture_output=True, timeout=300, env={**os.environ, "LD_PRELOAD": str(own)})
+    assert r.returncode == 0, r.stderr
+    assert r.stdout.split() == [str(L.LIBRETT_INVALID_DEVICE), str(L.LIBRETT_SUCCESS)]
