@@ -11,6 +11,7 @@
 #include <chrono>
 #include <cstdlib>
 #include <cstring>
+#include <exception>
 #include <list>
 #include <memory>
 #include <mutex>
@@ -61,10 +62,15 @@ bool lt::currentDevice(int& dev, int& sms, const char** name) {
   if (it == gDevs.end()) {
     cudaDeviceProp prop;
     if (cudaGetDeviceProperties(&prop, dev) != cudaSuccess) return false;
-    DevInfo di;
-    di.sms = prop.multiProcessorCount;
-    di.name = prop.name;
-    it = gDevs.emplace(dev, di).first;
+    sms = prop.multiProcessorCount;
+    try {
+      DevInfo di;
+      di.sms = sms;
+      di.name = prop.name;
+      it = gDevs.emplace(dev, std::move(di)).first;
+    } catch (const std::exception&) {
+      return name == nullptr;  // no host memory for the record
+    }
   }
   sms = it->second.sms;
   // entries are never erased and map nodes do not move: the name stays valid
@@ -74,7 +80,7 @@ bool lt::currentDevice(int& dev, int& sms, const char** name) {
 
 bool lt::currentDevice(int& dev, int& sms, std::string* name) {
   const char* n = nullptr;
-  if (!currentDevice(dev, sms, &n)) return false;
+  if (!currentDevice(dev, sms, name ? &n : static_cast<const char**>(nullptr))) return false;
   if (name) *name = n;
   return true;
 }

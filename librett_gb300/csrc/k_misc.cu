@@ -1,6 +1,7 @@
 // Copy and row-copy launches, occupancy cache, and the launch dispatcher
 // (the role of LibreTT's librettKernel switch, src/kernel.cpp:1008-1215).
 #include <atomic>
+#include <exception>
 #include <map>
 #include <mutex>
 #include <tuple>
@@ -68,7 +69,11 @@ int cachedOccupancy(const void* func, int threads, int smem) {
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, func, threads, smem) != cudaSuccess)
     return 0;
   std::lock_guard<std::mutex> lk(mu);
-  cache[key] = occ;
+  try {
+    cache[key] = occ;
+  } catch (const std::exception&) {
+    // no host memory: asked again next time
+  }
   return occ;
 }
 

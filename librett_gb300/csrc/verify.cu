@@ -398,13 +398,9 @@ cudaError_t checkTiles(const VerifyTiles& tiles, int sms, int smem, unsigned lon
                        cudaStream_t s) {
   const VerifyKernels k = verifyKernelsOf(reinterpret_cast<const TileBlock*>(tiles.block)->store);
   if (k.tiles == nullptr) return cudaErrorInvalidConfiguration;
-  int occ = 0;
-  try {
-    if (cachedOccupancy((const void*)k.map, TILE_THREADS, smem) > 0)
-      occ = cachedOccupancy((const void*)k.tiles, TILE_THREADS, smem);
-  } catch (const std::exception&) {  // no host memory for its record
-  }
-  if (occ < 1) return cudaErrorInvalidConfiguration;
+  const int occ = cachedOccupancy((const void*)k.tiles, TILE_THREADS, smem);
+  if (occ < 1 || cachedOccupancy((const void*)k.map, TILE_THREADS, smem) < 1)
+    return cudaErrorInvalidConfiguration;
   k.tiles<<<std::min(tiles.numTiles, (uint32_t)(sms * occ)), TILE_THREADS, smem, s>>>(tiles, d);
   const cudaError_t err = cudaGetLastError();
   return err != cudaSuccess ? err : launchDependent(k.map, 1, TILE_THREADS, smem, s, tiles, d);
@@ -755,11 +751,11 @@ extern "C" int librett_c_verify(int rank, const int* dim, const int* permutation
   // also after an error: a launch may have been made
   cudaError_t done = cudaStreamSynchronize(s);
   // Element by element: without a tile, where its map is not the formula's, or where a
-  // launch was refused (as after a device reset, which takes a kernel's limit on
-  // shared memory)
+  // launch was refused
   const bool refused = err == cudaErrorInvalidConfiguration || err == cudaErrorInvalidValue;
   if (done == cudaSuccess && (refused || (err == cudaSuccess && slot.host()[2] != 0))) {
     slot.clear();
+    cudaGetLastError();  // of what was refused
     err = lt::verifyElements(f, sms, idata, odata, d, s);
     done = cudaStreamSynchronize(s);
   }

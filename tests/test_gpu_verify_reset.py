@@ -1,6 +1,6 @@
-"""Checks go on after a cudaDeviceReset, which ends every registration and kernel
-attribute of the process: small and large tiles, errors counted, before and after.  In a
-process of its own, without torch, whose buffers would be lost."""
+"""Checks go on after a cudaDeviceReset, which ends every registration of host
+memory: small and large tiles, errors counted, before and after.  In a process of its
+own, without torch, whose buffers would be lost."""
 import subprocess
 import sys
 from pathlib import Path
