@@ -18,7 +18,7 @@
 // A layer-by-layer version (a 64 x 64-tiled SGEMM, bias, mask and column-sum
 // kernels, 22 launches) took 721 us for a step of 1,024 rows, most of it in the
 // weight gradients, whose four CTAs each summed all rows one after the other;
-// this takes 28.8 us (28.5 to 31.1 on several boxes), of which forward 8.1 and
+// this takes 28.8 us (28.5 to 31.1 from run to run), of which forward 8.1 and
 // backward 15.7.
 //
 // Everything is float32 on the FMA units: an output's products are added in
